@@ -27,12 +27,11 @@
 #define ADJ_BS 256
 
 // cell, weights and weight gradients at (x, y) (weight.f:61-101); 2D, one sector
-__device__ __forceinline__ bool adj_wgrad(const DevGeo& g, float x, float y, int& key, float* w,
+__device__ __forceinline__ bool adj_wgrad(const DevGeo& g, float x, float y, CellW& cw, float* w,
                                           float (*dw)[2]) {
-    const CellW cw = gx_cell(g, x, y, 0.f, true);
-    key = cw.key;
+    cw = gx_cell_t<true, 2>(g, x, y, 0.f, true);
     if (cw.key < 0) return false;
-    gx_weights(g, cw, w);
+    gx_weights<2>(g, cw, w);
     const float r2 = x * x + y * y;
     if (!(r2 > 0.f)) {
         for (int k = 0; k < 4; k++) dw[k][0] = dw[k][1] = 0.f;
@@ -55,12 +54,12 @@ __device__ __forceinline__ bool adj_wgrad(const DevGeo& g, float x, float y, int
 }
 
 // acceleration at (x, y) from the Cartesian field and the halo (grdacc + halfrc)
-__device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* __restrict__ F, int key,
+__device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* __restrict__ F, const CellW& cw,
                                           const float* w, float x, float y, float& ax, float& ay) {
     ax = ay = 0.f;
-    if (key < 0) return;
+    if (cw.key < 0) return;
     int ic[8];
-    gx_corners(g, key, ic);
+    gx_corners_rt<2>(g, cw.key, cw.jt, ic);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (ic[k] < 0) continue;
@@ -79,61 +78,102 @@ __device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* __restr
     }
 }
 
-// particles in load order from the context's storage order
+// particles in load order from the context's storage order, one record
+// (x, y, vx, vy) of 16 bytes each
 __global__ void k_adj_gather(const float* __restrict__ Pc, int64_t cap, int64_t n,
-                             const int32_t* __restrict__ origin, float* __restrict__ S) {
+                             const int32_t* __restrict__ origin, float4* __restrict__ S) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int64_t o = origin[i];
-    for (int k = 0; k < 4; k++) S[k * n + o] = Pc[k * cap + i];
+    S[origin[i]] = make_float4(Pc[i], Pc[cap + i], Pc[2 * cap + i], Pc[3 * cap + i]);
 }
 
-// forward step of particles in load order: v += a(x); x += v (stpgrp.f:26-32)
-__global__ void k_adj_fwd(DevGeo g, float* __restrict__ S, int64_t n, const float4* __restrict__ F) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float x = S[i], y = S[n + i], vx = S[2 * n + i], vy = S[3 * n + i];
-    const CellW cw = gx_cell(g, x, y, 0.f, true);
+// massgn of one particle at (x, y): its four weights as the 2^-20 integers of
+// gx_deposit.cu, added straight into the int64 mesh accumulator (integer
+// sums: the same mass whatever the order), and its ring into [rlo, rhi]
+__device__ __forceinline__ void adj_deposit(const DevGeo& g, float x, float y, unsigned long long* __restrict__ acc,
+                                            int& rlo, int& rhi) {
+    const CellW cw = gx_cell_t<true, 2>(g, x, y, 0.f, false);
+    if (cw.key < 0) return;
+    rlo = min(rlo, cw.row);
+    rhi = max(rhi, cw.row);
     float w[8];
-    if (cw.key >= 0) gx_weights(g, cw, w);
-    float ax, ay;
-    adj_accel(g, F, cw.key, w, x, y, ax, ay);
-    vx += ax;
-    vy += ay;
-    S[i] = x + vx;
-    S[n + i] = y + vy;
-    S[2 * n + i] = vx;
-    S[3 * n + i] = vy;
+    int ic[8];
+    gx_weights<2>(g, cw, w);
+    gx_corners_rt<2>(g, cw.key, cw.jt, ic);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int v = __float2int_rn(w[k] * 1048576.0f);
+        if (ic[k] >= 0 && v) atomicAdd(acc + ic[k], (unsigned long long)(long long)v);
+    }
 }
 
-// reverse drift x_s = x_{s+1} - v_{s+1}
-__global__ void k_adj_rdrift(float* __restrict__ S, int64_t n) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    S[i] -= S[2 * n + i];
-    S[n + i] -= S[3 * n + i];
+// the ring range of a pass (rng[0] first, rng[1] last), one atomic pair per warp
+__device__ __forceinline__ void adj_range(int rlo, int rhi, int32_t* __restrict__ rng) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        rlo = min(rlo, __shfl_xor_sync(0xffffffffu, rlo, o));
+        rhi = max(rhi, __shfl_xor_sync(0xffffffffu, rhi, o));
+    }
+    if ((threadIdx.x & 31) == 0 && rhi >= 0) {
+        atomicMin(rng, rlo);
+        atomicMax(rng + 1, rhi);
+    }
 }
 
-// largest |difference| between the reversed state and its checkpoint (max of
-// non-negative floats as ordered integers: order-free)
-__global__ void k_adj_drift(const float* __restrict__ S, const float* __restrict__ C, int64_t n4,
-                            unsigned int* __restrict__ out) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n4) return;
-    const float d = fabsf(S[i] - C[i]);
-    if (d > 0.f) atomicMax(out, __float_as_uint(d));
+// The sweeps' particle passes.  The particles stay in load order (16-byte
+// records): a pass waits on its gathers from the L2-resident field and on
+// its mesh reductions, not on the order.  Depositing the new position with
+// four 64-bit reductions into the accumulator inside the pass replaces a
+// pass that keyed the particles, their counting sort, the row deposit, the
+// combine and two copies of the positions (50 us a solve at 400k particles,
+// 128 x 256; the fused forward pass takes 23.7).  CTAs stride over the
+// particles so that the ring range costs one atomic pair per resident warp.
+
+// the mass of the records S (the first solve, and the context's mass afterwards)
+__global__ void __launch_bounds__(ADJ_BS) k_adj_mass(DevGeo g, const float4* __restrict__ S, int64_t n,
+                                                     unsigned long long* __restrict__ acc,
+                                                     int32_t* __restrict__ rng) {
+    int rlo = 0x7fffffff, rhi = -1;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float4 s = S[i];
+        adj_deposit(g, s.x, s.y, acc, rlo, rhi);
+    }
+    adj_range(rlo, rhi, rng);
+}
+
+// forward step: v += a(x); x += v (stpgrp.f:26-32); the new position deposited
+__global__ void __launch_bounds__(ADJ_BS) k_adj_fwd(DevGeo g, float4* __restrict__ S, int64_t n,
+                                                    const float4* __restrict__ F,
+                                                    unsigned long long* __restrict__ acc,
+                                                    int32_t* __restrict__ rng) {
+    int rlo = 0x7fffffff, rhi = -1;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        float4 s = S[i];
+        const CellW cw = gx_cell_t<true, 2>(g, s.x, s.y, 0.f, true);
+        float w[8];
+        if (cw.key >= 0) gx_weights<2>(g, cw, w);
+        float ax, ay;
+        adj_accel(g, F, cw, w, s.x, s.y, ax, ay);
+        s.z += ax;
+        s.w += ay;
+        s.x += s.z;
+        s.y += s.w;
+        S[i] = s;
+        adj_deposit(g, s.x, s.y, acc, rlo, rhi);
+    }
+    adj_range(rlo, rhi, rng);
 }
 
 // per-block FP64 sums of e^{2 i phi} over all particles
-__global__ void k_adj_a2(const float* __restrict__ S, int64_t n, double* __restrict__ part) {
+__global__ void k_adj_a2(const float4* __restrict__ S, int64_t n, double* __restrict__ part) {
     __shared__ double sh[2][ADJ_BS / 32];
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     double c = 0.0, s = 0.0;
-    if (i < n) {
-        const double x = S[i], y = S[n + i], r2 = x * x + y * y;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float4 q = S[i];
+        const double x = q.x, y = q.y, r2 = x * x + y * y;
         if (r2 > 0.0) {
-            c = (x * x - y * y) / r2;
-            s = 2.0 * x * y / r2;
+            c += (x * x - y * y) / r2;
+            s += 2.0 * x * y / r2;
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -158,12 +198,13 @@ __global__ void k_adj_a2(const float* __restrict__ S, int64_t n, double* __restr
 }
 
 // lambda_x at the final time: dJ/dx_T; lambda_v = 0
-__global__ void k_adj_init(const float* __restrict__ S, int64_t n, double a2r, double a2i, double J,
-                           float* __restrict__ L) {
+__global__ void k_adj_init(const float4* __restrict__ S, int64_t n, double a2r, double a2i, double J,
+                           float4* __restrict__ L) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     float gx = 0.f, gy = 0.f;
-    const double x = S[i], y = S[n + i], r2 = x * x + y * y;
+    const float4 q = S[i];
+    const double x = q.x, y = q.y, r2 = x * x + y * y;
     if (r2 > 0.0 && J > 0.0) {
         const double fr = (x * x - y * y) / r2, fi = 2.0 * x * y / r2, inv = 1.0 / (double)n;
         // dA2/dx = -2 i f y / (n r2), dA2/dy = 2 i f x / (n r2); dJ = Re(conj(A2) dA2) / J
@@ -172,40 +213,36 @@ __global__ void k_adj_init(const float* __restrict__ S, int64_t n, double a2r, d
         gx = (float)((a2r * dxr + a2i * dxi) / J);
         gy = (float)((a2r * dyr + a2i * dyi) / J);
     }
-    L[i] = gx;
-    L[n + i] = gy;
-    L[2 * n + i] = 0.f;
-    L[3 * n + i] = 0.f;
+    L[i] = make_float4(gx, gy, 0.f, 0.f);
 }
 
 // reverse step, first particle pass at x_s: reverse kick (unless the state
 // came from a checkpoint), mu, lambda_v <- mu, lambda_x += interpolation
-// slope . (F . mu) + halo Jacobian . mu, Q += W mu, halo parameter terms
-__global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float* __restrict__ S, float* __restrict__ L,
+// slope . (F . mu) + halo Jacobian . mu, Q += W mu (x and y of a cell side
+// by side), halo parameter terms
+__global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float4* __restrict__ S, float4* __restrict__ L,
                                                   int64_t n, const float4* __restrict__ F, int kick,
                                                   double* __restrict__ Q, double* __restrict__ tpart) {
     __shared__ double sh[2][ADJ_BS / 32];
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t mesh = g.mesh;
     double drc = 0.0, dv2 = 0.0;
-    if (i < n) {
-        const float x = S[i], y = S[n + i];
-        int key;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        float4 s = S[i], l = L[i];
+        const float x = s.x, y = s.y;
+        CellW cw;
         float w[8], dw[4][2];
-        const bool on = adj_wgrad(g, x, y, key, w, dw);
+        const bool on = adj_wgrad(g, x, y, cw, w, dw);
         if (kick) {
             float ax, ay;
-            adj_accel(g, F, on ? key : -1, w, x, y, ax, ay);
-            S[2 * n + i] -= ax;
-            S[3 * n + i] -= ay;
+            adj_accel(g, F, cw, w, x, y, ax, ay);
+            s.z -= ax;
+            s.w -= ay;
+            S[i] = s;
         }
-        float lx = L[i], ly = L[n + i];
-        const float m0 = L[2 * n + i] + lx, m1 = L[3 * n + i] + ly;
-        L[2 * n + i] = m0;
-        L[3 * n + i] = m1;
+        float lx = l.x, ly = l.y;
+        const float m0 = l.z + lx, m1 = l.w + ly;
         if (on) {
             int ic[8];
-            gx_corners(g, key, ic);
+            gx_corners_rt<2>(g, cw.key, cw.jt, ic);
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 if (ic[k] < 0) continue;
@@ -213,8 +250,8 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float* __restrict__ 
                 const float fdot = f.x * m0 + f.y * m1;
                 lx += dw[k][0] * fdot;
                 ly += dw[k][1] * fdot;
-                atomicAdd(&Q[ic[k]], (double)(w[k] * m0));
-                atomicAdd(&Q[mesh + ic[k]], (double)(w[k] * m1));
+                atomicAdd(&Q[2 * ic[k]], (double)(w[k] * m0));
+                atomicAdd(&Q[2 * ic[k] + 1], (double)(w[k] * m1));
             }
             if (g.halo == 1) {
                 // h = -v2 x / d, d = r^2 + rc^2: Jacobian -v2 (I / d - 2 x x^T / d^2)
@@ -225,12 +262,11 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float* __restrict__ 
                 lx += hxx * m0 + hxy * m1;
                 ly += hxy * m0 + hyy * m1;
                 const double xm = (double)x * m0 + (double)y * m1;
-                dv2 = -xm / (double)d;
-                drc = (double)v2 * 2.0 * sqrt((double)g.halo_rc2) * xm / ((double)d * d);
+                dv2 += -xm / (double)d;
+                drc += (double)v2 * 2.0 * sqrt((double)g.halo_rc2) * xm / ((double)d * d);
             }
         }
-        L[i] = lx;
-        L[n + i] = ly;
+        L[i] = make_float4(lx, ly, m0, m1);
     }
     for (int o = 16; o > 0; o >>= 1) {
         drc += __shfl_down_sync(0xffffffffu, drc, o);
@@ -254,26 +290,57 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float* __restrict__ 
     }
 }
 
-// second particle pass: lambda_x += pmass sum_c grad W_c(x) psi_c
-__global__ void k_adj_b(DevGeo g, const float* __restrict__ S, float* __restrict__ L, int64_t n,
-                        const float* __restrict__ psi, float pmass) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int key;
-    float w[8], dw[4][2];
-    if (!adj_wgrad(g, S[i], S[n + i], key, w, dw)) return;
-    int ic[8];
-    gx_corners(g, key, ic);
-    float gx = 0.f, gy = 0.f;
+// second particle pass of a reverse step fused with the start of the next:
+//   psi (else none yet): lambda_x += pmass sum_c grad W_c(x) psi_c at x_s;
+//   move: the reverse drift x_{s-1} = x_s - v_s; with a checkpoint ck its
+//   largest |difference| from the reversed position (max of non-negative
+//   floats as ordered integers: order-free), then the checkpoint itself; the
+//   position deposited for the next solve.
+__global__ void __launch_bounds__(ADJ_BS) k_adj_b(DevGeo g, float4* __restrict__ S, float4* __restrict__ L, int64_t n,
+                                                  const float* __restrict__ psi, float pmass, int move,
+                                                  const float4* __restrict__ ck, unsigned int* __restrict__ drift,
+                                                  unsigned long long* __restrict__ acc, int32_t* __restrict__ rng) {
+    int rlo = 0x7fffffff, rhi = -1;
+    float dm = 0.f;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        float4 s = S[i];
+        if (psi) {
+            CellW cw;
+            float w[8], dw[4][2];
+            if (adj_wgrad(g, s.x, s.y, cw, w, dw)) {
+                int ic[8];
+                gx_corners_rt<2>(g, cw.key, cw.jt, ic);
+                float gx = 0.f, gy = 0.f;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        if (ic[k] < 0) continue;
-        const float p = psi[ic[k]];
-        gx += dw[k][0] * p;
-        gy += dw[k][1] * p;
+                for (int k = 0; k < 4; k++) {
+                    if (ic[k] < 0) continue;
+                    const float p = __ldg(psi + ic[k]);
+                    gx += dw[k][0] * p;
+                    gy += dw[k][1] * p;
+                }
+                float2* l = reinterpret_cast<float2*>(L + i);
+                const float2 v = *l;
+                *l = make_float2(v.x + pmass * gx, v.y + pmass * gy);
+            }
+        }
+        if (!move) continue;
+        s.x -= s.z;
+        s.y -= s.w;
+        if (ck) {
+            const float4 c = __ldg(ck + i);
+            dm = fmaxf(dm, fmaxf(fabsf(s.x - c.x), fabsf(s.y - c.y)));
+            s = c;
+        }
+        S[i] = s;
+        adj_deposit(g, s.x, s.y, acc, rlo, rhi);
     }
-    L[i] += pmass * gx;
-    L[n + i] += pmass * gy;
+    if (!move) return;
+    adj_range(rlo, rhi, rng);
+    if (ck) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, o));
+        if ((threadIdx.x & 31) == 0 && dm > 0.f) atomicMax(drift, __float_as_uint(dm));
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -284,118 +351,129 @@ struct AdjAct {
     int m[64];
 };
 
-// polcat^T and synthesis^T: V[t][a][ir] = scale sum_j g_t(ir, j) (c_m(j), s_m(j))
-__global__ void k_adjt_syn(DevGeo g, AdjAct act, int nact, const double* __restrict__ Q,
-                           float2* __restrict__ V) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    const int nr = g.nr, na = g.na;
-    if (o >= 2 * nact * nr) return;
-    const int t = o / (nact * nr), rem = o - t * nact * nr, a = rem / nr, ir = rem - a * nr;
-    const int m = act.m[a];
-    const int64_t mesh = g.mesh;
-    float sa = 0.f, sb = 0.f;
-    for (int j = 0; j < na; j++) {
-        const int64_t l = (int64_t)ir * na + j;
-        const float qx = (float)Q[l], qy = (float)Q[mesh + l];
+// polcat^T and synthesis^T: V[t][a][ir] = scale sum_j g_t(ir, j) (c_m(j), s_m(j)).
+// One ring per CTA; thread (a, q) sums both components of harmonic a (of a
+// block of AT_H) over the spokes j = q (mod AT_Q), with the forward table
+// T[j][2a] = cos, T[j][2a + 1] = -sin (k_fwdtab) read through L1, the AT_Q
+// partials added in q order.  Q is cleared for the next step.  The sums are
+// latency-bound chains: one thread per output (2304 of them at 128 x 256, m =
+// 0..8, sines evaluated in place) took 97 us, this split takes 5.5.
+#define AT_H 16
+#define AT_Q 16
+__global__ void __launch_bounds__(AT_H * AT_Q) k_adjt_syn(DevGeo g, AdjAct act, int nact, int ncp,
+                                                          double2* __restrict__ Q, const float* __restrict__ T,
+                                                          float2* __restrict__ V) {
+    extern __shared__ __align__(16) float2 gv[];  // [na]: radial, azimuthal
+    __shared__ float4 part[AT_Q][AT_H];
+    const int nr = g.nr, na = g.na, ir = blockIdx.x;
+    for (int j = threadIdx.x; j < na; j += blockDim.x) {
+        double2* q = Q + (size_t)ir * na + j;
+        const float qx = (float)q->x, qy = (float)q->y;
+        *q = make_double2(0.0, 0.0);
         float sn, cs;
         sincospif(2.0f * (float)j / (float)na, &sn, &cs);
-        const float gv = (t == 0) ? (qx * cs + qy * sn) : (-qx * sn + qy * cs);
-        if (m == 0) {
-            sa += gv;
-        } else if (m == g.mmax - 1) {
-            sa += (j & 1) ? -gv : gv;
-        } else {
-            float sm, cm;
-            sincospif(2.0f * (float)(((int64_t)m * j) % na) / (float)na, &sm, &cm);
-            sa += 2.f * gv * cm;
-            sb -= 2.f * gv * sm;
-        }
+        gv[j] = make_float2(qx * cs + qy * sn, -qx * sn + qy * cs);
     }
+    __syncthreads();
+    const int h = threadIdx.x % AT_H, q = threadIdx.x / AT_H;
     const float scale = 1.0f / (float)na;
-    V[o] = make_float2(scale * sa, scale * sb);
-}
-
-// radial contraction^T: per (a, is) one warp over ir
-__global__ void k_adjt_conv(DevGeo g, AdjAct act, int nact, const float* __restrict__ G,
-                            const float2* __restrict__ V, float2* __restrict__ AB) {
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int nr = g.nr;
-    if (wid >= nact * nr) return;
-    const int a = wid / nr, is = wid - a * nr, m = act.m[a];
-    const bool hasb = (m > 0 && m < g.mmax - 1);
-    const bool ft = (g.ng > 1) && (m >= 1) && (m <= min(g.ng, g.mmax - 1) - 1);
-    const float* G0 = G + ((size_t)(0 * g.ng + m) * g.nkz) * nr * (size_t)nr + (size_t)is * nr;
-    const float* G1 = G + ((size_t)(1 * g.ng + m) * g.nkz) * nr * (size_t)nr + (size_t)is * nr;
-    const float2* V0 = V + (size_t)a * nr;
-    const float2* V1 = V + ((size_t)nact + a) * nr;
-    float sa = 0.f, sb = 0.f;
-    for (int ir = lane; ir < nr; ir += 32) {
-        const float g0 = __ldg(G0 + ir);
-        const float2 v0 = V0[ir];
-        sa += g0 * v0.x;
-        if (hasb) sb += g0 * v0.y;
-        if (ft) {
-            const float g1 = __ldg(G1 + ir);
-            const float2 v1 = V1[ir];
-            sb += g1 * v1.x;
-            sa -= g1 * v1.y;
+    for (int a0 = 0; a0 < nact; a0 += AT_H) {
+        const int a = a0 + h;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (a < nact) {
+#pragma unroll 4
+            for (int j = q; j < na; j += AT_Q) {
+                const float2 t = __ldg(reinterpret_cast<const float2*>(T + (size_t)j * ncp + 2 * a));
+                const float2 v = gv[j];
+                s.x += v.x * t.x;
+                s.y += v.x * t.y;
+                s.z += v.y * t.x;
+                s.w += v.y * t.y;
+            }
         }
+        part[q][h] = s;
+        __syncthreads();
+        if (threadIdx.x < AT_H && a < nact) {
+            float4 v = part[0][threadIdx.x];
+            for (int k = 1; k < AT_Q; k++) {
+                const float4 p = part[k][threadIdx.x];
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            const int m = act.m[a];
+            const bool two = m > 0 && m < g.mmax - 1;
+            const float f = two ? 2.f * scale : scale, fs = two ? f : 0.f;
+            V[(size_t)a * nr + ir] = make_float2(f * v.x, fs * v.y);
+            V[((size_t)nact + a) * nr + ir] = make_float2(f * v.z, fs * v.w);
+        }
+        __syncthreads();
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        sa += __shfl_down_sync(0xffffffffu, sa, o);
-        sb += __shfl_down_sync(0xffffffffu, sb, o);
-    }
-    if (lane == 0) AB[wid] = make_float2(sa, hasb ? sb : 0.f);
 }
 
-// forward DFT^T: psi(ir, j) = sum_a A cos(2 pi m j / na) - B sin(...)
-__global__ void k_adjt_fwd(DevGeo g, AdjAct act, int nact, const float2* __restrict__ AB,
-                           float* __restrict__ psi) {
-    const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (l >= g.mesh) return;
-    const int na = g.na, nr = g.nr;
-    const int ir = (int)(l / na), j = (int)(l - (int64_t)ir * na);
-    float s = 0.f;
-    for (int a = 0; a < nact; a++) {
-        const float2 ab = AB[(size_t)a * nr + ir];
-        float sm, cm;
-        sincospif(2.0f * (float)(((int64_t)act.m[a] * j) % na) / (float)na, &sm, &cm);
-        s += ab.x * cm - ab.y * sm;
+// radial contraction^T and forward DFT^T of one source ring per CTA: AB =
+// (A, B) of each harmonic, one warp per harmonic over the field rings; then
+// psi(is, j) = sum_a A cos(2 pi m j / na) - B sin(...)
+__global__ void __launch_bounds__(ADJ_BS) k_adjt_conv(DevGeo g, AdjAct act, int nact, int ncp,
+                                                      const float* __restrict__ G, const float2* __restrict__ V,
+                                                      const float* __restrict__ T, float* __restrict__ psi) {
+    __shared__ float2 AB[64];
+    const int lane = threadIdx.x & 31, nr = g.nr, na = g.na, is = blockIdx.x;
+    for (int a = threadIdx.x >> 5; a < nact; a += ADJ_BS / 32) {
+        const int m = act.m[a];
+        const bool hasb = (m > 0 && m < g.mmax - 1);
+        const bool ft = (g.ng > 1) && (m >= 1) && (m <= min(g.ng, g.mmax - 1) - 1);
+        const float* G0 = G + ((size_t)(0 * g.ng + m) * g.nkz) * nr * (size_t)nr + (size_t)is * nr;
+        const float* G1 = G + ((size_t)(1 * g.ng + m) * g.nkz) * nr * (size_t)nr + (size_t)is * nr;
+        const float2* V0 = V + (size_t)a * nr;
+        const float2* V1 = V + ((size_t)nact + a) * nr;
+        float sa = 0.f, sb = 0.f;
+#pragma unroll 4
+        for (int ir = lane; ir < nr; ir += 32) {
+            const float g0 = __ldg(G0 + ir);
+            const float2 v0 = __ldg(V0 + ir);
+            sa += g0 * v0.x;
+            if (hasb) sb += g0 * v0.y;
+            if (ft) {
+                const float g1 = __ldg(G1 + ir);
+                const float2 v1 = __ldg(V1 + ir);
+                sb += g1 * v1.x;
+                sa -= g1 * v1.y;
+            }
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            sa += __shfl_down_sync(0xffffffffu, sa, o);
+            sb += __shfl_down_sync(0xffffffffu, sb, o);
+        }
+        if (lane == 0) AB[a] = make_float2(sa, hasb ? sb : 0.f);
     }
-    psi[l] = s;
+    __syncthreads();
+    for (int j = threadIdx.x; j < na; j += ADJ_BS) {
+        float s = 0.f;
+        for (int a = 0; a < nact; a++) {
+            const float2 t = __ldg(reinterpret_cast<const float2*>(T + (size_t)j * ncp + 2 * a));
+            s += AB[a].x * t.x + AB[a].y * t.y;
+        }
+        psi[(size_t)is * na + j] = s;
+    }
 }
 
 // ---------------------------------------------------------------------------
-__global__ void k_adj_scatter(const float* __restrict__ S, int64_t n, float* __restrict__ Pc, int64_t cap,
+__global__ void k_adj_scatter(const float4* __restrict__ S, int64_t n, float* __restrict__ Pc, int64_t cap,
                               int32_t* __restrict__ origin, int32_t* __restrict__ perm) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    for (int k = 0; k < 4; k++) Pc[k * cap + i] = S[k * n + i];
+    const float4 s = S[i];
+    Pc[i] = s.x;
+    Pc[cap + i] = s.y;
+    Pc[2 * cap + i] = s.z;
+    Pc[3 * cap + i] = s.w;
     origin[i] = (int32_t)i;
     perm[i] = (int32_t)i;
 }
 
-namespace {
-struct AdjBuf {
-    float *S = nullptr, *L = nullptr, *ck = nullptr, *psi = nullptr;
-    double *Q = nullptr, *part = nullptr, *tpart = nullptr;
-    float2 *V = nullptr, *AB = nullptr;
-    unsigned int* drift = nullptr;
-    ~AdjBuf() {
-        void* p[] = {S, L, ck, psi, Q, part, tpart, V, AB, drift};
-        for (void* q : p)
-            if (q) cudaFree(q);
-    }
-};
-}  // namespace
-
-// positions of S into the context (storage = load order) -> mass, field
-static int adj_solve(GxCtx* c, const float* S, int64_t n) {
-    GX_CUDA(c, cudaMemcpyAsync(c->pbuf[c->cur], S, sizeof(float) * n, cudaMemcpyDeviceToDevice, c->stream));
-    GX_CUDA(c, cudaMemcpyAsync(c->pbuf[c->cur] + c->cap, S + n, sizeof(float) * n, cudaMemcpyDeviceToDevice,
-                               c->stream));
+// the deposited accumulator -> the mass, then its field
+static int adj_solve(GxCtx* c) {
     c->zr_valid = false;  // the mass array is no longer a fused pass's
-    int rc = gx_mixed_masset(c);
+    int rc = gx_mass_convert(c);
     if (rc) return rc;
     return gx_mixed_findf(c, 0, true);
 }
@@ -417,48 +495,86 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
         if (rc) return rc;
     }
     const DevGeo& g = c->g;
-    const int nact = c->spec.nact;
+    const int nact = c->spec.nact, ncp = (2 * nact + 3) & ~3;  // row of the forward table (gx_solve.cu)
     AdjAct act;
     for (int a = 0; a < 64; a++) act.m[a] = (a < nact) ? c->spec.m[a] : 0;
     const unsigned nb = (unsigned)((n + ADJ_BS - 1) / ADJ_BS);
+    const unsigned np = std::min(nb, 148u * 8u);  // CTAs of the strided passes
     const int nck = nsteps / ckpt_every + 1;
-    AdjBuf b;
-    GX_CUDA(c, cudaMalloc((void**)&b.S, sizeof(float) * 4 * n));
-    GX_CUDA(c, cudaMalloc((void**)&b.L, sizeof(float) * 4 * n));
-    GX_CUDA(c, cudaMalloc((void**)&b.ck, sizeof(float) * 4 * n * (size_t)nck));
-    GX_CUDA(c, cudaMalloc((void**)&b.psi, sizeof(float) * g.mesh));
-    GX_CUDA(c, cudaMalloc((void**)&b.Q, sizeof(double) * 2 * g.mesh));
-    GX_CUDA(c, cudaMalloc((void**)&b.part, sizeof(double) * 2 * nb));
-    GX_CUDA(c, cudaMalloc((void**)&b.tpart, sizeof(double) * 2 * nb));
-    GX_CUDA(c, cudaMalloc((void**)&b.V, sizeof(float2) * 2 * nact * g.nr));
-    GX_CUDA(c, cudaMalloc((void**)&b.AB, sizeof(float2) * nact * g.nr));
-    GX_CUDA(c, cudaMalloc((void**)&b.drift, sizeof(unsigned int)));
+    // the sweeps' buffers: one block kept with the context (allocating and
+    // freeing them took a tenth of a 100-step call), given back when the
+    // context's particle arrays grow and with the context
+    struct {
+        float4 *S, *L, *ck;
+        double2* Q;
+        double *part, *tpart;
+        float2* V;
+        float* psi;
+        unsigned int* drift;
+    } b;
+    size_t off = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = off;
+        off += (bytes + 255) & ~(size_t)255;
+        return o;
+    };
+    const size_t oS = take(sizeof(float4) * n), oL = take(sizeof(float4) * n),
+                 ock = take(sizeof(float4) * n * (size_t)nck), oQ = take(sizeof(double2) * g.mesh),
+                 opart = take(sizeof(double) * 2 * np), otpart = take(sizeof(double) * 2 * np),
+                 oV = take(sizeof(float2) * 2 * nact * g.nr), opsi = take(sizeof(float) * g.mesh),
+                 odrift = take(sizeof(unsigned int));
+    if (off > c->adj_bytes) {
+        if (c->adj_ws) cudaFree(c->adj_ws);
+        c->adj_ws = nullptr;
+        c->adj_bytes = 0;
+        GX_CUDA(c, cudaMalloc((void**)&c->adj_ws, off));
+        c->adj_bytes = off;
+    }
+    b.S = (float4*)(c->adj_ws + oS);
+    b.L = (float4*)(c->adj_ws + oL);
+    b.ck = (float4*)(c->adj_ws + ock);
+    b.Q = (double2*)(c->adj_ws + oQ);
+    b.part = (double*)(c->adj_ws + opart);
+    b.tpart = (double*)(c->adj_ws + otpart);
+    b.V = (float2*)(c->adj_ws + oV);
+    b.psi = (float*)(c->adj_ws + opsi);
+    b.drift = (unsigned int*)(c->adj_ws + odrift);
     cudaStream_t st = c->stream;
+    int32_t* rng = c->bk_ctl + 13;  // ring range of the accumulated mass (k_mass_convert reads and resets it)
     c->launches = 0;
     GX_CUDA(c, cudaEventRecord(c->ev0, st));
     // initial state in load order
     k_adj_gather<<<nb, ADJ_BS, 0, st>>>(c->pbuf[c->cur], c->cap, n, c->origin, b.S);
     GX_LAUNCHED(c);
-    const size_t sbytes = sizeof(float) * 4 * n;
+    const size_t sbytes = sizeof(float4) * n;
     GX_CUDA(c, cudaMemcpyAsync(b.ck, b.S, sbytes, cudaMemcpyDeviceToDevice, st));
     // forward sweep with checkpoints
+    if (nsteps > 0) {
+        k_adj_mass<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->macc, rng);
+        GX_LAUNCHED(c);
+    }
     for (int s = 0; s < nsteps; s++) {
-        int rc = adj_solve(c, b.S, n);
+        int rc = adj_solve(c);
         if (rc) return rc;
-        k_adj_fwd<<<nb, ADJ_BS, 0, st>>>(g, b.S, n, c->field);
+        k_adj_fwd<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->field, c->macc, rng);
         GX_LAUNCHED(c);
         if ((s + 1) % ckpt_every == 0)
-            GX_CUDA(c, cudaMemcpyAsync(b.ck + (size_t)((s + 1) / ckpt_every) * 4 * n, b.S, sbytes,
+            GX_CUDA(c, cudaMemcpyAsync(b.ck + (size_t)((s + 1) / ckpt_every) * n, b.S, sbytes,
                                        cudaMemcpyDeviceToDevice, st));
     }
+    if (nsteps > 0) {
+        // the last pass deposited the final positions, which no solve takes
+        int rc = gx_mass_convert(c);
+        if (rc) return rc;
+    }
     // objective
-    k_adj_a2<<<nb, ADJ_BS, 0, st>>>(b.S, n, b.part);
+    k_adj_a2<<<np, ADJ_BS, 0, st>>>(b.S, n, b.part);
     GX_LAUNCHED(c);
-    std::vector<double> hp(2 * (size_t)nb);
-    GX_CUDA(c, cudaMemcpyAsync(hp.data(), b.part, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, st));
+    std::vector<double> hp(2 * (size_t)np);
+    GX_CUDA(c, cudaMemcpyAsync(hp.data(), b.part, sizeof(double) * 2 * np, cudaMemcpyDeviceToHost, st));
     GX_CUDA(c, cudaStreamSynchronize(st));
     double sre = 0.0, sim = 0.0;
-    for (unsigned i = 0; i < nb; i++) {
+    for (unsigned i = 0; i < np; i++) {
         sre += hp[2 * i];
         sim += hp[2 * i + 1];
     }
@@ -466,49 +582,39 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     const double J = sqrt(a2r * a2r + a2i * a2i);
     k_adj_init<<<nb, ADJ_BS, 0, st>>>(b.S, n, a2r, a2i, J, b.L);
     GX_LAUNCHED(c);
-    GX_CUDA(c, cudaMemsetAsync(b.tpart, 0, sizeof(double) * 2 * nb, st));
+    GX_CUDA(c, cudaMemsetAsync(b.tpart, 0, sizeof(double) * 2 * np, st));
     GX_CUDA(c, cudaMemsetAsync(b.drift, 0, sizeof(unsigned int), st));
+    GX_CUDA(c, cudaMemsetAsync(b.Q, 0, sizeof(double2) * g.mesh, st));
     // reverse sweep
     for (int s = nsteps - 1; s >= 0; s--) {
         const bool ck = (s % ckpt_every) == 0;
-        k_adj_rdrift<<<nb, ADJ_BS, 0, st>>>(b.S, n);
+        // the psi term of step s + 1, the drift back to x_s and its deposit
+        k_adj_b<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, s == nsteps - 1 ? nullptr : b.psi, g.pmass, 1,
+                                       ck ? b.ck + (size_t)(s / ckpt_every) * n : nullptr, b.drift, c->macc, rng);
         GX_LAUNCHED(c);
-        if (ck) {
-            // the reversed positions against the checkpoint, then the checkpoint
-            const float* C0 = b.ck + (size_t)(s / ckpt_every) * 4 * n;
-            k_adj_drift<<<(unsigned)((2 * n + ADJ_BS - 1) / ADJ_BS), ADJ_BS, 0, st>>>(b.S, C0, 2 * n, b.drift);
-            GX_LAUNCHED(c);
-            GX_CUDA(c, cudaMemcpyAsync(b.S, C0, sbytes, cudaMemcpyDeviceToDevice, st));
-        }
-        int rc = adj_solve(c, b.S, n);
+        int rc = adj_solve(c);
         if (rc) return rc;
-        GX_CUDA(c, cudaMemsetAsync(b.Q, 0, sizeof(double) * 2 * g.mesh, st));
-        k_adj_a<<<nb, ADJ_BS, 0, st>>>(g, b.S, b.L, n, c->field, ck ? 0 : 1, b.Q, b.tpart);
+        k_adj_a<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, c->field, ck ? 0 : 1, reinterpret_cast<double*>(b.Q), b.tpart);
         GX_LAUNCHED(c);
-        const int n_syn = 2 * nact * g.nr;
-        k_adjt_syn<<<(n_syn + 127) / 128, 128, 0, st>>>(g, act, nact, b.Q, b.V);
+        k_adjt_syn<<<g.nr, AT_H * AT_Q, sizeof(float2) * g.na, st>>>(g, act, nact, ncp, b.Q, c->fwdtab, b.V);
         GX_LAUNCHED(c);
-        const int n_conv = nact * g.nr * 32;
-        k_adjt_conv<<<(n_conv + 255) / 256, 256, 0, st>>>(g, act, nact, c->green32, b.V, b.AB);
+        k_adjt_conv<<<g.nr, ADJ_BS, 0, st>>>(g, act, nact, ncp, c->green32, b.V, c->fwdtab, b.psi);
         GX_LAUNCHED(c);
-        k_adjt_fwd<<<(unsigned)((g.mesh + 255) / 256), 256, 0, st>>>(g, act, nact, b.AB, b.psi);
-        GX_LAUNCHED(c);
-        k_adj_b<<<nb, ADJ_BS, 0, st>>>(g, b.S, b.L, n, b.psi, g.pmass);
+    }
+    if (nsteps > 0) {
+        k_adj_b<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, b.psi, g.pmass, 0, nullptr, b.drift, c->macc, rng);
         GX_LAUNCHED(c);
     }
     GX_CUDA(c, cudaEventRecord(c->ev1, st));
-    // gradient in load order (x, y, vx, vy)
-    std::vector<float> hl(4 * (size_t)n);
-    GX_CUDA(c, cudaMemcpyAsync(hl.data(), b.L, sbytes, cudaMemcpyDeviceToHost, st));
-    GX_CUDA(c, cudaMemcpyAsync(hp.data(), b.tpart, sizeof(double) * 2 * nb, cudaMemcpyDeviceToHost, st));
+    // gradient in load order (x, y, vx, vy): the records as they are
+    GX_CUDA(c, cudaMemcpyAsync(grad, b.L, sbytes, cudaMemcpyDeviceToHost, st));
+    GX_CUDA(c, cudaMemcpyAsync(hp.data(), b.tpart, sizeof(double) * 2 * np, cudaMemcpyDeviceToHost, st));
     unsigned int hd = 0;
     GX_CUDA(c, cudaMemcpyAsync(&hd, b.drift, sizeof hd, cudaMemcpyDeviceToHost, st));
     GX_CUDA(c, cudaStreamSynchronize(st));
     GX_CUDA(c, cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));
-    for (int64_t i = 0; i < n; i++)
-        for (int k = 0; k < 4; k++) grad[4 * i + k] = hl[(size_t)k * n + i];
     double drc = 0.0, dv2 = 0.0;
-    for (unsigned i = 0; i < nb; i++) {
+    for (unsigned i = 0; i < np; i++) {
         drc += hp[2 * i];
         dv2 += hp[2 * i + 1];
     }

@@ -259,7 +259,7 @@ void gx_destroy(GxCtx* c) {
                     c->items, c->nitems_d, c->rowitem, c->rowcnt, c->rowfill, c->rowbase, c->rowtot, c->rowtile, c->stage, c->jrk_d,
                     c->errword, c->dsum, c->pzone[0], c->pzone[1], c->zbuf, c->zjrk_d, c->act_d,
                     c->bk_cap[0], c->bk_cap[1], c->bk_base[0], c->bk_base[1], c->bk_fill[0], c->bk_fill[1],
-                    c->bk_ctl, c->bk_items, c->bk_cnt, c->macc, c->bq[0], c->bq[1], c->zr_d};
+                    c->bk_ctl, c->bk_items, c->bk_cnt, c->macc, c->bq[0], c->bq[1], c->zr_d, c->adj_ws};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (cudaEvent_t e : c->pev) cudaEventDestroy(e);
@@ -417,6 +417,9 @@ static int alloc_particles(GxCtx* c, int64_t n) {
         c->bq[b] = nullptr;
     }
     c->bucketed = false;
+    if (c->adj_ws) cudaFree(c->adj_ws);
+    c->adj_ws = nullptr;
+    c->adj_bytes = 0;
     int64_t cap = std::max<int64_t>(n, 1);
     c->cap = cap;
     DALLOC(c, c->ppot, cap);

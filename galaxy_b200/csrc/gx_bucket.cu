@@ -916,6 +916,15 @@ static int bk_launch_push(GxCtx* c, int cur, int nxt) {
     return GX_OK;
 }
 
+// the accumulator -> the mass array, its ring and plane ranges; both cleared
+int gx_mass_convert(GxCtx* c) {
+    const DevGeo& g = c->g;
+    k_mass_convert<<<(unsigned)((g.mesh / 2 + 255) / 256), 256, 0, c->stream>>>(
+        c->macc, c->mass, g.mesh, g.pmass, c->bk_ctl + 13, c->jrk_d, g.nr, c->bk_ctl + 10, c->zr_d, g.ngz);
+    GX_LAUNCHED(c);
+    return GX_OK;
+}
+
 // the main stream waits for the plan queued on the side stream
 static int bk_join(GxCtx* c) {
     if (!c->bk_pending) return GX_OK;
@@ -941,9 +950,8 @@ int gx_fast_masset(GxCtx* c) {
     if (rc) return rc;
     // the pass took the items through the work counter: the next pass starts it afresh
     GX_CUDA(c, cudaMemsetAsync(c->bk_ctl + 9, 0, sizeof(int32_t), c->stream));
-    k_mass_convert<<<(unsigned)((g.mesh / 2 + 255) / 256), 256, 0, c->stream>>>(
-        c->macc, c->mass, g.mesh, g.pmass, c->bk_ctl + 13, c->jrk_d, g.nr, c->bk_ctl + 10, c->zr_d, g.ngz);
-    GX_LAUNCHED(c);
+    rc = gx_mass_convert(c);
+    if (rc) return rc;
     c->zr_valid = true;
     return GX_OK;
 }
@@ -982,9 +990,8 @@ static int fast_one_step(GxCtx* c, bool lpot) {
     }
     rc = gx_phase_mark(c, PH_COMBINE);
     if (rc) return rc;
-    k_mass_convert<<<(unsigned)((g.mesh / 2 + 255) / 256), 256, 0, c->stream>>>(
-        c->macc, c->mass, g.mesh, g.pmass, c->bk_ctl + 13, c->jrk_d, g.nr, c->bk_ctl + 10, c->zr_d, g.ngz);
-    GX_LAUNCHED(c);
+    rc = gx_mass_convert(c);
+    if (rc) return rc;
     c->zr_valid = true;
     c->bcur = nxt;
     return GX_OK;

@@ -190,6 +190,9 @@ struct GxCtx {
     cudaEvent_t bk_ev[2] = {nullptr, nullptr};  // push done (main), plan done (side)
     bool bk_pending = false;                 // a plan on bk_side the main stream has not joined
 
+    char* adj_ws = nullptr;                  // buffers of gx_adjoint's sweeps, one block
+    size_t adj_bytes = 0;
+
     // multi-GPU (gx_comm.cu): NCCL communicator of the particle decomposition
     void* comm = nullptr;
     int nranks = 1, rank = 0;
@@ -704,6 +707,7 @@ int gx_fast_step(GxCtx* c, int nsteps, int phys);
 int gx_dense(GxCtx* c);  // bucketed store -> dense store (no-op when dense)
 int gx_bucket_unload(GxCtx* c, float* aos);  // unload from the bucketed store
 int gx_fast_masset(GxCtx* c);  // masset by the deposit-only fused pass
+int gx_mass_convert(GxCtx* c);  // mass accumulator -> mass array (accumulator cleared)
 int gx_bucket_alloc(GxCtx* c);
 int gx_bucket_words(const GxCtx* c);  // float4 words per record of the bucketed store
 int gx_synthesis(GxCtx* c, int tmask, float* polar, const int32_t* frk = nullptr,

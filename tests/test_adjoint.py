@@ -97,3 +97,29 @@ def test_gpu_adjoint_is_deterministic_up_to_fp64_atomics():
     assert J1 == J2
     assert np.linalg.norm(g1 - g2) <= 1e-6 * np.linalg.norm(g1)
     assert np.all(np.abs(t1 - t2) <= 1e-9 * np.abs(t1))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nr,na,ng,n", [(33, 50, 20, 255), (24, 16, 9, 257), (40, 64, 1, 3000),
+                                        (32, 128, 9, 310001)])
+def test_gpu_adjoint_at_the_edges_of_its_tiles(nr, na, ng, n):
+    """More harmonics than one block of the transposed synthesis, the
+    harmonic na / 2, m = 0 alone, a partial last CTA, and more particles than
+    one stride of the passes.  A gradient component's error is that of the
+    cell fractions in FP32 (na / 2 x 6e-8 at most 4e-6 of a weight's slope) and
+    of the FP32 sums: 3e-5 leaves a factor of several, as in the test above."""
+    rec, pm = disc(n, 31)
+    cfg = cfg_adj(nr, na, ng, pm)
+    T = 3
+    J_ref, g_ref, th_ref = ox.adj_gradient(cfg, ox.green(cfg, 64), rec.astype(np.float64), T)
+    with Galaxy(cfg) as gal:
+        gal.greenm()
+        gal.loadup(rec)
+        gal.masset()
+        mass = gal.grid(0)
+        J, grad, dth, _ = gal.adjoint(T, 2)
+        assert np.array_equal(gal.unload(), rec)
+        assert np.array_equal(gal.grid(0), mass)
+    assert abs(J - J_ref) < 1e-6 * J_ref, (J, J_ref)
+    assert np.linalg.norm(grad - g_ref) < 3e-5 * np.linalg.norm(g_ref)
+    assert np.all(np.abs(dth - th_ref) < 1e-4 * np.abs(th_ref)), (dth, th_ref)
