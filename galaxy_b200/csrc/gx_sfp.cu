@@ -31,7 +31,8 @@
 
 #include "gx_common.cuh"
 
-#define SFP_CHUNK 1024  // particles per warp-chunk (FP32 accumulation span)
+#define SFP_CHUNK 1024  // most particles per warp-chunk (FP32 accumulation span)
+#define SFP_CHUNK_MIN 128  // least (the partial rows' memory is sized for it)
 #define SFP_MAXMOM (64 * 48)  // moments: [D][NCP] (D <= 64, NCP <= 32), or the tcgen05 path's raw [64][48]
 
 struct GxSfp {
@@ -51,6 +52,15 @@ struct GxSfp {
     float* xy = nullptr;        // [2][cap]
     float* vel = nullptr;       // [2][cap] velocities of the SFP-driven step
     float4* ftab = nullptr;     // [maxm + 1][SFP_NT] force table of the SFP-driven step
+    double* acheb_d = nullptr;  // [nfun][D] device copy of acheb
+    // the step loop's radial order (sfp_sort): the second buffers of the sort,
+    // the load index of each slot, and the per-block bin counts
+    float *xy_alt = nullptr, *vel_alt = nullptr;
+    int32_t* ord = nullptr;     // [cap] load index of each slot (valid when reordered)
+    int32_t* ord_alt = nullptr;
+    int32_t* bins = nullptr;    // [SRT_BINS][blocks] counts, then offsets; + [SRT_BINS] totals
+    bool reordered = false;
+    int since_sort = 0;         // steps since the last sort
     std::vector<double> qs_h;   // host staging of the force series
     float* part = nullptr;      // per-warp partial moments
     double* mom = nullptr;      // [D][NCP] FP64 moments
@@ -144,7 +154,7 @@ __device__ __forceinline__ void split_h2(float v0, float v1, uint32_t& hi, uint3
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-// Moments of one SFP_CHUNK of particles per warp; part[warp][d][c].
+// Moments of one chunk of particles (at most SFP_CHUNK) per warp; part[warp][d][c].
 // Rounds of 32 particles: lane l computes the features of particle l once --
 // T_d(x) for d < D by the three-term recurrence, and g_n (n >= 1) =
 // p^e cos m phi, p^e sin m phi (e = m mod 2) from repeated multiplication of
@@ -165,11 +175,13 @@ __device__ __forceinline__ void split_h2(float v0, float v1, uint32_t& hi, uint3
 // The recurrences
 // start from sw = 1 for particles inside the basis edge (p <= 1) and 0 for
 // the rest, which makes every feature of an outside particle zero.
-template <int MT, int NB>
+// CHUNK: the particles per warp at compile time, or 0 for the argument's.
+template <int MT, int NB, int CHUNK>
 __global__ void __launch_bounds__(256, MT == 2 ? 3 : 1) k_sfp_moments(const float* __restrict__ X,
                                                      const float* __restrict__ Y, int64_t n,
-                                                     float inv_maxr, int maxm, int NCP,
+                                                     float inv_maxr, int maxm, int NCP, int chunk_arg,
                                                      float* __restrict__ part) {
+    const int chunk = CHUNK ? CHUNK : chunk_arg;
     constexpr int D = MT * 16, TS = D + 8, GS = (NB == 3) ? 40 : 24;
     constexpr int WARP_HALVES = 2 * 32 * (TS + GS);
     static_assert(8 * NB <= GS, "g tile width");
@@ -180,7 +192,7 @@ __global__ void __launch_bounds__(256, MT == 2 ? 3 : 1) k_sfp_moments(const floa
     __half* Gh = Tl + 32 * TS;
     __half* Gl = Gh + 32 * GS;
     const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    const int64_t base = wid * SFP_CHUNK;
+    const int64_t base = wid * chunk;
     if (base >= n) return;
     // ldmatrix row addresses: lane = 8 j + i supplies row i of tile j
     const int li = lane & 7, lj = lane >> 3;
@@ -204,7 +216,7 @@ __global__ void __launch_bounds__(256, MT == 2 ? 3 : 1) k_sfp_moments(const floa
     for (int a = 0; a < MT; a++) run0[a][0] = run0[a][1] = 0.f;
     // B fragment of the column block (1, 0, ..., 0): b = B[2 c4 .. + 1][q], ones at q = 0
     const uint32_t ones[2] = {lane < 4 ? 0x3C003C00u : 0u, lane < 4 ? 0x3C003C00u : 0u};
-    const int64_t end = min(base + (int64_t)SFP_CHUNK, n);
+    const int64_t end = min(base + (int64_t)chunk, n);
     // the coordinates of the next round are loaded one round ahead
     // (raw values: they are scaled where they are used, a round later)
     bool nin = base + lane < end;
@@ -498,14 +510,14 @@ __device__ __forceinline__ void sfp_force(double x, double y, double maxr, int m
 
 __global__ void k_sfp_acc(const float* __restrict__ X, const float* __restrict__ Y, int64_t n,
                           double maxr, int maxm, int D, const double* __restrict__ qs,
-                          float* __restrict__ acc, float* __restrict__ pot) {
+                          const int32_t* __restrict__ ord, float* __restrict__ acc, float* __restrict__ pot) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     double ax, ay, ph;
     sfp_force(X[i], Y[i], maxr, maxm, D, qs, ax, ay, ph);
-    acc[2 * i] = (float)ax;
-    acc[2 * i + 1] = (float)ay;
-    if (pot) pot[i] = (float)ph;
+    const int64_t o = ord ? ord[i] : i;  // load order
+    reinterpret_cast<float2*>(acc)[o] = make_float2((float)ax, (float)ay);
+    if (pot) pot[o] = (float)ph;
 }
 
 // The time loop's force table, as the reference tabulates its basis
@@ -514,29 +526,225 @@ __global__ void k_sfp_acc(const float* __restrict__ X, const float* __restrict__
 // p-derivatives, at SFP_NT radii p_i = i / (SFP_NT - 1), evaluated in FP64
 // from the force series (Clenshaw, as sfp_force) and stored as FP32.
 #define SFP_NT 1025
-__global__ void k_sfp_ftab(int maxm, int D, const double* __restrict__ qs, float4* __restrict__ tab) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (maxm + 1) * SFP_NT) return;
-    const int m = i / SFP_NT, j = i - m * SFP_NT;
+// With the moments on the device the coefficients are formed here too: CTA
+// (m, block of radii) takes the moment columns of its m, forms the
+// coefficients C[n] = fac sum_d a_nmd M[d] of its functions and their series
+// sum_n C[n] a_nmd in FP64 (a few hundred products, repeated by the CTAs of an
+// m), then tabulates.  The loop therefore runs without the host: reading the
+// moments back, forming the coefficients and sending the series took about
+// 60 us a step, this kernel takes 5.1 us.
+struct SfpSel {
+    int minm, maxm, minn, maxn, nsect, D, NCP, raw;
+    double fac;
+};
+
+// moment M[d][c] (c = 0: ones; 2 m - 1, 2 m: cosine, sine) from the summed
+// rows: [D][NCP], or (raw) the tcgen05 path's [64][UM_N] hi/lo products
+__device__ __forceinline__ double sfp_moment(const SfpSel& f, const double* __restrict__ mom, int d, int c) {
+    if (!f.raw) return mom[(size_t)d * f.NCP + c];
+    const double* rh = mom + (size_t)((d & 1) ? 16 + d / 2 : d / 2) * 48;
+    const double* rl = rh + 32 * 48;
+    return c == 0 ? rh[32] + rl[32] : rh[c - 1] + rh[c + 15] + rl[c - 1] + rl[c + 15];
+}
+
+__global__ void __launch_bounds__(128) k_sfp_ftab(SfpSel f, const double* __restrict__ mom,
+                                                  const double* __restrict__ acheb, float4* __restrict__ tab) {
+    __shared__ double M[2][64], C[2][64], q[2][64];
+    const int m = blockIdx.y, D = f.D, nn = f.maxn - f.minn + 1;
+    const bool sel = m >= f.minm && (m - f.minm) % f.nsect == 0;
+    const double* a = acheb + (sel ? (size_t)((m - f.minm) / f.nsect) * nn * D : 0);
+    for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) {
+        const int h = i / D, d = i - h * D;
+        M[h][d] = (sel && (h == 0 || m > 0)) ? sfp_moment(f, mom, d, m == 0 ? 0 : 2 * m - 1 + h) : 0.0;
+    }
+    __syncthreads();
+    // eight lanes per coefficient
+    for (int i0 = 0; i0 < 2 * nn; i0 += blockDim.x / 8) {
+        const int i = i0 + threadIdx.x / 8, l = threadIdx.x & 7, h = i / nn, k = i - h * nn;
+        double v = 0.0;
+        if (sel && i < 2 * nn)
+            for (int d = l; d < D; d += 8) v += a[(size_t)k * D + d] * M[h][d];
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (i < 2 * nn && l == 0) C[h][k] = v * f.fac;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) {
+        const int h = i / D, d = i - h * D;
+        double v = 0.0;
+        if (sel)
+            for (int k = 0; k < nn; k++) v += C[h][k] * a[(size_t)k * D + d];
+        q[h][d] = v;
+    }
+    __syncthreads();
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= SFP_NT) return;
     const double p = (double)j / (double)(SFP_NT - 1), xc = 2.0 * p * p - 1.0;
     double val[2], der[2];
+#pragma unroll
     for (int h = 0; h < 2; h++) {
-        const double* a = qs + ((size_t)h * (maxm + 1) + m) * D;
         double b1 = 0, b2 = 0, d1 = 0, d2 = 0;
         for (int d = D - 1; d >= 1; d--) {
-            const double bn = 2.0 * xc * b1 - b2 + a[d];
+            const double bn = 2.0 * xc * b1 - b2 + q[h][d];
             const double dn = 2.0 * xc * d1 - d2 + 2.0 * b1;
             b2 = b1;
             b1 = bn;
             d2 = d1;
             d1 = dn;
         }
-        val[h] = xc * b1 - b2 + a[0];
+        val[h] = xc * b1 - b2 + q[h][0];
         der[h] = xc * d1 - d2 + b1;
     }
     const double pe = (m & 1) ? p : 1.0, e = (double)(m & 1);
-    tab[i] = make_float4((float)(pe * val[0]), (float)(pe * val[1]), (float)(e * val[0] + pe * der[0] * 4.0 * p),
-                         (float)(e * val[1] + pe * der[1] * 4.0 * p));
+    tab[(size_t)m * SFP_NT + j] =
+        make_float4((float)(pe * val[0]), (float)(pe * val[1]), (float)(e * val[0] + pe * der[0] * 4.0 * p),
+                    (float)(e * val[1] + pe * der[1] * 4.0 * p));
+}
+
+// ---------------------------------------------------------------------------
+// The step loop keeps the particles ordered by radius (SRT_BINS equal bins
+// of p = r / maxr, the last also holding r > maxr): the force of a particle
+// reads 4 consecutive radii of every m's table, so particles of nearby radii
+// in a warp read the same few lines.  In load order each of a warp's 36 loads
+// (maxm = 8) touched up to 32 lines of the first-level cache and the kick of
+// 1M particles took 50.8 us; in radial
+// order it takes 26.7 (the loads' 576 bytes a particle into registers).  A stable
+// counting sort (deterministic: ranks by position, no atomics decide an
+// order), repeated every SRT_EVERY steps as orbits move through the bins,
+// 22.7 us for 1M particles.
+#define SRT_BINS 256
+#define SRT_THREADS 256
+#define SRT_ROUNDS 8                              // 32-particle rounds per warp
+#define SRT_BLOCK (SRT_THREADS * SRT_ROUNDS)      // particles per block
+#define SRT_EVERY 8
+#define SRT_MIN 32768  // fewer particles: the kick is as short as the sort's launches
+
+__device__ __forceinline__ int sfp_bin(float x, float y, float scale) {
+    const float r2 = __fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y));
+    const float b = __fmul_rn(__fsqrt_rn(r2), scale);
+    return b < (float)(SRT_BINS - 1) ? (int)b : SRT_BINS - 1;  // NaN: the last bin
+}
+
+// counts of each bin per block: cnt[bin][block]
+__global__ void __launch_bounds__(SRT_THREADS) k_sfp_count(const float* __restrict__ X, const float* __restrict__ Y,
+                                                           int64_t n, float scale, int nblk,
+                                                           int32_t* __restrict__ cnt) {
+    __shared__ int h[SRT_BINS];
+    static_assert(SRT_BINS == SRT_THREADS, "one bin per thread");
+    h[threadIdx.x] = 0;
+    __syncthreads();
+    const int64_t i0 = (int64_t)blockIdx.x * SRT_BLOCK;
+#pragma unroll
+    for (int k = 0; k < SRT_ROUNDS; k++) {
+        const int64_t i = i0 + k * SRT_THREADS + threadIdx.x;
+        if (i < n) atomicAdd(&h[sfp_bin(X[i], Y[i], scale)], 1);
+    }
+    __syncthreads();
+    cnt[(size_t)threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
+}
+
+// exclusive sums over the blocks of one bin (one CTA per bin), and its total
+__global__ void __launch_bounds__(256) k_sfp_offsets(int nblk, int32_t* __restrict__ cnt, int32_t* __restrict__ tot) {
+    __shared__ int ws[8];
+    int32_t* c = cnt + (size_t)blockIdx.x * nblk;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;
+    for (int b0 = 0; b0 < nblk; b0 += 256) {
+        const int b = b0 + threadIdx.x;
+        const int v = b < nblk ? c[b] : 0;
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        int before = carry, all = 0;
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            before += w < warp ? ws[w] : 0;
+            all += ws[w];
+        }
+        if (b < nblk) c[b] = before + x - v;
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) tot[blockIdx.x] = carry;
+}
+
+// the particles of a block to their slots: warp w ranks its SRT_ROUNDS x 32
+// consecutive particles in order against its own bin counters
+__global__ void __launch_bounds__(SRT_THREADS) k_sfp_reorder(
+    const float* __restrict__ P, const float* __restrict__ V, int64_t n, int64_t cap,
+    const int32_t* __restrict__ oin, float scale, int nblk, const int32_t* __restrict__ cnt,
+    const int32_t* __restrict__ tot, float* __restrict__ P2, float* __restrict__ V2, int32_t* __restrict__ oout) {
+    constexpr int NWP = SRT_THREADS / 32;
+    __shared__ int wc[NWP][SRT_BINS];
+    __shared__ int base[SRT_BINS], ws[NWP];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = threadIdx.x;
+#pragma unroll
+    for (int w = 0; w < NWP; w++) wc[w][t] = 0;
+    // first slot of each bin: exclusive sum of the totals, + this block's offset
+    {
+        const int v = tot[t];
+        int x = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        int before = 0;
+#pragma unroll
+        for (int w = 0; w < NWP; w++) before += w < warp ? ws[w] : 0;
+        base[t] = before + x - v + cnt[(size_t)t * nblk + blockIdx.x];
+    }
+    const int64_t i0 = (int64_t)blockIdx.x * SRT_BLOCK + (int64_t)warp * SRT_ROUNDS * 32 + lane;
+    float x[SRT_ROUNDS], y[SRT_ROUNDS];
+    int bin[SRT_ROUNDS], rank[SRT_ROUNDS];
+#pragma unroll
+    for (int k = 0; k < SRT_ROUNDS; k++) {
+        const int64_t i = i0 + 32 * k;
+        x[k] = i < n ? P[i] : 0.f;
+        y[k] = i < n ? P[cap + i] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < SRT_ROUNDS; k++) {
+        const bool act = i0 + 32 * k < n;
+        bin[k] = sfp_bin(x[k], y[k], scale);
+        const uint32_t am = __ballot_sync(0xffffffffu, act);
+        const uint32_t peers = __match_any_sync(0xffffffffu, bin[k]) & am;
+        const int c = act ? wc[warp][bin[k]] : 0;
+        rank[k] = c + __popc(peers & lanemask_lt());
+        __syncwarp();
+        if (act && (peers & lanemask_lt()) == 0) wc[warp][bin[k]] = c + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    // each warp's counters -> the first slot of its particles of every bin
+    {
+        int run = base[t];
+#pragma unroll
+        for (int w = 0; w < NWP; w++) {
+            const int v = wc[w][t];
+            wc[w][t] = run;
+            run += v;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < SRT_ROUNDS; k++) {
+        const int64_t i = i0 + 32 * k;
+        if (i >= n) continue;
+        const int64_t d = wc[warp][bin[k]] + rank[k];
+        P2[d] = x[k];
+        P2[cap + d] = y[k];
+        V2[d] = V[i];
+        V2[cap + d] = V[cap + i];
+        oout[d] = oin ? oin[i] : (int32_t)i;
+    }
 }
 
 // one leapfrog step in the SFP field (stpgrp.f:26-32 with the time step
@@ -562,6 +770,7 @@ __global__ void k_sfp_kick(float* __restrict__ X, float* __restrict__ Y, float* 
         const float w2 = -t * (t - 1.f) * (t - 3.f) * 0.5f;
         const float w3 = t * (t - 1.f) * (t - 2.f) * (1.f / 6.f);
         float ar = 0.f, at = 0.f, cm = 1.f, sm = 0.f;
+#pragma unroll 3
         for (int m = 0; m <= maxm; m++) {
             if (m > 0) {
                 const float nc = cm * c1 - sm * s1;
@@ -655,7 +864,8 @@ extern "C" void gx_sfp_destroy(GxSfp* s) {
     if (!s) return;
     cudaSetDevice(s->dev);
     if (s->stream) cudaStreamSynchronize(s->stream);
-    void* p[] = {s->xy, s->vel, s->ftab, s->part, s->mom, s->qc, s->upart, s->slab, s->errword};
+    void* p[] = {s->xy, s->vel, s->ftab, s->part, s->mom, s->qc, s->upart, s->slab, s->errword,
+                 s->acheb_d, s->xy_alt, s->vel_alt, s->ord, s->ord_alt, s->bins};
     for (void* q : p)
         if (q) cudaFree(q);
     if (s->e0) cudaEventDestroy(s->e0);
@@ -678,12 +888,12 @@ __global__ void k_sfp_xy(const float* __restrict__ aos, int stride, int64_t n, i
     vel[cap + i] = stride >= 4 ? aos[i * stride + 3] : 0.f;
 }
 
-// SoA -> records (x, y, vx, vy)
+// SoA -> records (x, y, vx, vy) in load order
 __global__ void k_sfp_unxy(const float* __restrict__ xy, const float* __restrict__ vel, int64_t n, int64_t cap,
-                           float4* __restrict__ aos) {
+                           const int32_t* __restrict__ ord, float4* __restrict__ aos) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    aos[i] = make_float4(xy[i], xy[cap + i], vel[i], vel[cap + i]);
+    aos[ord ? ord[i] : i] = make_float4(xy[i], xy[cap + i], vel[i], vel[cap + i]);
 }
 
 extern "C" int gx_sfp_load(GxSfp* s, const float* coords, int64_t n, int stride) {
@@ -696,15 +906,22 @@ extern "C" int gx_sfp_load(GxSfp* s, const float* coords, int64_t n, int stride)
         s->xy = nullptr;
         s->vel = nullptr;
         s->part = nullptr;
+        void* old[] = {s->xy_alt, s->vel_alt, s->ord, s->ord_alt, s->bins};
+        for (void* q : old)
+            if (q) cudaFree(q);
+        s->xy_alt = s->vel_alt = nullptr;
+        s->ord = s->ord_alt = s->bins = nullptr;
         s->cap = std::max<int64_t>(n, 1);
         SFP_CUDA(s, cudaMalloc((void**)&s->xy, sizeof(float) * 2 * s->cap));
         SFP_CUDA(s, cudaMalloc((void**)&s->vel, sizeof(float) * 2 * s->cap));
-        const int64_t nw = (s->cap + SFP_CHUNK - 1) / SFP_CHUNK;
+        const int64_t nw = (s->cap + SFP_CHUNK_MIN - 1) / SFP_CHUNK_MIN;
         const int64_t nb = (s->cap + 255) / 256;
         const size_t bytes = std::max(sizeof(float) * nw * 64 * 32, sizeof(double) * nb * 64 * 32);
         SFP_CUDA(s, cudaMalloc((void**)&s->part, bytes));
     }
     s->n = n;
+    s->reordered = false;
+    s->since_sort = 0;
     if (n == 0) return GX_OK;
     float* tmp = nullptr;
     SFP_CUDA(s, cudaMallocAsync((void**)&tmp, sizeof(float) * stride * n, s->stream));
@@ -1067,6 +1284,14 @@ static int sfp_sum_rows(GxSfp* s, const T* part, int64_t nrow, int nmom) {
     return GX_OK;
 }
 
+template <int CHUNK>
+static auto sfp_moments_kernel(int D, int NB) {
+    return (D == 32) ? ((NB <= 1) ? k_sfp_moments<2, 1, CHUNK> : (NB == 2) ? k_sfp_moments<2, 2, CHUNK>
+                                                                           : k_sfp_moments<2, 3, CHUNK>)
+                     : ((NB <= 1) ? k_sfp_moments<4, 1, CHUNK> : (NB == 2) ? k_sfp_moments<4, 2, CHUNK>
+                                                                           : k_sfp_moments<4, 3, CHUNK>);
+}
+
 // moments on the device (precision GX_PREC_MIXED: tensor cores; GX_PREC_FP64: CUDA cores)
 static int sfp_moments(GxSfp* s, int precision) {
     const int D = s->D, NCP = (s->NC + 7) / 8 * 8, nmom = D * NCP;
@@ -1097,19 +1322,35 @@ static int sfp_moments(GxSfp* s, int precision) {
         s->launches += 1;
         return sfp_sum_rows<double>(s, s->upart, grid, UM_NRAW);
     }
-    const int64_t nw = (n + SFP_CHUNK - 1) / SFP_CHUNK;
+    // particles per warp: the full chunk when that fills the chip (24 resident
+    // warps per SM), else as many fewer (a multiple of the 32-particle round)
+    // as it takes to fill it once; 1M particles: 27.8 us with chunks of 1024
+    // (122 CTAs of 8 warps), 23.3 with 288
+    const int64_t fill = (int64_t)s->nsm * 24;
+    const int chunk = (int)std::min<int64_t>(SFP_CHUNK, std::max<int64_t>(SFP_CHUNK_MIN, (n / fill + 32) / 32 * 32));
+    const int64_t nw = (n + chunk - 1) / chunk;
     const unsigned grid = (unsigned)((nw * 32 + 255) / 256);
     // feature columns 1 .. NC - 1 in blocks of 8
     const int NB = (s->NC - 1 + 7) / 8;
     if (NB > 3) return s->err = "more than 11 harmonics on the tensor-core path", GX_ERR_RANGE;
     const size_t sm = sizeof(__half) * 8 * 2 * 32 * ((size_t)(D + 8) + (NB == 3 ? 40 : 24));
-    auto k = (D == 32) ? ((NB <= 1) ? k_sfp_moments<2, 1> : (NB == 2) ? k_sfp_moments<2, 2> : k_sfp_moments<2, 3>)
-                       : ((NB <= 1) ? k_sfp_moments<4, 1> : (NB == 2) ? k_sfp_moments<4, 2> : k_sfp_moments<4, 3>);
+    auto k = (chunk == SFP_CHUNK) ? sfp_moments_kernel<SFP_CHUNK>(D, NB) : sfp_moments_kernel<0>(D, NB);
     SFP_CUDA(s, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k<<<grid, 256, sm, s->stream>>>(s->xy, s->xy + s->cap, n, inv, s->b.maxm, NCP, s->part);
+    k<<<grid, 256, sm, s->stream>>>(s->xy, s->xy + s->cap, n, inv, s->b.maxm, NCP, chunk, s->part);
     SFP_CUDA(s, cudaGetLastError());
     s->launches += 1;
     return sfp_sum_rows<float>(s, s->part, nw, nmom);
+}
+
+// the device error word (bounded waits of the tcgen05 path), cleared
+static int sfp_check(GxSfp* s) {
+    int32_t ew = 0;
+    SFP_CUDA(s, cudaMemcpy(&ew, s->errword, sizeof ew, cudaMemcpyDeviceToHost));
+    if (ew) {
+        cudaMemset(s->errword, 0, sizeof ew);
+        return s->err = "device check raised the error word", GX_ERR_DEVICE;
+    }
+    return GX_OK;
 }
 
 // sfpsum + scaled: coeff[n * (2 maxm + 1) + m + maxm] (cosine +m, sine -m)
@@ -1144,12 +1385,8 @@ static int sfp_coeff(GxSfp* s, int precision, double pmass, double* coeff) {
     }
     SFP_CUDA(s, cudaEventElapsedTime(&s->last_ms, s->e0, s->e1));
     {
-        int32_t ew = 0;
-        SFP_CUDA(s, cudaMemcpy(&ew, s->errword, sizeof ew, cudaMemcpyDeviceToHost));
-        if (ew) {
-            cudaMemset(s->errword, 0, sizeof ew);
-            return s->err = "device check raised the error word", GX_ERR_DEVICE;
-        }
+        const int rc = sfp_check(s);
+        if (rc) return rc;
     }
     memset(coeff, 0, sizeof(double) * (size_t)(s->b.maxn + 1) * ngx);
     const double fac = pmass / (s->maxr * s->maxr);
@@ -1212,7 +1449,8 @@ extern "C" int gx_sfp_acc(GxSfp* s, const double* coeff, float* acc, float* pot)
         SFP_CUDA(s, cudaMallocAsync((void**)&dacc, sizeof(float) * 2 * n, s->stream));
         SFP_CUDA(s, cudaMallocAsync((void**)&dpot, sizeof(float) * n, s->stream));
         k_sfp_acc<<<(unsigned)((n + 127) / 128), 128, 0, s->stream>>>(s->xy, s->xy + s->cap, n, s->maxr,
-                                                                    maxm, D, s->qc, dacc, dpot);
+                                                                    maxm, D, s->qc,
+                                                                    s->reordered ? s->ord : nullptr, dacc, dpot);
         SFP_CUDA(s, cudaGetLastError());
         SFP_CUDA(s, cudaMemcpyAsync(acc, dacc, sizeof(float) * 2 * n, cudaMemcpyDeviceToHost, s->stream));
         if (pot) SFP_CUDA(s, cudaMemcpyAsync(pot, dpot, sizeof(float) * n, cudaMemcpyDeviceToHost, s->stream));
@@ -1223,42 +1461,80 @@ extern "C" int gx_sfp_acc(GxSfp* s, const double* coeff, float* acc, float* pot)
     return GX_OK;
 }
 
+// the particles into radial order (see k_sfp_count); the buffers stay with
+// the loaded particles
+static int sfp_sort(GxSfp* s) {
+    const int64_t n = s->n;
+    const int nblk = (int)((n + SRT_BLOCK - 1) / SRT_BLOCK);
+    const int cblk = (int)((s->cap + SRT_BLOCK - 1) / SRT_BLOCK);
+    if (!s->xy_alt) SFP_CUDA(s, cudaMalloc((void**)&s->xy_alt, sizeof(float) * 2 * s->cap));
+    if (!s->vel_alt) SFP_CUDA(s, cudaMalloc((void**)&s->vel_alt, sizeof(float) * 2 * s->cap));
+    if (!s->ord) SFP_CUDA(s, cudaMalloc((void**)&s->ord, sizeof(int32_t) * s->cap));
+    if (!s->ord_alt) SFP_CUDA(s, cudaMalloc((void**)&s->ord_alt, sizeof(int32_t) * s->cap));
+    if (!s->bins) SFP_CUDA(s, cudaMalloc((void**)&s->bins, sizeof(int32_t) * SRT_BINS * ((size_t)cblk + 1)));
+    int32_t* tot = s->bins + (size_t)SRT_BINS * nblk;
+    const float scale = (float)((double)(SRT_BINS - 1) / s->maxr);
+    k_sfp_count<<<nblk, SRT_THREADS, 0, s->stream>>>(s->xy, s->xy + s->cap, n, scale, nblk, s->bins);
+    SFP_CUDA(s, cudaGetLastError());
+    k_sfp_offsets<<<SRT_BINS, 256, 0, s->stream>>>(nblk, s->bins, tot);
+    SFP_CUDA(s, cudaGetLastError());
+    k_sfp_reorder<<<nblk, SRT_THREADS, 0, s->stream>>>(s->xy, s->vel, n, s->cap, s->reordered ? s->ord : nullptr,
+                                                       scale, nblk, s->bins, tot, s->xy_alt, s->vel_alt,
+                                                       s->ord_alt);
+    SFP_CUDA(s, cudaGetLastError());
+    std::swap(s->xy, s->xy_alt);
+    std::swap(s->vel, s->vel_alt);
+    std::swap(s->ord, s->ord_alt);
+    s->reordered = true;
+    s->since_sort = 0;
+    return GX_OK;
+}
+
 // The SFP-driven time loop (the sf2d code's step, step.f:135-290: getacc
 // -> sfpacc, stpgrp, massgn -> sfpadd, then sfpsum at step.f:250): per
-// step the coefficients of the current positions (gx_sfp_sum's arithmetic
-// at `precision`), then one kernel that evaluates the force at each
-// particle and moves it, v += a dt, x += v dt.  The particles stay on the
-// device; coeff_out (may be NULL) receives the coefficients of the final
-// positions.
+// step the moments of the current positions (gx_sfp_sum's arithmetic
+// at `precision`), the coefficients and the force table (k_sfp_ftab), then
+// one kernel that evaluates the force at each particle and moves it, v += a
+// dt, x += v dt; nothing waits on the host between steps.  The particles stay
+// on the device; coeff_out (may be NULL) receives the coefficients of the
+// final positions.
 extern "C" int gx_sfp_step(GxSfp* s, int nsteps, double dt, int precision, double pmass, double* coeff_out) {
     if (!s || nsteps < 0) return GX_ERR_ARG;
     if (precision != GX_PREC_MIXED && precision != GX_PREC_FP64 && precision != GX_PREC_MIXED_TC05)
         return GX_ERR_ARG;
     cudaSetDevice(s->dev);
-    const int ngx = 2 * s->b.maxm + 1;
-    std::vector<double> coeff((size_t)(s->b.maxn + 1) * ngx);
     const int64_t n = s->n;
     if (!s->ftab) SFP_CUDA(s, cudaMalloc((void**)&s->ftab, sizeof(float4) * 12 * SFP_NT));
-    for (int k = 0; k < nsteps; k++) {
-        int rc = sfp_coeff(s, precision, pmass, coeff.data());
+    if (!s->acheb_d) {
+        SFP_CUDA(s, cudaMalloc((void**)&s->acheb_d, sizeof(double) * s->acheb.size()));
+        SFP_CUDA(s, cudaMemcpyAsync(s->acheb_d, s->acheb.data(), sizeof(double) * s->acheb.size(),
+                                    cudaMemcpyHostToDevice, s->stream));
+    }
+    const SfpSel f = {s->b.minm, s->b.maxm, s->b.minn, s->b.maxn, s->b.nsect, s->D, (s->NC + 7) / 8 * 8,
+                      precision == GX_PREC_MIXED_TC05, pmass / (s->maxr * s->maxr)};
+    for (int k = 0; k < nsteps && n > 0; k++) {
+        int rc = GX_OK;
+        if (n >= SRT_MIN && (!s->reordered || s->since_sort >= SRT_EVERY)) rc = sfp_sort(s);
         if (rc) return rc;
-        rc = sfp_series(s, coeff.data());
+        rc = sfp_moments(s, precision);
         if (rc) return rc;
-        if (n > 0) {
-            const int nt = (s->b.maxm + 1) * SFP_NT;
-            k_sfp_ftab<<<(unsigned)((nt + 127) / 128), 128, 0, s->stream>>>(s->b.maxm, s->D, s->qc, s->ftab);
-            SFP_CUDA(s, cudaGetLastError());
-            k_sfp_kick<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
-                s->xy, s->xy + s->cap, s->vel, s->vel + s->cap, n, (float)s->maxr, s->b.maxm, s->ftab, (float)dt);
-            SFP_CUDA(s, cudaGetLastError());
-        }
+        k_sfp_ftab<<<dim3((SFP_NT + 127) / 128, s->b.maxm + 1), 128, 0, s->stream>>>(f, s->mom, s->acheb_d, s->ftab);
+        SFP_CUDA(s, cudaGetLastError());
+        k_sfp_kick<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
+            s->xy, s->xy + s->cap, s->vel, s->vel + s->cap, n, (float)s->maxr, s->b.maxm, s->ftab, (float)dt);
+        SFP_CUDA(s, cudaGetLastError());
+        s->since_sort++;
     }
     if (coeff_out) {
-        int rc = sfp_coeff(s, precision, pmass, coeff_out);
+        // (also waits for the steps and reads the error word)
+        std::vector<double> coeff((size_t)(s->b.maxn + 1) * (2 * s->b.maxm + 1));
+        int rc = sfp_coeff(s, precision, pmass, coeff.data());
         if (rc) return rc;
+        std::copy(coeff.begin(), coeff.end(), coeff_out);
+        return GX_OK;
     }
     SFP_CUDA(s, cudaStreamSynchronize(s->stream));
-    return GX_OK;
+    return sfp_check(s);
 }
 
 // the loaded particles back as records (x, y, vx, vy)
@@ -1269,7 +1545,8 @@ extern "C" int gx_sfp_unload(GxSfp* s, float* coords) {
     if (n == 0) return GX_OK;
     float4* tmp = nullptr;
     SFP_CUDA(s, cudaMallocAsync((void**)&tmp, sizeof(float4) * n, s->stream));
-    k_sfp_unxy<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->xy, s->vel, n, s->cap, tmp);
+    k_sfp_unxy<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(s->xy, s->vel, n, s->cap,
+                                                                     s->reordered ? s->ord : nullptr, tmp);
     SFP_CUDA(s, cudaGetLastError());
     SFP_CUDA(s, cudaMemcpyAsync(coords, tmp, sizeof(float4) * n, cudaMemcpyDeviceToHost, s->stream));
     SFP_CUDA(s, cudaFreeAsync(tmp, s->stream));

@@ -164,3 +164,40 @@ def test_sfp_sum_64_chebyshev_terms(basis):
     e64 = np.linalg.norm(c64 - ref) / np.linalg.norm(ref)
     assert e64 < 1e-7, e64
     assert e32 < 1e-6, e32
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [32768, 40001])
+def test_sfp_step_in_radial_order_tracks_oracle(basis, n):
+    """Enough particles for the loop to keep them in radial order: 18 steps
+    (the order renewed twice), some particles outside the basis edge and one
+    at the centre.  Records, forces and coefficients come back in load order;
+    the bounds are those of the unordered loop above."""
+    from galaxy_b200.sfp import Sfp
+    nsteps, dt, maxr = 18, 0.05, 6.0
+    pm = 1.0 / n
+    rng = np.random.default_rng(n)
+    rec = np.zeros((n, 4), np.float32)
+    rec[:, :2] = exp_disk(n, seed=23)
+    rec[::997, :2] *= 3.0
+    rec[5] = 0.0
+    rec[:, 2:] = 0.4 * rng.standard_normal((n, 2))
+    x, v = rec[:, :2].astype(np.float64), rec[:, 2:].astype(np.float64)
+    for _ in range(nsteps):
+        a, _ = ox.sfp_acc(basis, ox.sfp_coeffs(basis, x, maxr, pmass=pm), x, maxr)
+        v = v + a * dt
+        x = x + v * dt
+    c_ref = ox.sfp_coeffs(basis, x, maxr, pmass=pm)
+    with Sfp(basis, maxr) as s:
+        s.load(rec)
+        s.step(5, dt, pmass=pm)
+        c = s.step(nsteps - 5, dt, pmass=pm)
+        out = s.unload()
+        acc, _ = s.acc(c)
+        s.load(out)
+        acc2, _ = s.acc(c)
+    assert np.array_equal(acc, acc2)
+    ok = np.hypot(x[:, 0], x[:, 1]) < 0.99 * maxr  # the force jumps to zero at the edge
+    far = np.abs(out[:, :2] - x).max(axis=1) / np.abs(x).max()
+    assert np.mean(far > 1e-5) < 2e-3 and far[ok].max() < 1e-3, far.max()
+    assert np.linalg.norm(c - c_ref) < 1e-4 * np.linalg.norm(c_ref)
