@@ -1,6 +1,6 @@
 // gx_ensemble.cu -- an ensemble of independent 2D discs on one polar grid
-// geometry, advanced together: one persistent cooperative launch per step,
-// the launches of a batch of steps replayed from a CUDA graph.
+// geometry, advanced together by persistent cooperative launches of up to
+// ENS_MAXSTEPS steps each.
 //
 // Each disc is the run the single-disc path makes of it (SRC/progs/galaxy.f
 // time loop: findf, getacc + stpgrp, massgn): same cell keys and weights
@@ -10,24 +10,39 @@
 // synthesis arithmetic (p2manl.f:32-45, p2conv.f:99-187, p2fsyn.f:34-56,
 // polcat.f:22-41) with FP32 sums, the m = 0 forward sum in FP64.
 //
-// One step launch:
-//   solve   CTA d (d < ndisc, strided) turns disc d's integer mass into its
-//           (fx, fy) field grid: forward DFT of the active harmonics per
-//           ring, radial contraction with the shared Green table (read from
-//           L2), synthesis + polcat; it then zeroes the integer mass and
-//           publishes the field with a ready flag (the launch's epoch).
-//   push    every CTA takes chunks of particles (one disc each); it waits
-//           (bounded) for the disc's ready flag, stages the disc's field in
-//           shared memory, and for each particle interpolates (grdacc),
-//           kicks and drifts (stpgrp), and deposits the new position into a
-//           shared-memory copy of the disc's integer mass grid, flushed
-//           with integer atomics (order-free, deterministic).  The particle
-//           sums of the m = 2 amplitude go to a per-chunk slot.
-//   close   the last CTA to finish sums the chunk slots of every disc in
-//           chunk order (deterministic FP64) into the A2 series and
-//           advances the step counter.
+// One launch:
+//   solve   turns a disc's integer mass into its (fx, fy) field grid: forward
+//           DFT of the active harmonics per ring, radial contraction with the
+//           shared Green table (read from L2), synthesis + polcat; it then
+//           zeroes the integer mass and publishes the field with the disc's
+//           ready flag (the step's epoch).  The first solves of a launch are
+//           dealt over the CTAs; the later ones are made by the CTA that
+//           flushed the last chunk of the disc's previous step, so that no
+//           disc waits for another and one disc's solve runs beside the
+//           others' particles.
+//   push    every CTA takes its chunks of particles (one disc each), step by
+//           step; it waits (bounded) for the disc's ready flag, stages the
+//           disc's field in shared memory, and for each particle interpolates
+//           (grdacc), kicks and drifts (stpgrp), and deposits the new position
+//           into shared-memory bins over the disc's mesh, flushed with integer
+//           atomics (order-free, deterministic).  The particle sums of the m =
+//           2 amplitude go to a per-chunk slot; the CTA that completes the
+//           disc's step sums them in chunk order (deterministic FP64) into the
+//           A2 series.
+// The waits end: all CTAs are resident, each takes its (step, chunk) pairs in
+// order, and the solve of a disc's step is made by the CTA that completes the
+// step before it, inside that step's work.
 // The deposit-only launch (mode 0) makes the initial mass (masset) and A2 at
 // step 0.
+//
+// What bounds the pass: shared-memory atomics and instruction issue.  The
+// bins are unsigned 32-bit words (native shared-memory atomics; 64-bit ones
+// are compare-and-swap loops): a word that wraps adds 2^32 to the cell in the
+// mesh, and a negative weight goes straight to the mesh, so the flushed
+// integers are the exact 64-bit sums.  Half the bins' size also lets two CTAs
+// share an SM when the grid is small enough.  16 discs, 2M particles on 64 x
+// 128: 87.0 us a step with one launch per step, 64-bit bins and the solves
+// before the pushes, 60.1 so.
 #include <algorithm>
 #include <vector>
 
@@ -37,6 +52,7 @@
 #define ENS_MAXACT 64
 #define ENS_SPIN (1u << 24)
 #define ENS_TUNE_REPS 3
+#define ENS_MAXSTEPS 64  // steps per launch
 // series entries past max_steps that the tuner's trial steps may write
 #define ENS_SPARE (2 + ENS_TUNE_REPS + 1)
 
@@ -56,14 +72,12 @@ struct GxEnsemble {
     int32_t* dchunk = nullptr;           // [ndisc + 1] first chunk of each disc
     double* a2part = nullptr;            // [nchunks][3]: sum cos 2phi, sum sin 2phi, count
     double* series = nullptr;            // [max_steps + ENS_SPARE][ndisc][2]
-    uint32_t* ctl = nullptr;             // [0] entries recorded, [1] CTAs done, [2 + d] ready epoch
+    uint32_t* ctl = nullptr;             // [0] entries recorded, [1] CTAs done, [2 + d] ready epoch,
+                                         // [2 + ndisc + d] chunks done of the disc's current step
     float* tw = nullptr;                 // twiddle tables (ens_tables)
     // tuning and launch
     int threads = 512, chunk = 16384, nchunks = 0, grid = 0, nchunks_cap = 0;
     size_t smem = 0;
-    cudaGraphExec_t gexec = nullptr;
-    int gsteps = 0;
-    bool use_graph = true;
     float last_ms = 0.f;
     int64_t launches = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -118,98 +132,184 @@ __global__ void k_ens_tables(DevGeo g, int nact, const int* __restrict__ mlist, 
 }
 
 // ---------------------------------------------------------------------------
-// field solve of disc d by the whole CTA (p2fndf.f:25-66 with polcat)
+// field solve of disc d by the whole CTA (p2fndf.f:25-66 with polcat).  The
+// sums of each output run in the same order on any number of threads; the
+// threads share operands instead: a forward thread takes ENS_FH harmonics of
+// one ring, a contraction thread both components, a synthesis thread two
+// rings, which cuts the shared-memory reads that bounded each phase.
+#define ENS_FH 3
+struct __align__(16) EnsTw {
+    float2 f[4];  // (cos, -sin) of harmonics ENS_FH g .. + 2 (one unused)
+};
+
+// floats of the solve's workspace: M, forward twiddles [groups][na][8], S, O
+__host__ __device__ __forceinline__ size_t ens_solve_floats(int nr, int na, int nact) {
+    const size_t ng = (nact + ENS_FH - 1) / ENS_FH;
+    return (((size_t)nr * (na + 1) + 3) & ~(size_t)3) + ng * na * 8 + 2 * (size_t)nact * nr + 4 * (size_t)nact * nr;
+}
+
 __device__ void ens_solve(const EnsArgs& A, int d, float* sm) {
     const DevGeo& g = A.g;
     const int nr = g.nr, na = g.na, nact = A.nact, mesh = g.mesh;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int ldm = na + 1;
     const size_t pl = (size_t)nact * na;
-    float* M = sm;                                   // [nr][na + 1]
-    float* Tw = M + (size_t)nr * ldm;                // [4][nact][na]
-    // float2 arrays start on a 16-byte boundary
-    float2* S = reinterpret_cast<float2*>(M + ((nr * ldm + 4 * pl + 3) & ~(size_t)3));  // [nact][nr]: (a_m, b_m)
-    float2* O = S + (size_t)nact * nr;               // [2][nact][nr]: (W_c, W_s) of fr, ftheta
+    const int ngr = (nact + ENS_FH - 1) / ENS_FH;
+    float* M = sm;                                                               // [nr][na + 1]
+    EnsTw* Tw = reinterpret_cast<EnsTw*>(M + (((size_t)nr * ldm + 3) & ~(size_t)3));  // [ngr][na]
+    float2* S = reinterpret_cast<float2*>(Tw + (size_t)ngr * na);                // [nact][nr]: (a_m, b_m)
+    float4* O = reinterpret_cast<float4*>(S + (size_t)nact * nr + ((nact * nr) & 1));  // [nact][nr]: (W_c, W_s) of fr, ftheta
     unsigned long long* m64 = A.mass64 + (size_t)d * mesh;
     const float pmass = A.pm[d];
     // integer mass -> FP32 x pmass (scaled.f:89-92); the integers are cleared
-    // for the deposit of this step
-    for (int i = threadIdx.x; i < mesh; i += blockDim.x) {
-        const long long v = (long long)m64[i];
-        m64[i] = 0ull;
-        M[(i / na) * ldm + (i % na)] = (float)((double)v * (1.0 / (double)ENS_FIXQ)) * pmass;
+    // for the deposit of this step.  Read past the first-level cache: other
+    // SMs' atomics made them.
+    for (int ir = warp; ir < nr; ir += nw) {
+#pragma unroll 4
+        for (int j = 2 * lane; j < na; j += 64) {
+            ulonglong2* q = reinterpret_cast<ulonglong2*>(m64 + (size_t)ir * na + j);
+            const ulonglong2 v = __ldcg(q);
+            *q = make_ulonglong2(0ull, 0ull);
+            M[ir * ldm + j] = (float)((double)(long long)v.x * (1.0 / (double)ENS_FIXQ)) * pmass;
+            M[ir * ldm + j + 1] = (float)((double)(long long)v.y * (1.0 / (double)ENS_FIXQ)) * pmass;
+        }
     }
-    for (int i = threadIdx.x; i < 4 * (int)pl; i += blockDim.x) Tw[i] = A.tw[i];
+    for (int i = threadIdx.x; i < ngr * na; i += blockDim.x) {
+        const int gq = i / na, j = i - gq * na;
+        EnsTw t;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int a = gq * ENS_FH + k;
+            t.f[k] = (k < ENS_FH && a < nact) ? make_float2(__ldg(A.tw + (size_t)a * na + j), __ldg(A.tw + pl + (size_t)a * na + j))
+                                              : make_float2(0.f, 0.f);
+        }
+        Tw[i] = t;
+    }
     __syncthreads();
     // forward transform per ring (p2manl.f:32-45): a_m = sum x cos, b_m = -sum x sin
-    for (int o = threadIdx.x; o < nact * nr; o += blockDim.x) {
-        const int a = o / nr, ir = o - a * nr;
-        const float* row = M + (size_t)ir * ldm;
-        float2 r;
-        if (A.act_m[a] == 0) {
-            double s = 0.0;
-            for (int j = 0; j < na; j++) s += (double)row[j];
-            r = make_float2((float)s, 0.f);
-        } else {
-            const float* tc = Tw + (size_t)a * na;
-            const float* ts = Tw + pl + (size_t)a * na;
-            float ca = 0.f, sa = 0.f;
-            for (int j = 0; j < na; j++) {
-                ca = fmaf(row[j], tc[j], ca);
-                sa = fmaf(row[j], ts[j], sa);
+    {
+        // groups of harmonics, then the FP64 sums of m = 0 (in spoke order)
+        const int n0 = A.act_m[0] == 0 ? nr : 0;
+        const int ng32 = (ngr * nr + 31) & ~31;
+        for (int o = threadIdx.x; o < ng32 + n0; o += blockDim.x) {
+            if (o >= ng32) {
+                const int ir = o - ng32;
+                const float* row = M + (size_t)ir * ldm;
+                double s = 0.0;
+#pragma unroll 8
+                for (int j = 0; j < na; j++) s += (double)row[j];
+                S[ir] = make_float2((float)s, 0.f);
+            } else if (o < ngr * nr) {
+                const int gq = o / nr, ir = o - gq * nr;
+                const float* row = M + (size_t)ir * ldm;
+                const EnsTw* t = Tw + (size_t)gq * na;
+                float ca[ENS_FH], sa[ENS_FH];
+#pragma unroll
+                for (int k = 0; k < ENS_FH; k++) ca[k] = sa[k] = 0.f;
+#pragma unroll 4
+                for (int j = 0; j < na; j++) {
+                    const float x = row[j];
+#pragma unroll
+                    for (int k = 0; k < ENS_FH; k++) {
+                        ca[k] = fmaf(x, t[j].f[k].x, ca[k]);
+                        sa[k] = fmaf(x, t[j].f[k].y, sa[k]);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < ENS_FH; k++) {
+                    const int a = gq * ENS_FH + k;
+                    if (a < nact && A.act_m[a] != 0) S[(size_t)a * nr + ir] = make_float2(ca[k], sa[k]);
+                }
             }
-            r = make_float2(ca, sa);
         }
-        S[o] = r;
     }
     __syncthreads();
     // radial contraction (p2conv.f:114-181): fr uses (G.M_c, G.M_s), ftheta
     // (+G.M_s, -G.M_c); Green rows of source ring is, columns of field ring ir
-    for (int o = threadIdx.x; o < 2 * nact * nr; o += blockDim.x) {
-        const int t = o / (nact * nr), rem = o - t * nact * nr, a = rem / nr, ir = rem - a * nr;
+    for (int o = threadIdx.x; o < nact * nr; o += blockDim.x) {
+        const int a = o / nr, ir = o - a * nr;
         const int m = A.act_m[a];
-        float2 w = make_float2(0.f, 0.f);
-        const bool valid = ((A.tmask >> t) & 1) && (t == 0 || ((m >= 1) && (m <= min(g.ng, g.mmax - 1) - 1)));
-        if (valid) {
-            const float* G = A.green + (((size_t)t * g.ng + m) * g.nkz) * nr * (size_t)nr + ir;
-            const float2* Sa = S + (size_t)a * nr;
-            float wc = 0.f, ws = 0.f;
+        const bool v0 = (A.tmask & 1) != 0;
+        const bool v1 = ((A.tmask >> 1) & 1) && (m >= 1) && (m <= min(g.ng, g.mmax - 1) - 1);
+        const float* G0 = A.green + ((size_t)m * g.nkz) * nr * (size_t)nr + ir;
+        const float* G1 = A.green + (((size_t)g.ng + m) * g.nkz) * nr * (size_t)nr + ir;
+        const float2* Sa = S + (size_t)a * nr;
+        float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+        float wc = 0.f, ws = 0.f;
+        if (v0 && v1) {
+            // both tables' loads in flight together
+#pragma unroll 8
+            for (int is = 0; is < nr; is++) {
+                const float g0 = __ldg(G0 + (size_t)is * nr), g1 = __ldg(G1 + (size_t)is * nr);
+                const float2 sv = Sa[is];
+                w.x = fmaf(g0, sv.x, w.x);
+                w.y = fmaf(g0, sv.y, w.y);
+                wc = fmaf(g1, sv.x, wc);
+                ws = fmaf(g1, sv.y, ws);
+            }
+        } else if (v0 || v1) {
+            const float* G = v0 ? G0 : G1;
+            float c0 = 0.f, s0 = 0.f;
+#pragma unroll 8
             for (int is = 0; is < nr; is++) {
                 const float gv = __ldg(G + (size_t)is * nr);
                 const float2 sv = Sa[is];
-                wc = fmaf(gv, sv.x, wc);
-                ws = fmaf(gv, sv.y, ws);
+                c0 = fmaf(gv, sv.x, c0);
+                s0 = fmaf(gv, sv.y, s0);
             }
-            w = (t == 0) ? make_float2(wc, ws) : make_float2(ws, -wc);
+            if (v0) {
+                w.x = c0;
+                w.y = s0;
+            } else {
+                wc = c0;
+                ws = s0;
+            }
+        }
+        if (v1) {
+            w.z = ws;
+            w.w = -wc;
         }
         O[o] = w;
     }
     __syncthreads();
     // synthesis (p2fsyn.f:34-56, 1/na) and polcat (polcat.f:22-41):
-    // f(j) = C + S, f(na - j) = C - S
-    const float* TC = Tw + 2 * pl;
-    const float* TS = Tw + 3 * pl;
-    const int half = na / 2, nj = half + 1;
+    // f(j) = C + S, f(na - j) = C - S; a warp takes two rings, its lanes spokes
+    const float* TC = A.tw + 2 * pl;
+    const float* TS = A.tw + 3 * pl;
+    const int half = na / 2, nj = half + 1, njb = (nj + 31) >> 5, nrp = (nr + 1) >> 1;
     float2* F = A.field + (size_t)d * mesh;
-    for (int o = threadIdx.x; o < nr * nj; o += blockDim.x) {
-        const int ir = o / nj, j = o - ir * nj;
-        float c0 = 0.f, s0 = 0.f, c1 = 0.f, s1 = 0.f;
+    for (int o = warp; o < njb * nrp; o += nw) {
+        const int jb = o / nrp, ip = o - jb * nrp, j = jb * 32 + lane;
+        const int i0 = 2 * ip, i1 = min(2 * ip + 1, nr - 1);
+        if (j >= nj) continue;
+        float c[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, sn2[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 3
         for (int a = 0; a < nact; a++) {
-            const float tc = TC[(size_t)a * na + j], ts = TS[(size_t)a * na + j];
-            const float2 w0 = O[(size_t)a * nr + ir], w1 = O[(size_t)(nact + a) * nr + ir];
-            c0 = fmaf(w0.x, tc, c0);
-            s0 = fmaf(w0.y, ts, s0);
-            c1 = fmaf(w1.x, tc, c1);
-            s1 = fmaf(w1.y, ts, s1);
+            const float tc = __ldg(TC + (size_t)a * na + j), ts = __ldg(TS + (size_t)a * na + j);
+            const float4 w0 = O[(size_t)a * nr + i0], w1 = O[(size_t)a * nr + i1];
+            c[0][0] = fmaf(w0.x, tc, c[0][0]);
+            sn2[0][0] = fmaf(w0.y, ts, sn2[0][0]);
+            c[0][1] = fmaf(w0.z, tc, c[0][1]);
+            sn2[0][1] = fmaf(w0.w, ts, sn2[0][1]);
+            c[1][0] = fmaf(w1.x, tc, c[1][0]);
+            sn2[1][0] = fmaf(w1.y, ts, sn2[1][0]);
+            c[1][1] = fmaf(w1.z, tc, c[1][1]);
+            sn2[1][1] = fmaf(w1.w, ts, sn2[1][1]);
         }
         float sn, cs;
         sincospif(2.0f * (float)j / (float)na, &sn, &cs);
-        {
-            const float fr = c0 + s0, ft = c1 + s1;
-            F[(size_t)ir * na + j] = make_float2(fr * cs - ft * sn, fr * sn + ft * cs);
-        }
-        if (j > 0 && j < half) {
-            const float fr = c0 - s0, ft = c1 - s1;
-            F[(size_t)ir * na + (na - j)] = make_float2(fr * cs + ft * sn, -fr * sn + ft * cs);
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int ir = 2 * ip + u;
+            if (ir >= nr) continue;
+            {
+                const float fr = c[u][0] + sn2[u][0], ft = c[u][1] + sn2[u][1];
+                F[(size_t)ir * na + j] = make_float2(fr * cs - ft * sn, fr * sn + ft * cs);
+            }
+            if (j > 0 && j < half) {
+                const float fr = c[u][0] - sn2[u][0], ft = c[u][1] - sn2[u][1];
+                F[(size_t)ir * na + (na - j)] = make_float2(fr * cs + ft * sn, -fr * sn + ft * cs);
+            }
         }
     }
 }
@@ -224,188 +324,231 @@ __device__ __forceinline__ void ens_st_release(uint32_t* p, uint32_t v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// mode 0: deposit at the current positions (masset) and A2; mode 1: one step
-__global__ void __launch_bounds__(1024) k_ens_step(EnsArgs A) {
+// the field of disc d for the step of epoch e, by the whole CTA
+__device__ __forceinline__ void ens_publish(const EnsArgs& A, int d, uint32_t e, unsigned char* sm) {
+    ens_solve(A, d, reinterpret_cast<float*>(sm));
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        ens_st_release(&A.ctl[2 + d], e);
+    }
+    __syncthreads();
+}
+
+// mode 0: deposit at the current positions (masset) and A2; mode 1: nsteps steps
+template <int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) k_ens_step(EnsArgs A, int nsteps) {
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ uint32_t s_epoch;
     __shared__ int s_last;
-    __shared__ double red[3][32];
+    __shared__ double red[2][32];
+    __shared__ int redn[32];
     const DevGeo& g = A.g;
     const int mesh = g.mesh;
     if (threadIdx.x == 0) s_epoch = ens_ld_acquire(&A.ctl[0]) + 1u;
     __syncthreads();
-    const uint32_t epoch = s_epoch;
+    const uint32_t epoch0 = s_epoch;
 
-    // ---- field solve of the discs of this CTA, each published by its flag
-    if (A.mode == 1) {
-        for (int d = blockIdx.x; d < A.ndisc; d += gridDim.x) {
-            ens_solve(A, d, reinterpret_cast<float*>(smraw));
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                ens_st_release(&A.ctl[2 + d], epoch);
-            }
-            __syncthreads();
-        }
-    }
+    // ---- the first step's field solves
+    if (A.mode == 1)
+        for (int d = blockIdx.x; d < A.ndisc; d += gridDim.x) ens_publish(A, d, epoch0, smraw);
 
-    // ---- particle chunks
-    float2* F = reinterpret_cast<float2*>(smraw);                              // [mesh]
-    unsigned long long* bins = reinterpret_cast<unsigned long long*>(F + mesh);  // [mesh]
+    // ---- particle chunks, step by step
+    float2* F = reinterpret_cast<float2*>(smraw);          // [mesh]
+    uint32_t* bins = reinterpret_cast<uint32_t*>(F + mesh);  // [mesh]
+    bool clean = false;  // the bins are zero
     float* X = A.P;
     float* Y = A.P + A.ntot;
     float* VX = A.P + 2 * A.ntot;
     float* VY = A.P + 3 * A.ntot;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c = blockIdx.x; c < A.nchunks; c += gridDim.x) {
-        const int d = A.chunks[3 * c], s0 = A.chunks[3 * c + 1], s1 = A.chunks[3 * c + 2];
-        if (A.mode == 1) {
-            if (threadIdx.x == 0) {
-                uint32_t it = 0;
-                while (ens_ld_acquire(&A.ctl[2 + d]) != epoch) {
-                    if (++it > ENS_SPIN) {
-                        atomicExch(A.errword, 4);
-                        break;
+    for (int k = 0; k < nsteps; k++) {
+        const uint32_t epoch = epoch0 + (uint32_t)k;
+        for (int c = blockIdx.x; c < A.nchunks; c += gridDim.x) {
+            const int d = A.chunks[3 * c], s0 = A.chunks[3 * c + 1], s1 = A.chunks[3 * c + 2];
+            unsigned long long* m64 = A.mass64 + (size_t)d * mesh;
+            if (!clean)
+                for (int i = threadIdx.x; i < mesh; i += blockDim.x) bins[i] = 0u;
+            if (A.mode == 1) {
+                if (threadIdx.x == 0) {
+                    uint32_t it = 0;
+                    while ((int32_t)(ens_ld_acquire(&A.ctl[2 + d]) - epoch) < 0) {
+                        if (++it > ENS_SPIN) {
+                            atomicExch(A.errword, 4);
+                            break;
+                        }
+                        __nanosleep(100);
                     }
-                    __nanosleep(100);
+                }
+                __syncthreads();
+                const float4* src = reinterpret_cast<const float4*>(A.field + (size_t)d * mesh);
+#pragma unroll 4
+                for (int i = threadIdx.x; i < mesh / 2; i += blockDim.x)
+                    reinterpret_cast<float4*>(F)[i] = __ldcg(src + i);
+            }
+            __syncthreads();
+            double sc = 0.0, ss = 0.0;
+            int sn = 0;
+            for (int p = s0 + threadIdx.x; p < s1; p += blockDim.x) {
+                float x = X[p], y = Y[p];
+                if (A.mode == 1) {
+                    float vx = VX[p], vy = VY[p];
+                    // grdacc.f:40-84 at the old position, halo (frhalo.f:55-56);
+                    // the interpolation cell from the fast FP32 arithmetic, as the
+                    // single-disc pass forms it (the field is continuous across a
+                    // cell boundary, so a cell off by rounding changes nothing)
+                    const CellW cw = gx_cell_t<false, 2>(g, x, y, 0.f, true);
+                    float ax = 0.f, ay = 0.f;
+                    if (cw.key >= 0) {
+                        float w[8];
+                        int ic[8];
+                        gx_weights<2>(g, cw, w);
+                        gx_corners_rt<2>(g, cw.key, cw.jt, ic);
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            if (ic[q] < 0) continue;
+                            const float2 f = F[ic[q]];
+                            ax += f.x * w[q];
+                            ay += f.y * w[q];
+                        }
+                    }
+                    if (g.halo == 1 && cw.key >= 0) {
+                        const float r2 = x * x + y * y;
+                        const float rr = sqrtf(r2);
+                        float fr = -g.halo_v2 * rr / (r2 + g.halo_rc2);
+                        if (fr != 0.f) {
+                            fr = fr / rr;
+                            ax += fr * x;
+                            ay += fr * y;
+                        }
+                    } else if (g.halo == 2 && cw.key >= 0) {
+                        float az_ = 0.f, ph_ = 0.f;
+                        gx_disc_force(g, x, y, 0.f, ax, ay, az_, ph_);
+                    }
+                    // stpgrp.f:26-32
+                    vx += ax;
+                    vy += ay;
+                    x += vx;
+                    y += vy;
+                    X[p] = x;
+                    Y[p] = y;
+                    VX[p] = vx;
+                    VY[p] = vy;
+                }
+                // massgn.f:68-89 at the new position
+                const CellW cn = gx_cell_t<true, 2>(g, x, y, 0.f, false);
+                if (cn.key >= 0) {
+                    float w[8];
+                    int ic[8];
+                    gx_weights<2>(g, cn, w);
+                    gx_corners_rt<2>(g, cn.key, cn.jt, ic);
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        if (ic[q] >= 0) {
+                            // round(w 2^20), ties to even, by one FMA with 1.5 2^23
+                            const int v = __float_as_int(fmaf(w[q], ENS_FIXQ, 12582912.0f)) - 0x4B400000;
+                            if (v >= 0) {
+                                const uint32_t o = atomicAdd(&bins[ic[q]], (uint32_t)v);
+                                if (o + (uint32_t)v < o) atomicAdd(&m64[ic[q]], 1ull << 32);  // the word wrapped
+                            } else {
+                                atomicAdd(&m64[ic[q]], (unsigned long long)(long long)v);
+                            }
+                        }
+                    const double xd = x, yd = y, r2 = xd * xd + yd * yd;
+                    if (r2 > 0.0) {
+                        const double inv = 1.0 / r2;
+                        sc += (xd * xd - yd * yd) * inv;
+                        ss += 2.0 * xd * yd * inv;
+                    }
+                    sn++;
+                }
+            }
+            // chunk sums of the m = 2 amplitude (fixed order: deterministic)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                sc += __shfl_down_sync(0xffffffffu, sc, o);
+                ss += __shfl_down_sync(0xffffffffu, ss, o);
+                sn += __shfl_down_sync(0xffffffffu, sn, o);
+            }
+            if (lane == 0) {
+                red[0][warp] = sc;
+                red[1][warp] = ss;
+                redn[warp] = sn;
+            }
+            __syncthreads();
+            // flush the chunk's integer mass (integer atomics: order-free)
+            for (int i = threadIdx.x; i < mesh; i += blockDim.x) {
+                const uint32_t v = bins[i];
+                if (v) {
+                    atomicAdd(&m64[i], (unsigned long long)v);
+                    bins[i] = 0u;
+                }
+            }
+            clean = true;
+            if (threadIdx.x == 0) {
+                double a = 0.0, b = 0.0, n = 0.0;
+                for (int w = 0; w < nw; w++) {
+                    a += red[0][w];
+                    b += red[1][w];
+                    n += (double)redn[w];
+                }
+                A.a2part[3 * c] = a;
+                A.a2part[3 * c + 1] = b;
+                A.a2part[3 * c + 2] = n;
+            }
+            __syncthreads();
+            // the CTA that completes the disc's step records its A2 and makes
+            // its next field
+            if (threadIdx.x == 0) {
+                __threadfence();
+                const int nc = A.dchunk[d + 1] - A.dchunk[d];
+                const uint32_t prev = atomicAdd(&A.ctl[2 + A.ndisc + d], 1u);
+                s_last = (prev == (uint32_t)nc - 1u) ? 1 : 0;
+                if (s_last) {
+                    __threadfence();
+                    A.ctl[2 + A.ndisc + d] = 0u;
                 }
             }
             __syncthreads();
-            const float4* src = reinterpret_cast<const float4*>(A.field + (size_t)d * mesh);
-            for (int i = threadIdx.x; i < mesh / 2; i += blockDim.x)
-                reinterpret_cast<float4*>(F)[i] = __ldcg(src + i);
-        }
-        for (int i = threadIdx.x; i < mesh; i += blockDim.x) bins[i] = 0ull;
-        __syncthreads();
-        double sc = 0.0, ss = 0.0, sn = 0.0;
-        for (int p = s0 + threadIdx.x; p < s1; p += blockDim.x) {
-            float x = X[p], y = Y[p];
-            if (A.mode == 1) {
-                float vx = VX[p], vy = VY[p];
-                // grdacc.f:40-84 at the old position, halo (frhalo.f:55-56);
-                // the interpolation cell from the fast FP32 arithmetic, as the
-                // single-disc pass forms it (the field is continuous across a
-                // cell boundary, so a cell off by rounding changes nothing)
-                const CellW cw = gx_cell_t<false, 2>(g, x, y, 0.f, true);
-                float ax = 0.f, ay = 0.f;
-                if (cw.key >= 0) {
-                    float w[8];
-                    int ic[8];
-                    gx_weights(g, cw, w);
-                    gx_corners(g, cw.key, ic);
-#pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (ic[k] < 0) continue;
-                        const float2 f = F[ic[k]];
-                        ax += f.x * w[k];
-                        ay += f.y * w[k];
+            if (s_last) {
+                if (threadIdx.x < 32) {
+                    // the chunk slots loaded by a warp, added in chunk order
+                    double a = 0.0, b = 0.0, n = 0.0;
+                    const int q1 = A.dchunk[d + 1];
+                    for (int q0 = A.dchunk[d]; q0 < q1; q0 += 32) {
+                        const int q = q0 + lane;
+                        const double pa = q < q1 ? __ldcg(&A.a2part[3 * q]) : 0.0;
+                        const double pb = q < q1 ? __ldcg(&A.a2part[3 * q + 1]) : 0.0;
+                        const double pn = q < q1 ? __ldcg(&A.a2part[3 * q + 2]) : 0.0;
+                        for (int u = 0; u < min(32, q1 - q0); u++) {
+                            a += __shfl_sync(0xffffffffu, pa, u);
+                            b += __shfl_sync(0xffffffffu, pb, u);
+                            n += __shfl_sync(0xffffffffu, pn, u);
+                        }
+                    }
+                    if (lane == 0) {
+                        double* out = A.series + ((size_t)(epoch - 1) * A.ndisc + d) * 2;
+                        out[0] = (n > 0.0) ? a / n : 0.0;
+                        out[1] = (n > 0.0) ? b / n : 0.0;
                     }
                 }
-                if (g.halo == 1 && cw.key >= 0) {
-                    const float r2 = x * x + y * y;
-                    const float rr = sqrtf(r2);
-                    float fr = -g.halo_v2 * rr / (r2 + g.halo_rc2);
-                    if (fr != 0.f) {
-                        fr = fr / rr;
-                        ax += fr * x;
-                        ay += fr * y;
-                    }
-                } else if (g.halo == 2 && cw.key >= 0) {
-                    float az_ = 0.f, ph_ = 0.f;
-                    gx_disc_force(g, x, y, 0.f, ax, ay, az_, ph_);
+                if (k + 1 < nsteps) {
+                    ens_publish(A, d, epoch + 1u, smraw);
+                    clean = false;
                 }
-                // stpgrp.f:26-32
-                vx += ax;
-                vy += ay;
-                x += vx;
-                y += vy;
-                X[p] = x;
-                Y[p] = y;
-                VX[p] = vx;
-                VY[p] = vy;
-            }
-            // massgn.f:68-89 at the new position
-            const CellW cn = gx_cell(g, x, y, 0.f, false);
-            if (cn.key >= 0) {
-                float w[8];
-                int ic[8];
-                gx_weights(g, cn, w);
-                gx_corners(g, cn.key, ic);
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (ic[k] >= 0) {
-                        // round(w 2^20), ties to even, by one FMA with 1.5 2^23
-                        const int v = __float_as_int(fmaf(w[k], ENS_FIXQ, 12582912.0f)) - 0x4B400000;
-                        atomicAdd(&bins[ic[k]], (unsigned long long)(long long)v);
-                    }
-                const double xd = x, yd = y, r2 = xd * xd + yd * yd;
-                if (r2 > 0.0) {
-                    const double inv = 1.0 / r2;
-                    sc += (xd * xd - yd * yd) * inv;
-                    ss += 2.0 * xd * yd * inv;
-                }
-                sn += 1.0;
             }
         }
-        // chunk sums of the m = 2 amplitude (fixed order: deterministic)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            sc += __shfl_down_sync(0xffffffffu, sc, o);
-            ss += __shfl_down_sync(0xffffffffu, ss, o);
-            sn += __shfl_down_sync(0xffffffffu, sn, o);
-        }
-        if (lane == 0) {
-            red[0][warp] = sc;
-            red[1][warp] = ss;
-            red[2][warp] = sn;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0.0, b = 0.0, n = 0.0;
-            for (int w = 0; w < nw; w++) {
-                a += red[0][w];
-                b += red[1][w];
-                n += red[2][w];
-            }
-            A.a2part[3 * c] = a;
-            A.a2part[3 * c + 1] = b;
-            A.a2part[3 * c + 2] = n;
-        }
-        // flush the chunk's integer mass (integer atomics: order-free)
-        unsigned long long* m64 = A.mass64 + (size_t)d * mesh;
-        for (int i = threadIdx.x; i < mesh; i += blockDim.x) {
-            const unsigned long long v = bins[i];
-            if (v) atomicAdd(&m64[i], v);
-        }
-        __syncthreads();
     }
 
-    // ---- the last CTA to finish records the A2 series entry
+    // ---- the last CTA to finish records the steps
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
         const uint32_t prev = atomicAdd(&A.ctl[1], 1u);
-        s_last = (prev == gridDim.x - 1) ? 1 : 0;
-    }
-    __syncthreads();
-    if (s_last) {
-        __threadfence();
-        double* out = A.series + (size_t)(epoch - 1) * A.ndisc * 2;
-        for (int d = threadIdx.x; d < A.ndisc; d += blockDim.x) {
-            double a = 0.0, b = 0.0, n = 0.0;
-            for (int c = A.dchunk[d]; c < A.dchunk[d + 1]; c++) {
-                a += __ldcg(&A.a2part[3 * c]);
-                b += __ldcg(&A.a2part[3 * c + 1]);
-                n += __ldcg(&A.a2part[3 * c + 2]);
-            }
-            out[2 * d] = (n > 0.0) ? a / n : 0.0;
-            out[2 * d + 1] = (n > 0.0) ? b / n : 0.0;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
+        if (prev == gridDim.x - 1) {
             A.ctl[1] = 0u;
             __threadfence();
-            ens_st_release(&A.ctl[0], epoch);
+            ens_st_release(&A.ctl[0], epoch0 + (uint32_t)nsteps - 1u);
         }
     }
 }
@@ -432,6 +575,12 @@ __global__ void k_ens_soa_to_aos(const float* __restrict__ P, float* __restrict_
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     for (int k = 0; k < 4; k++) aos[4 * i + k] = P[k * n + i];
+}
+
+// the kernel of a block size: 1024 threads take the SM alone, smaller blocks
+// share it with the same 64 registers a thread
+static const void* ens_kernel(int threads) {
+    return threads > 512 ? (const void*)k_ens_step<1024, 1> : (const void*)k_ens_step<512, 2>;
 }
 
 // chunk table for the current chunk size, launch geometry for the current
@@ -469,22 +618,16 @@ static int ens_configure(GxEnsemble* e, int threads, int chunk) {
     e->threads = threads;
     e->chunk = chunk;
     const DevGeo& g = c->g;
-    const size_t pl = (size_t)c->spec.nact * g.na;
-    const size_t solve = sizeof(float) * (((size_t)g.nr * (g.na + 1) + 4 * pl + 3) & ~(size_t)3) +
-                         sizeof(float2) * 3 * (size_t)c->spec.nact * g.nr;
-    const size_t push = (sizeof(float2) + sizeof(unsigned long long)) * (size_t)g.mesh;
+    const size_t solve = sizeof(float) * (ens_solve_floats(g.nr, g.na, c->spec.nact) + 4);
+    const size_t push = (sizeof(float2) + sizeof(uint32_t)) * (size_t)g.mesh;
     e->smem = std::max(solve, push);
-    ENS_CUDA(e, cudaFuncSetAttribute(k_ens_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem));
     int per_sm = 0, sms = 0;
-    ENS_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ens_step, threads, e->smem));
+    const void* kern = ens_kernel(threads);
+    ENS_CUDA(e, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e->smem));
+    ENS_CUDA(e, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, e->smem));
     ENS_CUDA(e, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
     if (per_sm < 1) return e->err = "ensemble step kernel does not fit on an SM", GX_ERR_RANGE;
     e->grid = per_sm * sms;
-    if (e->gexec) {
-        cudaGraphExecDestroy(e->gexec);
-        e->gexec = nullptr;
-        e->gsteps = 0;
-    }
     return GX_OK;
 }
 
@@ -514,20 +657,13 @@ static EnsArgs ens_args(GxEnsemble* e, int mode) {
     return A;
 }
 
-// one cooperative launch (all CTAs resident: the flag waits always end)
-static int ens_launch(GxEnsemble* e, int mode) {
+// one cooperative launch of nsteps steps (all CTAs resident: the flag waits
+// always end)
+static int ens_launch(GxEnsemble* e, int mode, int nsteps = 1) {
     EnsArgs A = ens_args(e, mode);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)e->grid);
-    cfg.blockDim = dim3((unsigned)e->threads);
-    cfg.dynamicSmemBytes = e->smem;
-    cfg.stream = e->ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    ENS_CUDA(e, cudaLaunchKernelEx(&cfg, k_ens_step, A));
+    void* args[] = {&A, &nsteps};
+    ENS_CUDA(e, cudaLaunchCooperativeKernel(ens_kernel(e->threads), dim3((unsigned)e->grid), dim3((unsigned)e->threads),
+                                            args, e->smem, e->ctx->stream));
     e->launches++;
     return GX_OK;
 }
@@ -552,7 +688,6 @@ void gx_ensemble_destroy(GxEnsemble* e) {
         cudaSetDevice(e->ctx->dev);
         cudaStreamSynchronize(e->ctx->stream);
     }
-    if (e->gexec) cudaGraphExecDestroy(e->gexec);
     void* ptrs[] = {e->P, e->pm, e->mass64, e->field, e->chunks, e->dchunk, e->a2part, e->series, e->ctl, e->tw};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -630,13 +765,13 @@ int gx_ensemble_create(const GxConfig* cfg, int ndisc, const int64_t* counts, co
         ENS_CUDA(e, cudaMalloc((void**)&e->field, sizeof(float2) * ndisc * (size_t)g.mesh));
         ENS_CUDA(e, cudaMalloc((void**)&e->dchunk, sizeof(int32_t) * (ndisc + 1)));
         ENS_CUDA(e, cudaMalloc((void**)&e->series, sizeof(double) * 2 * ndisc * ((size_t)max_steps + ENS_SPARE)));
-        ENS_CUDA(e, cudaMalloc((void**)&e->ctl, sizeof(uint32_t) * (2 + ndisc)));
+        ENS_CUDA(e, cudaMalloc((void**)&e->ctl, sizeof(uint32_t) * (2 + 2 * (size_t)ndisc)));
         ENS_CUDA(e, cudaMalloc((void**)&e->tw, sizeof(float) * 4 * (size_t)c->spec.nact * g.na));
         ENS_CUDA(e, cudaEventCreate(&e->ev0));
         ENS_CUDA(e, cudaEventCreate(&e->ev1));
         ENS_CUDA(e, cudaMemcpyAsync(e->pm, pmass, sizeof(float) * ndisc, cudaMemcpyHostToDevice, st));
         ENS_CUDA(e, cudaMemsetAsync(e->mass64, 0, sizeof(unsigned long long) * ndisc * (size_t)g.mesh, st));
-        ENS_CUDA(e, cudaMemsetAsync(e->ctl, 0, sizeof(uint32_t) * (2 + ndisc), st));
+        ENS_CUDA(e, cudaMemsetAsync(e->ctl, 0, sizeof(uint32_t) * (2 + 2 * (size_t)ndisc), st));
         ENS_CUDA(e, cudaMemsetAsync(e->series, 0, sizeof(double) * 2 * ndisc * ((size_t)max_steps + ENS_SPARE), st));
         int* mlist = nullptr;
         ENS_CUDA(e, cudaMallocAsync((void**)&mlist, sizeof(int) * c->spec.nact, st));
@@ -671,9 +806,7 @@ int gx_ensemble_create(const GxConfig* cfg, int ndisc, const int64_t* counts, co
     return GX_OK;
 }
 
-// nsteps steps; the launches of a batch of steps are captured once into a
-// CUDA graph and replayed (when capture of the cooperative launch is
-// refused, the steps are launched directly and use_graph turns off)
+// nsteps steps in launches of at most ENS_MAXSTEPS
 int gx_ensemble_step(GxEnsemble* e, int nsteps) {
     if (!e || nsteps < 0) return GX_ERR_ARG;
     if (e->steps_done + nsteps > e->max_steps) return e->err = "more steps than max_steps", GX_ERR_RANGE;
@@ -682,48 +815,8 @@ int gx_ensemble_step(GxEnsemble* e, int nsteps) {
     cudaStream_t st = c->stream;
     e->launches = 0;
     ENS_CUDA(e, cudaEventRecord(e->ev0, st));
-    int left = nsteps;
-    const int G = 16;
-    if (e->use_graph && left >= G) {
-        if (!e->gexec || e->gsteps != G) {
-            if (e->gexec) cudaGraphExecDestroy(e->gexec);
-            e->gexec = nullptr;
-            cudaGraph_t graph = nullptr;
-            bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
-            for (int k = 0; ok && k < G; k++) {
-                EnsArgs A = ens_args(e, 1);
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3((unsigned)e->grid);
-                cfg.blockDim = dim3((unsigned)e->threads);
-                cfg.dynamicSmemBytes = e->smem;
-                cfg.stream = st;
-                cudaLaunchAttribute at[1];
-                at[0].id = cudaLaunchAttributeCooperative;
-                at[0].val.cooperative = 1;
-                cfg.attrs = at;
-                cfg.numAttrs = 1;
-                ok = cudaLaunchKernelEx(&cfg, k_ens_step, A) == cudaSuccess;
-            }
-            cudaError_t ec = cudaStreamEndCapture(st, &graph);
-            ok = ok && ec == cudaSuccess && graph;
-            if (ok) ok = cudaGraphInstantiate(&e->gexec, graph, 0) == cudaSuccess;
-            if (graph) cudaGraphDestroy(graph);
-            cudaGetLastError();
-            if (ok) {
-                e->gsteps = G;
-            } else {
-                e->gexec = nullptr;
-                e->use_graph = false;
-            }
-        }
-        while (e->gexec && left >= G) {
-            ENS_CUDA(e, cudaGraphLaunch(e->gexec, st));
-            e->launches += G;
-            left -= G;
-        }
-    }
-    for (; left > 0; left--) {
-        int rc = ens_launch(e, 1);
+    for (int left = nsteps; left > 0; left -= ENS_MAXSTEPS) {
+        int rc = ens_launch(e, 1, std::min(left, ENS_MAXSTEPS));
         if (rc) return rc;
     }
     ENS_CUDA(e, cudaEventRecord(e->ev1, st));
@@ -743,7 +836,7 @@ int gx_ensemble_tune(GxEnsemble* e, int* threads_out, int* chunk_out) {
     const DevGeo& g = c->g;
     const size_t pbytes = sizeof(float) * 4 * std::max<int64_t>(e->ntot, 1);
     const size_t mbytes = sizeof(unsigned long long) * e->ndisc * (size_t)g.mesh;
-    const size_t cbytes = sizeof(uint32_t) * (2 + e->ndisc);
+    const size_t cbytes = sizeof(uint32_t) * (2 + 2 * (size_t)e->ndisc);
     char *sp = nullptr, *sm = nullptr, *sc = nullptr;
     ENS_CUDA(e, cudaMalloc((void**)&sp, pbytes));
     ENS_CUDA(e, cudaMalloc((void**)&sm, mbytes));
@@ -767,7 +860,7 @@ int gx_ensemble_tune(GxEnsemble* e, int* threads_out, int* chunk_out) {
             rc = ens_launch(e, 1);
             if (rc) break;
             ENS_CUDA(e, cudaEventRecord(e->ev0, st));
-            for (int r = 0; r < reps && rc == GX_OK; r++) rc = ens_launch(e, 1);
+            rc = ens_launch(e, 1, reps);
             ENS_CUDA(e, cudaEventRecord(e->ev1, st));
             if (rc) break;
             ENS_CUDA(e, cudaEventSynchronize(e->ev1));
@@ -800,7 +893,7 @@ int gx_ensemble_config(const GxEnsemble* e, int* threads, int* chunk, int* grid,
     if (threads) *threads = e->threads;
     if (chunk) *chunk = e->chunk;
     if (grid) *grid = e->grid;
-    if (graph) *graph = e->use_graph ? 1 : 0;
+    if (graph) *graph = 0;
     return GX_OK;
 }
 
