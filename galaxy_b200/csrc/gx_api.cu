@@ -257,7 +257,7 @@ void gx_destroy(GxCtx* c) {
                     c->pacc, c->mass, c->mass64, c->field, c->polar, c->field64, c->polar64,
                     c->specS, c->specO, c->syntab, c->synR, c->fwdtab, c->fwdC1, c->spec64, c->out64, c->az64, c->rows64, c->pot64, c->stagebuf, c->perm_next, c->rowstart,
                     c->items, c->nitems_d, c->rowitem, c->rowcnt, c->rowfill, c->rowbase, c->rowtot, c->rowtile, c->stage, c->jrk_d,
-                    c->errword, c->dsum, c->pzone[0], c->pzone[1], c->zbuf, c->zjrk_d, c->act_d,
+                    c->errword, c->dsum, c->pzone[0], c->pzone[1], c->zbuf, c->zacc, c->zjrk_d, c->act_d,
                     c->bk_cap[0], c->bk_cap[1], c->bk_base[0], c->bk_base[1], c->bk_fill[0], c->bk_fill[1],
                     c->bk_ctl, c->bk_items, c->bk_cnt, c->macc, c->bq[0], c->bq[1], c->zr_d, c->adj_ws};
     for (void* p : ptrs)

@@ -155,8 +155,10 @@ struct GxCtx {
     float* zbuf = nullptr;                   // [2][nzones][mesh] mass arrays of zones 2..nzones
     float* znew[GX_MAX_ZONES] = {};          // newest array of each zone (index >= 1)
     float* zold[GX_MAX_ZONES] = {};          // the one before it
+    unsigned long long* zacc = nullptr;      // [nzones - 1][mesh] accumulators of zones 2..nzones (zone 1: macc)
     int32_t* zjrk_d = nullptr;               // [GX_MAX_ZONES][2] ring range of each zone's mass,
-                                             // then [2] the field rings of the next partial solve
+                                             // then [2] the field rings of the next partial solve,
+                                             // then [GX_MAX_ZONES][2] the rings of the accumulated deposits
     int istep = 0;                           // step counter of the zone schedule
     int lstep[GX_MAX_ZONES][2] = {};         // step numbers of zold, znew
     bool zones_ready = false;                // zone arrays deposited (gx_masset)

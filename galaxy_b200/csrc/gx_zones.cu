@@ -21,11 +21,14 @@
 //                          times pmass
 //   p2fndf.f:25-33         the source ring range over all zones
 //
-// Here the particle pass of a step (k_push_zone) moves the particles of the
-// active zones in one launch and copies the others through; the deposit
-// runs once per active zone through the deterministic counting-sort
-// deposit (gx_deposit.cu) filtered by zone code, into that zone's array;
-// k_zone_combine forms the solve's mass.  The solve always covers the
+// Here the particle pass of a step (k_zone_push) moves the particles of the
+// active zones in place and adds their weights, as the 2^-20 integers of
+// gx_deposit.cu, straight into their zone's int64 accumulator; k_zone_mix
+// turns the moved zones' accumulators into their arrays and forms the solve's
+// mass.  Runs of more than ZONE_DIRECT particles keep them sorted by row
+// instead (k_push_zone, which copies the others through, then per active zone
+// the counting-sort deposit of gx_deposit.cu filtered by zone code, and
+// k_zone_combine): the same integers, converted the same way.  The solve always covers the
 // whole grid (findf.f:41-54 allows the reference a partial grid when only
 // inner zones move; the forces at the moving particles are the same).
 #include <algorithm>
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(256) k_push_zone(
     int64_t cap, int64_t n, const int32_t* __restrict__ perm, const int32_t* __restrict__ orig_in,
     int32_t* __restrict__ orig_out, const float4* __restrict__ F, const int32_t* __restrict__ key_in,
     int32_t* __restrict__ key_out, float* __restrict__ fr_out, const int32_t* __restrict__ zone_in,
-    int32_t* __restrict__ zone_out, float* __restrict__ pot) {
+    int32_t* __restrict__ zone_out) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int p = perm[s];
@@ -144,11 +147,10 @@ __global__ void __launch_bounds__(256) k_push_zone(
     orig_out[s] = orig_in[p];
     const bool moves = z0 <= mzone || (z0 == off && mzone == nz);
     float a[3] = {0.f, 0.f, 0.f}, ph = 0.f;
-    if (z0 != off && (moves || pot)) {
+    if (z0 != off && moves) {
         const CellW cw = gx_cell(g, q[0], q[1], z, true);
         gx_accel_cell(g, F, cw, q[0], q[1], z, a[0], a[1], a[2], ph);
     }
-    if (pot) pot[s] = ph;
     if (!moves) {
         for (int k = 0; k < nw; k++) Pout[k * cap + s] = q[k];
         key_out[s] = key_in[p];
@@ -201,6 +203,28 @@ struct ZoneSrc {
     int n;
 };
 
+// the source ring range over the zones and the field rings of a partial-grid
+// solve in which zones 1..mz move (one thread)
+__device__ __forceinline__ void zone_ranges(int nz, int nr, int mz, int32_t* __restrict__ zjrk,
+                                            int32_t* __restrict__ jrk) {
+    int jrs = nr, krs = 0;
+    for (int k = 0; k < nz; k++) {
+        jrs = min(jrs, zjrk[2 * k]);
+        krs = max(krs, zjrk[2 * k + 1]);
+        if (k > 0 && krs > zjrk[2 * k + 1]) zjrk[2 * k + 1] = krs;
+    }
+    jrk[0] = jrs;
+    jrk[1] = krs;
+    // p3fndf.f:66-80, p2fndf.f:41-55: from jrad(1) to krad(mz), the
+    // outer edge moved out while it lies inside jrad(1)
+    int jrf = zjrk[0] < nr ? zjrk[0] : 1;
+    int kz = mz - 1, krf = zjrk[2 * kz + 1];
+    while (krf < jrf && kz + 1 < nz) krf = zjrk[2 * (++kz) + 1];
+    int32_t* frk = zjrk + 2 * GX_MAX_ZONES;
+    frk[0] = krf < jrf ? 1 : jrf;
+    frk[1] = krf < jrf ? nr : min(krf, nr);
+}
+
 // zoncmb + scaled: mass = (mass + sum fr_k src_k) pmass, in the reference's
 // order; block 0 also forms the source ring range over the zones and the
 // field rings of a partial-grid solve in which zones 1..mz move
@@ -213,23 +237,217 @@ __global__ void k_zone_combine(int64_t mesh, float* __restrict__ mass, ZoneSrc s
         for (int k = 0; k < src.n; k++) v = __fadd_rn(v, __fmul_rn(src.fr[k], src.p[k][i]));
         mass[i] = v * pm;
     }
-    if (i == 0) {
-        int jrs = nr, krs = 0;
-        for (int k = 0; k < nz; k++) {
-            jrs = min(jrs, zjrk[2 * k]);
-            krs = max(krs, zjrk[2 * k + 1]);
-            if (k > 0 && krs > zjrk[2 * k + 1]) zjrk[2 * k + 1] = krs;
+    if (i == 0) zone_ranges(nz, nr, mz, zjrk, jrk);
+}
+
+// ---------------------------------------------------------------------------
+// Steps of at most ZONE_DIRECT particles.  A zoned step of a few ten thousand
+// particles is bound by its launches: run100 (15000 particles on 93 x 128) took
+// 14 launches and 81 us a step with the per-zone sort, deposit and combine,
+// five launches and 26 us here.  The direct reductions into the mesh and the
+// unordered gathers cost more per particle than the sorted path's passes, so
+// the two meet at the line below.  Step times, direct and sorted, 2 zones:
+// 2D 93 x 128, 100k 30 / 80 us, 300k 45 / 87, 1M 91 / 127, 2M 155 / 183; 3D 85 x
+// 128 x 75, 100k 86 / 146, 300k 108 / 158, 1M 173 / 215, 2M 273 / 284.
+#define ZONE_DIRECT 2000000
+
+// the nodes and weights of a deposit cell into acc, as integers
+template <int ND, bool Q>
+__device__ __forceinline__ void zone_add(const DevGeo& g, const CellW& c, unsigned long long* __restrict__ acc) {
+    constexpr int NW = Q ? 27 : (ND == 3) ? 8 : 4;
+    float w[NW < 8 ? 8 : NW];
+    int ic[NW < 8 ? 8 : NW];
+    if constexpr (Q) {
+        gx_weights27(c, w);
+        gx_corners27(g, c.row, c.jt, ic);
+    } else {
+        gx_weights<ND>(g, c, w);
+        gx_corners_rt<ND>(g, c.key, c.jt, ic);
+    }
+#pragma unroll
+    for (int k = 0; k < NW; k++) {
+        const int v = __float2int_rn(w[k] * 1048576.0f);
+        if (ic[k] >= 0 && v) atomicAdd(acc + ic[k], (unsigned long long)(long long)v);
+    }
+}
+
+// accumulators of the zones: acc[0] zone 1, then zones 2..nz, mesh cells each
+struct ZoneAcc {
+    unsigned long long* a0;
+    unsigned long long* a1;  // zones 2..nz, one after the other
+    int32_t* rng;            // [GX_MAX_ZONES][2] ring range of each zone's deposits
+    __device__ __forceinline__ unsigned long long* of(int iz, int mesh) const {
+        return iz == 1 ? a0 : a1 + (size_t)(iz - 2) * mesh;
+    }
+};
+
+// ring ranges of a CTA's deposits, gathered in shared memory (all lanes of a
+// warp call zone_rows; iz 0: none)
+__device__ __forceinline__ void zone_rows(int iz, int ring, int nz, int (*sr)[2]) {
+    for (int k = 1; k <= nz; k++) {
+        const bool in = iz == k;
+        if (!__any_sync(0xffffffffu, in)) continue;
+        const int lo = __reduce_min_sync(0xffffffffu, in ? ring : 0x7fffffff);
+        const int hi = __reduce_max_sync(0xffffffffu, in ? ring : -1);
+        if ((threadIdx.x & 31) == 0) {
+            if (lo < sr[k - 1][0]) atomicMin(&sr[k - 1][0], lo);
+            if (hi > sr[k - 1][1]) atomicMax(&sr[k - 1][1], hi);
         }
-        jrk[0] = jrs;
-        jrk[1] = krs;
-        // p3fndf.f:66-80, p2fndf.f:41-55: from jrad(1) to krad(mz), the
-        // outer edge moved out while it lies inside jrad(1)
-        int jrf = zjrk[0] < nr ? zjrk[0] : 1;
-        int kz = mz - 1, krf = zjrk[2 * kz + 1];
-        while (krf < jrf && kz + 1 < nz) krf = zjrk[2 * (++kz) + 1];
-        int32_t* frk = zjrk + 2 * GX_MAX_ZONES;
-        frk[0] = krf < jrf ? 1 : jrf;
-        frk[1] = krf < jrf ? nr : min(krf, nr);
+    }
+}
+__device__ __forceinline__ void zone_rows_begin(int (*sr)[2]) {
+    if (threadIdx.x < GX_MAX_ZONES) {
+        sr[threadIdx.x][0] = 0x7fffffff;
+        sr[threadIdx.x][1] = -1;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ void zone_rows_end(int nz, int (*sr)[2], int32_t* __restrict__ rng) {
+    __syncthreads();
+    if ((int)threadIdx.x < nz && sr[threadIdx.x][1] >= 0) {
+        atomicMin(rng + 2 * threadIdx.x, sr[threadIdx.x][0]);
+        atomicMax(rng + 2 * threadIdx.x + 1, sr[threadIdx.x][1]);
+    }
+}
+
+// every particle's mass into its zone's accumulator (masset)
+template <int ND, bool Q>
+__global__ void __launch_bounds__(256) k_zone_dep(DevGeo g, int nz, const float* __restrict__ P, int64_t cap, int64_t n,
+                                                  const int32_t* __restrict__ zone, ZoneAcc A) {
+    __shared__ int sr[GX_MAX_ZONES][2];
+    zone_rows_begin(sr);
+    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + threadIdx.x;
+        int iz = 0, ring = 0;
+        if (i < n) {
+            const int z = zone[i];
+            const CellW c = gx_cell_t<true, ND>(g, P[i], P[cap + i], ND == 3 ? P[2 * cap + i] : 0.f, false);
+            if (c.key >= 0 && z <= nz) {
+                iz = z;
+                ring = c.row / g.ngz;
+                zone_add<ND, Q>(g, c, A.of(z, g.mesh));
+            }
+        }
+        zone_rows(iz, ring, nz, sr);
+    }
+    zone_rows_end(nz, sr, A.rng);
+}
+
+// the particle pass of a zoned step in place: the particles of zones
+// 1..mzone (and, when mzone = nz, those off the grid) move (as k_push_zone)
+// and are deposited; the others are not touched
+template <int ND, bool Q>
+__global__ void __launch_bounds__(256) k_zone_push(DevGeo g, ZoneTab zt, int mzone, float* __restrict__ P, int64_t cap,
+                                                   int64_t n, const float4* __restrict__ F, int32_t* __restrict__ zone,
+                                                   ZoneAcc A) {
+    __shared__ int sr[GX_MAX_ZONES][2];
+    zone_rows_begin(sr);
+    constexpr int nd = ND, nw = 2 * ND;
+    const int nz = zt.nz, off = nz + 1;
+    for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = i0 + threadIdx.x;
+        const int z0 = i < n ? zone[i] : off + 1;
+        int dz = 0, ring = 0;
+        if (z0 <= mzone || (z0 == off && mzone == nz)) {
+            float q[6], qo[6];
+#pragma unroll
+            for (int k = 0; k < nw; k++) q[k] = qo[k] = P[k * cap + i];
+            float a[3] = {0.f, 0.f, 0.f}, ph;
+            if (z0 != off) {
+                const float z = (ND == 3) ? q[2] : 0.f;
+                const CellW cw = gx_cell_t<true, ND>(g, q[0], q[1], z, true);
+                gx_accel_cell_t<Q, ND>(g, F, cw, q[0], q[1], z, a[0], a[1], a[2], ph);
+            }
+            if (z0 > 1) {
+                const float t = zt_tsfac(zt, z0);
+                for (int d = 0; d < nd; d++) a[d] *= t * t;
+            }
+            for (int d = 0; d < nd; d++) {
+                q[nd + d] += a[d];
+                q[d] += q[nd + d];
+            }
+            CellW cn = gx_cell_t<true, ND>(g, q[0], q[1], (ND == 3) ? q[2] : 0.f, false);
+            int iz = z0;
+            if (z0 != off) {
+                if (cn.key < 0) {
+                    iz = off;
+                    if (z0 < nz) {
+                        zt_chstep(nd, qo, q, a, zt_tsfac(zt, nz) / zt_tsfac(zt, z0));
+                        cn = gx_cell_t<true, ND>(g, q[0], q[1], (ND == 3) ? q[2] : 0.f, false);
+                    }
+                }
+            } else if (cn.key >= 0) {
+                iz = nz;
+            }
+            if (z0 != off && mzone > 1 && iz <= mzone) {
+                int kz = min(zt_zoneno(zt, nd, q[0], q[1], (ND == 3) ? q[2] : 0.f), mzone);
+                if (kz > iz) kz = zt_zoneno(zt, nd, qo[0], qo[1], (ND == 3) ? qo[2] : 0.f);
+                if (kz != iz) {
+                    zt_chstep(nd, qo, q, a, zt_tsfac(zt, kz) / zt_tsfac(zt, iz));
+                    iz = kz;
+                    cn = gx_cell_t<true, ND>(g, q[0], q[1], (ND == 3) ? q[2] : 0.f, false);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < nw; k++) P[k * cap + i] = q[k];
+            if (iz != z0) zone[i] = iz;
+            // the zones deposited this step are those that moved
+            if (cn.key >= 0 && iz <= mzone) {
+                dz = iz;
+                ring = cn.row / g.ngz;
+                zone_add<ND, Q>(g, cn, A.of(iz, g.mesh));
+            }
+        }
+        zone_rows(dz, ring, nz, sr);
+    }
+    zone_rows_end(nz, sr, A.rng);
+}
+
+// zones' arrays in the solve's mass: fr new + fr old, in the order of zoncmb
+struct ZoneMix {
+    float* znew[GX_MAX_ZONES];
+    const float* zold[GX_MAX_ZONES];
+    float fn[GX_MAX_ZONES], fo[GX_MAX_ZONES];
+    bool un[GX_MAX_ZONES], uo[GX_MAX_ZONES];
+};
+
+// the accumulators of zones 1..mdep (deposited since the last call) -> their
+// arrays, cleared; then zoncmb + scaled, and the ring ranges, as k_zone_combine
+__global__ void __launch_bounds__(256) k_zone_mix(int mesh, float* __restrict__ mass, ZoneAcc A, ZoneMix X, float pm, int nz, int nr, int mdep,
+                           int mz, int quad, int32_t* __restrict__ zjrk, int32_t* __restrict__ jrk) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < mesh) {
+        float v = 0.f;
+        for (int k = 0; k < nz; k++) {
+            float w = 0.f;
+            if (k < mdep) {
+                unsigned long long* a = A.of(k + 1, mesh) + i;
+                const unsigned long long q = *a;
+                if (q) *a = 0ull;
+                w = (float)((double)(long long)q * (1.0 / 1048576.0)) * 1.f;
+                if (k > 0) X.znew[k][i] = w;
+            } else if (X.un[k]) {
+                w = X.znew[k][i];
+            }
+            if (k == 0) {
+                v = w;
+                continue;
+            }
+            if (X.un[k]) v = __fadd_rn(v, __fmul_rn(X.fn[k], w));
+            if (X.uo[k]) v = __fadd_rn(v, __fmul_rn(X.fo[k], X.zold[k][i]));
+        }
+        mass[i] = v * pm;
+    }
+    if (i == 0) {
+        for (int k = 0; k < mdep; k++) {
+            // as the sort's row scan gives it: jrad, krad 1-based (empty: nr, 0)
+            const int lo = A.rng[2 * k], hi = A.rng[2 * k + 1];
+            zjrk[2 * k] = hi >= 0 ? lo + (quad ? 0 : 1) : nr;
+            zjrk[2 * k + 1] = hi >= 0 ? min(hi + 2, nr) : 0;
+            A.rng[2 * k] = 0x7fffffff;
+            A.rng[2 * k + 1] = -1;
+        }
+        zone_ranges(nz, nr, mz, zjrk, jrk);
     }
 }
 
@@ -275,29 +493,67 @@ static int zone_deposit(GxCtx* c, int mzone, int32_t* perm_out) {
     return GX_OK;
 }
 
-// zoncmb at the current step number
-static int zone_combine(GxCtx* c) {
+// whether this context's particles take the direct path (GX_FLAG_SORTED_DEPOSIT: the sorted one)
+static bool zone_direct(const GxCtx* c) {
+    return c->n <= ZONE_DIRECT && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT);
+}
+
+static ZoneAcc zone_acc(const GxCtx* c) { return {c->macc, c->zacc, c->zjrk_d + 2 * GX_MAX_ZONES + 2}; }
+
+// deposit (mzone = 0, all zones) or move and deposit zones 1..mzone, direct path
+template <int ND, bool Q>
+static void zone_direct_launch(GxCtx* c, int mzone) {
+    const int64_t n = c->n;
+    const unsigned nb = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8);
+    if (mzone)
+        k_zone_push<ND, Q><<<nb, 256, 0, c->stream>>>(c->g, c->zt, mzone, c->pbuf[c->cur], c->cap, n, c->field,
+                                                      c->pzone[c->cur], zone_acc(c));
+    else
+        k_zone_dep<ND, Q><<<nb, 256, 0, c->stream>>>(c->g, c->nzones, c->pbuf[c->cur], c->cap, n, c->pzone[c->cur],
+                                                     zone_acc(c));
+}
+static int zone_direct_pass(GxCtx* c, int mzone) {
+    if (c->n == 0) return GX_OK;
+    if (c->g.quad) zone_direct_launch<3, true>(c, mzone);
+    else if (c->g.ndim == 3) zone_direct_launch<3, false>(c, mzone);
+    else zone_direct_launch<2, false>(c, mzone);
+    GX_LAUNCHED(c);
+    return GX_OK;
+}
+
+// zoncmb at the current step number; direct path: after the deposit of zones
+// 1..mdep
+static int zone_combine(GxCtx* c, int mdep) {
+    ZoneMix mix = {};
     ZoneSrc src = {};
     for (int k = 1; k < c->nzones; k++) {
         const int ns = c->zt.nstep[k];
+        mix.znew[k] = c->znew[k];
+        mix.zold[k] = c->zold[k];
         int i = c->lstep[k][1] - c->istep;
         if (i < 0 || i > ns) return c->err = "zone mass array at a useless time", GX_ERR_STATE;
         if (i != ns) {
             src.p[src.n] = c->znew[k];
-            src.fr[src.n++] = 1.f - (float)i / (float)ns;
+            mix.un[k] = true;
+            mix.fn[k] = src.fr[src.n++] = 1.f - (float)i / (float)ns;
         }
         if (c->lstep[k][1] != c->istep) {
             i = c->istep - c->lstep[k][0];
             if (c->lstep[k][0] < 0 || i < 0 || i > ns)
                 return c->err = "older zone mass array at a useless time", GX_ERR_STATE;
             src.p[src.n] = c->zold[k];
-            src.fr[src.n++] = 1.f - (float)i / (float)ns;
+            mix.uo[k] = true;
+            mix.fo[k] = src.fr[src.n++] = 1.f - (float)i / (float)ns;
         }
     }
-    const int64_t mesh = c->g.mesh;
-    k_zone_combine<<<(unsigned)((mesh + 255) / 256), 256, 0, c->stream>>>(
-        mesh, c->mass, src, c->g.pmass, c->nzones, c->g.nr, zone_mzone(c, c->istep), c->zjrk_d,
-        c->jrk_d);
+    const int mesh = c->g.mesh, mz = zone_mzone(c, c->istep);
+    const unsigned nb = (unsigned)((mesh + 255) / 256);
+    if (zone_direct(c))
+        k_zone_mix<<<nb, 256, 0, c->stream>>>(mesh, c->mass, zone_acc(c), mix, c->g.pmass, c->nzones, c->g.nr, mdep, mz,
+                                              c->g.quad, c->zjrk_d, c->jrk_d);
+    else
+        k_zone_combine<<<nb, 256, 0, c->stream>>>(mesh, c->mass, src, c->g.pmass, c->nzones, c->g.nr, mz, c->zjrk_d,
+                                                  c->jrk_d);
     GX_LAUNCHED(c);
     return GX_OK;
 }
@@ -330,15 +586,21 @@ int gx_zone_unload(GxCtx* c, float* staging) {
 
 int gx_zone_masset(GxCtx* c) {
     const int64_t n = c->n;
-    if (n > 0) {
-        k_zone_keys<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
-            c->g, c->pbuf[c->cur], c->cap, n, c->pkey[c->cur], c->pfr);
-        GX_LAUNCHED(c);
+    int rc;
+    if (zone_direct(c)) {
+        zone_masscl(c, c->nzones, false);
+        rc = zone_direct_pass(c, 0);
+    } else {
+        if (n > 0) {
+            k_zone_keys<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
+                c->g, c->pbuf[c->cur], c->cap, n, c->pkey[c->cur], c->pfr);
+            GX_LAUNCHED(c);
+        }
+        zone_masscl(c, c->nzones, false);
+        rc = zone_deposit(c, c->nzones, c->perm);
     }
-    zone_masscl(c, c->nzones, false);
-    int rc = zone_deposit(c, c->nzones, c->perm);
     if (rc) return rc;
-    rc = zone_combine(c);
+    rc = zone_combine(c, c->nzones);
     if (rc) return rc;
     c->have_keys = true;
     c->zones_ready = true;
@@ -358,23 +620,29 @@ int gx_zone_step(GxCtx* c, int nsteps, int phys) {
         int rc = gx_mixed_findf(c, lpot, true, partial ? c->zjrk_d + 2 * GX_MAX_ZONES : nullptr);
         if (rc) return rc;
         zone_masscl(c, mzone, true);
-        const int nxt = c->cur ^ 1;
         rc = gx_phase_mark(c, PH_PUSH);
         if (rc) return rc;
-        if (n > 0) {
-            k_push_zone<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
-                c->g, c->zt, mzone, c->pbuf[c->cur], c->pbuf[nxt], c->cap, n, c->perm, c->origin,
-                c->origin_tmp, c->field, c->pkey[c->cur], c->pkey[nxt], c->pfr, c->pzone[c->cur],
-                c->pzone[nxt], (phys && last) ? c->ppot : nullptr);
-            GX_LAUNCHED(c);
+        if (zone_direct(c)) {
+            rc = zone_direct_pass(c, mzone);
+            if (!rc) rc = gx_phase_mark(c, PH_COMBINE);
+            if (rc) return rc;
+        } else {
+            const int nxt = c->cur ^ 1;
+            if (n > 0) {
+                k_push_zone<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(
+                    c->g, c->zt, mzone, c->pbuf[c->cur], c->pbuf[nxt], c->cap, n, c->perm, c->origin,
+                    c->origin_tmp, c->field, c->pkey[c->cur], c->pkey[nxt], c->pfr, c->pzone[c->cur],
+                    c->pzone[nxt]);
+                GX_LAUNCHED(c);
+            }
+            std::swap(c->origin, c->origin_tmp);
+            c->cur = nxt;
+            rc = zone_deposit(c, mzone, c->perm_next);
+            if (rc) return rc;
+            std::swap(c->perm, c->perm_next);
         }
-        std::swap(c->origin, c->origin_tmp);
-        c->cur = nxt;
-        rc = zone_deposit(c, mzone, c->perm_next);
-        if (rc) return rc;
-        std::swap(c->perm, c->perm_next);
         c->istep += 1;
-        rc = zone_combine(c);
+        rc = zone_combine(c, mzone);
         if (rc) return rc;
     }
     int rc = gx_phase_end(c);
@@ -404,6 +672,8 @@ int gx_set_zones(GxCtx* c, int32_t nzones, const int32_t* nstep, const float* zb
     cudaSetDevice(c->dev);
     if (c->zbuf) cudaFree(c->zbuf);
     if (c->zjrk_d) cudaFree(c->zjrk_d);
+    if (c->zacc) cudaFree(c->zacc);
+    c->zacc = nullptr;
     c->zbuf = nullptr;
     c->zjrk_d = nullptr;
     c->zt = ZoneTab{};
@@ -419,7 +689,8 @@ int gx_set_zones(GxCtx* c, int32_t nzones, const int32_t* nstep, const float* zb
     if (nzones == 1) return GX_OK;
     const size_t mesh = c->g.mesh;
     if (cudaMalloc((void**)&c->zbuf, sizeof(float) * 2 * (nzones - 1) * mesh) != cudaSuccess ||
-        cudaMalloc((void**)&c->zjrk_d, sizeof(int32_t) * (2 * GX_MAX_ZONES + 2)) != cudaSuccess) {
+        cudaMalloc((void**)&c->zacc, sizeof(unsigned long long) * (nzones - 1) * mesh) != cudaSuccess ||
+        cudaMalloc((void**)&c->zjrk_d, sizeof(int32_t) * (4 * GX_MAX_ZONES + 2)) != cudaSuccess) {
         c->nzones = 1;
         return c->err = "cudaMalloc of the zone mass arrays failed", GX_ERR_NOMEM;
     }
@@ -428,6 +699,13 @@ int gx_set_zones(GxCtx* c, int32_t nzones, const int32_t* nstep, const float* zb
         c->zold[k] = c->zbuf + (size_t)(2 * (k - 1) + 1) * mesh;
     }
     GX_CUDA(c, cudaMemset(c->zbuf, 0, sizeof(float) * 2 * (nzones - 1) * mesh));
+    GX_CUDA(c, cudaMemset(c->zacc, 0, sizeof(unsigned long long) * (nzones - 1) * mesh));
+    int32_t rng[2 * GX_MAX_ZONES];
+    for (int k = 0; k < GX_MAX_ZONES; k++) {
+        rng[2 * k] = 0x7fffffff;
+        rng[2 * k + 1] = -1;
+    }
+    GX_CUDA(c, cudaMemcpy(c->zjrk_d + 2 * GX_MAX_ZONES + 2, rng, sizeof rng, cudaMemcpyHostToDevice));
     return GX_OK;
 }
 
