@@ -650,9 +650,19 @@ __global__ void __launch_bounds__(F2_THREADS) k_fwd2(DevGeo g, int nact, int ncp
 }
 
 // ---------------------------------------------------------------------------
-// radial contraction; grid (nact, nkz); 8 warps split the source rings.
+// radial contraction of one (harmonic, wavenumber, type) over NC chunks of 32
+// field rings: a lane takes one ring of each chunk (coalesced rows of the
+// Green matrix whatever nr), 8 warps split the source rings, and their sums
+// are added in warp order, so an output's sum is formed the same way whatever
+// NC.  blockIdx.z = 4 (chunk / NC) + type.
 // Types: 0 radial, 1 azimuthal, 2 vertical, 3 potential (p3conv.f:173-226).
-template <bool VEC>
+// Each entry is used for 4 products, so the kernel is bound by its loads: by
+// latency in 2D (a few dozen matrices: one chunk per CTA and 16 rows in flight
+// per warp; with a CTA per matrix and lanes on 4 rings each, 4.2 -> 2.8 us at 64
+// x 128 and 11.8 -> 3.9 at 128 x 256, m = 0..8), by the stream in 3D (85 x 126 x
+// 75, m = 0..8, 53 MB: 26.7 -> 17.3 us; on 128 x 256 x 125 it takes 94 us, the
+// bulk-copy kernel 84).
+template <int NC>
 __global__ void __launch_bounds__(256) k_conv(DevGeo g, int nact, int tmask,
                                               const float* __restrict__ G,
                                               const float4* __restrict__ S,
@@ -660,78 +670,70 @@ __global__ void __launch_bounds__(256) k_conv(DevGeo g, int nact, int tmask,
                                               const int32_t* __restrict__ jrk) {
     extern __shared__ __align__(16) float4 sh4[];
     const int nr = g.nr, nkz = g.nkz, ng = g.ng, mmax = g.mmax, ngz = g.ngz;
+    const int t = blockIdx.z & 3, ir0 = (blockIdx.z >> 2) * NC * 32;
+    if (!((tmask >> t) & 1)) return;
     // source rings jrs..krs (p3conv.f:149-150)
     const int js = max(jrk[0], 1) - 1, ks = min(jrk[1], nr) - 1;
     const int a = blockIdx.x, k = blockIdx.y, m = g.act[a];
+    const int rings = min(NC * 32, nr - ir0);
+    // ring-major output [t][ir][kz][a] (read as one block per ring by the synthesis)
+    const size_t ost = (size_t)nkz * nact;
+    float4* out = O + ((size_t)t * nr * nkz + k) * nact + a + (size_t)ir0 * ost;
+    bool valid = true;
+    if (t == 1) valid = (m >= 1) && (m <= min(ng, mmax - 1) - 1);
+    if (t == 2) valid = (g.ndim == 3) && (k >= 1) && (k <= ngz - 1);
+    if (!valid) {
+        for (int i = threadIdx.x; i < rings; i += blockDim.x) out[i * ost] = make_float4(0, 0, 0, 0);
+        return;
+    }
     float4* Sin = sh4;              // [nr]
-    float4* part = sh4 + nr;        // [8][nr]
+    float4* part = sh4 + nr;        // [8][32 NC]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < nr; i += blockDim.x)
-        Sin[i] = (i >= js && i <= ks) ? S[((size_t)a * nkz + k) * nr + i] : make_float4(0, 0, 0, 0);
+    for (int i = js + threadIdx.x; i <= ks; i += blockDim.x) Sin[i] = S[((size_t)a * nkz + k) * nr + i];
     __syncthreads();
-    {
-        // one field type per CTA (blockIdx.z)
-        const int t = blockIdx.z;
-        if (!((tmask >> t) & 1)) return;
-        bool valid = true;
-        if (t == 1) valid = (m >= 1) && (m <= min(ng, mmax - 1) - 1);
-        if (t == 2) valid = (g.ndim == 3) && (k >= 1) && (k <= ngz - 1);
-        // ring-major output [t][ir][kz][a] (read as one block per ring by the synthesis)
-        const size_t ost = (size_t)nkz * nact;
-        float4* out = O + ((size_t)t * nr * nkz + k) * nact + a;
-        if (!valid) {
-            for (int i = threadIdx.x; i < nr; i += blockDim.x) out[i * ost] = make_float4(0, 0, 0, 0);
-            return;
-        }
-        const float* Gt = G + ((((size_t)t * ng + m) * nkz + k) * nr) * (size_t)nr;
-        for (int ib = 0; ib < nr; ib += 128) {
-            const int ir0 = ib + lane * 4;
-            float4 acc[4];
+    const float* Gt = G + ((((size_t)t * ng + m) * nkz + k) * nr) * (size_t)nr + ir0 + lane;
+    float4 acc[NC];
 #pragma unroll
-            for (int q = 0; q < 4; q++) acc[q] = make_float4(0, 0, 0, 0);
-            if (ir0 < nr) {
-#pragma unroll 4
-                for (int is = js + warp; is <= ks; is += 8) {
-                    float gv[4];
-                    const float* gp = Gt + (size_t)is * nr + ir0;
-                    if (VEC) {
-                        float4 g4 = __ldg(reinterpret_cast<const float4*>(gp));
-                        gv[0] = g4.x; gv[1] = g4.y; gv[2] = g4.z; gv[3] = g4.w;
-                    } else {
+    for (int c = 0; c < NC; c++) acc[c] = make_float4(0, 0, 0, 0);
+    constexpr int U = NC == 1 ? 16 : 4;  // rows in flight per warp
+    for (int is0 = js + warp; is0 <= ks; is0 += 8 * U) {
+        float gv[U][NC];
 #pragma unroll
-                        for (int q = 0; q < 4; q++) gv[q] = (ir0 + q < nr) ? __ldg(gp + q) : 0.f;
-                    }
-                    const float4 s = Sin[is];
+        for (int u = 0; u < U; u++)
 #pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const float gq = gv[q];
-                        if (t == 0 || t == 3) {
-                            acc[q].x += gq * s.x; acc[q].y += gq * s.y;
-                            acc[q].z += gq * s.z; acc[q].w += gq * s.w;
-                        } else if (t == 1) {
-                            acc[q].x += gq * s.z; acc[q].z -= gq * s.x;
-                            acc[q].y += gq * s.w; acc[q].w -= gq * s.y;
-                        } else {
-                            acc[q].x += gq * s.y; acc[q].y -= gq * s.x;
-                            acc[q].z += gq * s.w; acc[q].w -= gq * s.z;
-                        }
-                    }
+            for (int c = 0; c < NC; c++)
+                gv[u][c] = (is0 + 8 * u <= ks && 32 * c + lane < rings) ? __ldg(Gt + (size_t)(is0 + 8 * u) * nr + 32 * c)
+                                                                       : 0.f;
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (is0 + 8 * u > ks) break;
+            const float4 s = Sin[is0 + 8 * u];
+#pragma unroll
+            for (int c = 0; c < NC; c++) {
+                const float gq = gv[u][c];
+                if (t == 0 || t == 3) {
+                    acc[c].x += gq * s.x; acc[c].y += gq * s.y;
+                    acc[c].z += gq * s.z; acc[c].w += gq * s.w;
+                } else if (t == 1) {
+                    acc[c].x += gq * s.z; acc[c].z -= gq * s.x;
+                    acc[c].y += gq * s.w; acc[c].w -= gq * s.y;
+                } else {
+                    acc[c].x += gq * s.y; acc[c].y -= gq * s.x;
+                    acc[c].z += gq * s.w; acc[c].w -= gq * s.z;
                 }
+            }
+        }
+    }
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (ir0 + q < nr) part[warp * nr + ir0 + q] = acc[q];
-            }
+    for (int c = 0; c < NC; c++) part[(warp * NC + c) * 32 + lane] = acc[c];
+    __syncthreads();
+    for (int i = threadIdx.x; i < rings; i += blockDim.x) {
+        float4 s = part[i];
+        for (int w = 1; w < 8; w++) {
+            const float4 p = part[w * NC * 32 + i];
+            s.x += p.x; s.y += p.y; s.z += p.z; s.w += p.w;
         }
-        __syncthreads();
-        for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-            float4 s = part[i];
-            for (int w = 1; w < 8; w++) {
-                float4 p = part[w * nr + i];
-                s.x += p.x; s.y += p.y; s.z += p.z; s.w += p.w;
-            }
-            out[i * ost] = s;
-        }
-        __syncthreads();
+        out[i * ost] = s;
     }
 }
 
@@ -822,16 +824,13 @@ int gx_mixed_findf(GxCtx* c, int lpot, bool polcat_only_field, const int32_t* fr
             if (rc) return rc;
         }
     } else {
-        size_t sm = sizeof(float4) * (size_t)g.nr * 9;
-        dim3 grid(nact, g.nkz, 4);
-        bool vec = (g.nr % 4) == 0;
-        if (vec) {
-            GX_CUDA(c, cudaFuncSetAttribute(k_conv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            k_conv<true><<<grid, 256, sm, c->stream>>>(g, nact, tmask, c->green32, c->specS, c->specO, c->jrk_d);
-        } else {
-            GX_CUDA(c, cudaFuncSetAttribute(k_conv<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            k_conv<false><<<grid, 256, sm, c->stream>>>(g, nact, tmask, c->green32, c->specS, c->specO, c->jrk_d);
-        }
+        // 2D: one chunk of rings per CTA; 3D: all of them (up to 128 rings)
+        const int nch = (g.nr + 31) / 32, nc = (g.ndim == 2) ? 1 : std::min(nch, 4);
+        const size_t sm = sizeof(float4) * ((size_t)g.nr + 8 * 32 * nc);
+        auto kc = nc == 1 ? k_conv<1> : nc == 2 ? k_conv<2> : nc == 3 ? k_conv<3> : k_conv<4>;
+        GX_CUDA(c, cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+        kc<<<dim3(nact, g.nkz, 4 * ((nch + nc - 1) / nc)), 256, sm, c->stream>>>(g, nact, tmask, c->green32, c->specS,
+                                                                                c->specO, c->jrk_d);
         GX_LAUNCHED(c);
     }
     rc = gx_phase_mark(c, PH_SYN);
