@@ -575,16 +575,17 @@ __global__ void k_bk_rows(DevGeo g, const float* __restrict__ P, int64_t cap, in
 // tens of thousands of particles, whose single-address atomics otherwise
 // serialise.  The scatter reserves each row's slots for the CTA with one
 // atomic on the row's fill counter and hands them out from shared memory.
+// A run is BK_RUN particles, or fewer when that would leave SMs idle (bk_run).
 #define BK_RUN 32768
 template <int ND>
 __global__ void __launch_bounds__(256) k_bk_rows_cta(DevGeo g, const float* __restrict__ P, int64_t cap,
-                                                     int64_t n, int32_t* __restrict__ rows,
+                                                     int64_t n, int run, int32_t* __restrict__ rows,
                                                      int32_t* __restrict__ cnt) {
     extern __shared__ int32_t hist[];  // [nrow + 1]
     const int nr1 = g.nrow + 1;
     for (int r = threadIdx.x; r < nr1; r += blockDim.x) hist[r] = 0;
     __syncthreads();
-    const int64_t i0 = (int64_t)blockIdx.x * BK_RUN, i1 = min(n, i0 + BK_RUN);
+    const int64_t i0 = (int64_t)blockIdx.x * run, i1 = min(n, i0 + run);
     for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
         const CellW c = gx_cell_t<true, ND>(g, P[i], P[cap + i], ND == 3 ? P[2 * cap + i] : 0.f, false);
         const int rk = (c.key >= 0) ? c.row : g.nrow;
@@ -597,7 +598,7 @@ __global__ void __launch_bounds__(256) k_bk_rows_cta(DevGeo g, const float* __re
 }
 
 template <int NP>
-__global__ void __launch_bounds__(256) k_bk_scatter_cta(const float* __restrict__ P, int64_t cap, int64_t n,
+__global__ void __launch_bounds__(256) k_bk_scatter_cta(const float* __restrict__ P, int64_t cap, int64_t n, int run,
                                                         const int32_t* __restrict__ oin, float4* __restrict__ Qout,
                                                         int64_t bcap, const int32_t* __restrict__ rows, int nr1,
                                                         const int32_t* __restrict__ cap_o,
@@ -607,7 +608,7 @@ __global__ void __launch_bounds__(256) k_bk_scatter_cta(const float* __restrict_
     extern __shared__ int32_t slot[];  // [nrow + 1]: this CTA's count, then its next slot
     for (int r = threadIdx.x; r < nr1; r += blockDim.x) slot[r] = 0;
     __syncthreads();
-    const int64_t i0 = (int64_t)blockIdx.x * BK_RUN, i1 = min(n, i0 + BK_RUN);
+    const int64_t i0 = (int64_t)blockIdx.x * run, i1 = min(n, i0 + run);
     for (int64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) atomicAdd(slot + rows[i], 1);
     __syncthreads();
     for (int r = threadIdx.x; r < nr1; r += blockDim.x)
@@ -784,14 +785,23 @@ static int bk_plan(GxCtx* c, int out, bool with_items, cudaStream_t st) {
     return GX_OK;
 }
 
+// particles per CTA of the bucketing: two CTAs per SM when the particles
+// suffice for runs of at least 1024, BK_RUN at most.  1M particles in runs of
+// 32768 (31 CTAs) took 234 us to count and place, in runs of 3584 60 us.
+static int bk_run(int64_t n) {
+    const int64_t r = (n / (2 * 148) + 256) / 256 * 256;
+    return (int)std::min<int64_t>(BK_RUN, std::max<int64_t>(1024, r));
+}
+
 template <int NP>
 static void bk_scatter_cta_launch(GxCtx* c, int b) {
     const int nr1 = c->g.nrow + 1;
-    const unsigned nruns = (unsigned)((c->n + BK_RUN - 1) / BK_RUN);
+    const int run = bk_run(c->n);
+    const unsigned nruns = (unsigned)((c->n + run - 1) / run);
     cudaFuncSetAttribute(k_bk_scatter_cta<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)(sizeof(int32_t) * nr1));
     k_bk_scatter_cta<NP><<<nruns, 256, sizeof(int32_t) * nr1, c->stream>>>(
-        c->pbuf[c->cur], c->cap, c->n, c->origin, c->bq[b], c->bcap, c->pkey[0], nr1, c->bk_cap[b], c->bk_base[b],
+        c->pbuf[c->cur], c->cap, c->n, run, c->origin, c->bq[b], c->bcap, c->pkey[0], nr1, c->bk_cap[b], c->bk_base[b],
         c->bk_fill[b], c->bk_ctl + 4 * b, c->bk_main);
 }
 
@@ -824,8 +834,9 @@ static int gx_bucketize(GxCtx* c) {
         if (cta) {
             auto kr = (g.ndim == 3) ? k_bk_rows_cta<3> : k_bk_rows_cta<2>;
             cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hbytes);
-            kr<<<(unsigned)((n + BK_RUN - 1) / BK_RUN), 256, hbytes, c->stream>>>(g, c->pbuf[c->cur], c->cap, n,
-                                                                                c->pkey[0], c->bk_cnt);
+            const int run = bk_run(n);
+            kr<<<(unsigned)((n + run - 1) / run), 256, hbytes, c->stream>>>(g, c->pbuf[c->cur], c->cap, n, run,
+                                                                            c->pkey[0], c->bk_cnt);
         } else {
             auto kr = (g.ndim == 3) ? k_bk_rows<3> : k_bk_rows<2>;
             kr<<<nb, 256, 0, c->stream>>>(g, c->pbuf[c->cur], c->cap, n, c->pkey[0], c->bk_cnt);
