@@ -454,13 +454,16 @@ static int alloc_particles(GxCtx* c, int64_t n) {
     DALLOC(c, c->stage, (size_t)c->maxitems * nq * c->g.na);
     // fused-pass work items: every row's segment in chunks of bk_item
     // particles, and the overflow area's.  bk_item: at most BK_ITEM, at
-    // least half a deposit window of particles (the bins each item
-    // flushes), and otherwise small enough that a B200's resident CTAs
-    // (148 SMs x 5) get two items each when the particles are few
+    // least a quarter of a deposit window of particles (the bins each item
+    // flushes; half of it in 2D), and otherwise small enough that a B200's
+    // resident CTAs (148 SMs x 5) get a few items each: 2 in 3D, where an item
+    // more costs a window's flush (10M particles: 262 us a pass in items of
+    // 4095, 292 in items of 1024; 1M: 73 us in items of 2048, 67 in items of
+    // 1024), 4 in 2D (3M: 76 and 73 us)
     {
-        const int64_t wrows = (c->g.ndim == 3) ? 16 : 4;
-        const int64_t wmin = std::min<int64_t>(BK_ITEM, std::max<int64_t>(256, wrows * c->g.na / 2));
-        c->bk_item = (int)std::min<int64_t>(BK_ITEM, std::max<int64_t>(wmin, n / (2 * 148 * 5)));
+        const bool d3 = c->g.ndim == 3;
+        const int64_t wmin = std::max<int64_t>(256, (d3 ? 16 : 4) * c->g.na / (d3 ? 4 : 2));
+        c->bk_item = (int)std::min<int64_t>(BK_ITEM, std::max<int64_t>(wmin, n / ((d3 ? 2 : 4) * 148 * 5)));
     }
     c->bk_maxitems = (int64_t)c->g.nrow + 1 + 2 * (n / c->bk_item + 2);
     DALLOC(c, c->bk_items, (size_t)c->bk_maxitems);

@@ -51,6 +51,13 @@
 
 #define BK_FIXQ 1048576.0f  // 2^20: the fixed-point quantum of gx_deposit.cu
 #define BK_SPARSE 256       // items with fewer particles add straight into the mesh
+// items with at least this many particles copy the field rows of their cells
+// (4 rows in 3D, 2 in 2D) into shared memory and gather there: the gathers of a
+// row's particles touch some 20 lines of the first-level cache per load, in
+// shared memory some 11 wavefronts (10M particles, 3D: the pass 282 -> 262 us;
+// 3M in 2D and short items: no change)
+#define BK_STAGE 512
+#define BK_CTASLOT 768      // 2D items with at least this many take their slots by CTA
 #define BK_THREADS 256
 #define PLAN_THREADS 512
 #define PLAN_ROWS 8         // rows per plan thread per pass
@@ -307,27 +314,51 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
     const int32_t* __restrict__ base_o, int32_t* __restrict__ fill_o, int32_t* __restrict__ ovf_o,
     int64_t ovf_base, unsigned long long* __restrict__ acc) {
     extern __shared__ __align__(16) uint32_t bins[];
-    __shared__ int s_item;
+    __shared__ int s_it[2];
+    __shared__ int4 s_I[2];
     constexpr bool d3 = ND == 3;
     constexpr int WROWS = d3 ? 16 : 4;
+    // 2D: an iteration's particles of each window row and their first slot
+    // (double-buffered: the next iteration counts while this one stores)
+    constexpr int OWN = 1;  // the item's row in its window
+    __shared__ int s_cnt[2][4], s_slot[2][4];
     constexpr int NW = 2 * ND;
     const int na = g.na, ngz = d3 ? g.ngz : 1, nrow = g.nrow;
     const int nit = ctl[0];
     int rmin_l = 0x7fffffff, rmax_l = -1;  // ring range of this lane's new cells
     int zmin_l = 0x7fffffff, zmax_l = -1;  // and their plane range (3D)
+    // the field rows of a cell of the item's row: (row, row + 1) and in 3D
+    // (row + ngz, row + ngz + 1), na float4 each
+    float4* fw = reinterpret_cast<float4*>(bins + WROWS * na);
+    auto fetch = [&](int b) {
+        const int it = atomicAdd(ctl + 1, 1);
+        s_it[b] = it;
+        if (it < nit) s_I[b] = items[it];
+    };
     for (int i = threadIdx.x; i < WROWS * na; i += BK_THREADS) bins[i] = 0u;
-    for (;;) {
-        if (threadIdx.x == 0) s_item = atomicAdd(ctl + 1, 1);
-        __syncthreads();  // also orders the previous item's flush before these deposits
-        const int it = s_item;
-        if (it >= nit) break;
-        const int4 I = items[it];
+    if (threadIdx.x == 0) fetch(0);
+    if (!d3 && threadIdx.x < 8) (&s_cnt[0][0])[threadIdx.x] = 0;
+    __syncthreads();
+    int ph = 0;  // buffer of s_cnt, s_slot
+    for (int b = 0;; b ^= 1) {
+        if (s_it[b] >= nit) break;
+        const int4 I = s_I[b];
+        if (threadIdx.x == 0) fetch(b ^ 1);  // the next item, while this one runs
         const int row = I.x, s0 = I.y, s1 = I.z;
         const bool win = row >= 0 && row < nrow && (s1 - s0) >= BK_SPARSE;
         // ring and plane of the item's row (the plan stores the ring): the
         // window's origin is one below
         const int wir = I.w;
         const int wiz = d3 ? row - wir * ngz : 0;
+        const bool cta = !d3 && (s1 - s0) >= BK_CTASLOT;
+        const bool stage = !DEP && row >= 0 && row + (d3 ? ngz : 0) + 1 < nrow && (s1 - s0) >= BK_STAGE;
+        if (stage) {
+            const float4* f0 = F + (size_t)row * na;
+#pragma unroll 4
+            for (int i = threadIdx.x; i < (d3 ? 4 : 2) * na; i += BK_THREADS)
+                fw[i] = __ldg(f0 + (d3 && i >= 2 * na ? i + (ngz - 2) * na : i));
+            __syncthreads();
+        }
         constexpr int NP = NW + (COMP ? ND : 0);
         constexpr int NQC = d3 ? 4 : 2;  // corner rows of a cell
         for (int b0 = s0; b0 < s1; b0 += BK_THREADS) {
@@ -345,7 +376,27 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                 if (!DEP) {
                     const CellW cw = gx_cell_t<false, ND>(g, x, y, z, true);
                     float ax, ay, az, ph;
-                    gx_accel_cell_t<false, ND>(g, F, cw, x, y, z, ax, ay, az, ph);
+                    if (stage && cw.key >= 0 && cw.row == row) {
+                        // the common case: the corners from the staged rows
+                        // (in the order of gx_accel_cell_t)
+                        float w[8];
+                        gx_weights<ND>(g, cw, w);
+                        const int j0 = cw.jt, j1 = (cw.jt == na - 1) ? 0 : cw.jt + 1;
+                        ax = ay = az = ph = 0.f;
+#pragma unroll
+                        for (int q = 0; q < NQC; q++) {
+                            const float4 a = fw[q * na + j0], c = fw[q * na + j1];
+                            ax += a.x * w[2 * q];
+                            ay += a.y * w[2 * q];
+                            if (d3) az += a.z * w[2 * q];
+                            ax += c.x * w[2 * q + 1];
+                            ay += c.y * w[2 * q + 1];
+                            if (d3) az += c.z * w[2 * q + 1];
+                        }
+                        gx_rigid_force(g, x, y, z, ax, ay, az, ph);
+                    } else {
+                        gx_accel_cell_t<false, ND>(g, F, cw, x, y, z, ax, ay, az, ph);
+                    }
                     float& vx = P[ND];
                     float& vy = P[ND + 1];
                     vx += ax;
@@ -376,19 +427,51 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                     }
                 }
             }
-            // the row's slot: warp-aggregated atomic on its fill counter,
-            // issued before the deposit so that its latency overlaps it
+            // the slot in the new row's segment, taken before the deposit so that
+            // the latency of the fill counter's atomic overlaps it.  3D (rows by
+            // the thousand): one atomic per warp and row.  2D: those serialise on
+            // the few rows' counters, so a particle takes a rank among the
+            // CTA's particles of its row in shared memory (those that stay in
+            // the item's row by warp, the others one by one) and one thread per
+            // window row takes the slots of all of them (3M particles on 128 x
+            // 256, items of 1013: the pass 85 -> 73 us).  In 3D the barriers this
+            // needs cost more than the atomics (10M: 262 -> 321 us), as they do
+            // for short items.
             const unsigned lane = threadIdx.x & 31;
             uint32_t peers = 0;
-            int leader = -1, bslot = 0, capr = 0, baser = 0;
+            int leader = -1, bslot = 0, capr = 0, baser = 0, wi = -1, rank = 0;
             if (!DEP) {
-                const uint32_t am = __ballot_sync(0xffffffffu, act);
-                peers = __match_any_sync(0xffffffffu, act ? rk : 0xffffffffu) & am;
-                leader = __ffs(peers) - 1;
-                if (act && (int)lane == leader) bslot = atomicAdd(fill_o + rk, __popc(peers));
+                if (cta) {
+                    if (act && cn.key >= 0 && row >= 0 && row < nrow && (unsigned)(cn.row - row + 1) < 4u)
+                        wi = cn.row - row + 1;
+                    const uint32_t st = __ballot_sync(0xffffffffu, wi == OWN);
+                    if (st) {
+                        const int l0 = __ffs(st) - 1;
+                        if ((int)lane == l0) rank = atomicAdd(&s_cnt[ph][OWN], __popc(st));
+                        rank = __shfl_sync(0xffffffffu, rank, l0) + __popc(st & lanemask_lt());
+                    }
+                    if (wi >= 0 && wi != OWN) rank = atomicAdd(&s_cnt[ph][wi], 1);
+                }
+                const bool far = act && wi < 0;
+                if (!cta || __any_sync(0xffffffffu, far)) {
+                    const uint32_t am = __ballot_sync(0xffffffffu, far);
+                    peers = __match_any_sync(0xffffffffu, far ? rk : 0xffffffffu) & am;
+                    leader = __ffs(peers) - 1;
+                    if (far && (int)lane == leader) bslot = atomicAdd(fill_o + rk, __popc(peers));
+                }
                 if (act) {
                     capr = __ldg(cap_o + rk);
                     baser = __ldg(base_o + rk);
+                }
+                if (cta) {
+                    __syncthreads();
+                    if (threadIdx.x < 4) {
+                        const int c = s_cnt[ph][threadIdx.x];
+                        if (c) {
+                            s_slot[ph][threadIdx.x] = atomicAdd(fill_o + row - 1 + (int)threadIdx.x, c);
+                            s_cnt[ph][threadIdx.x] = 0;
+                        }
+                    }
                 }
             }
             // the common case: every corner inside the window (the new cell
@@ -467,7 +550,12 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
             }
             if (!DEP) {
                 bslot = __shfl_sync(0xffffffffu, bslot, leader < 0 ? 0 : leader);
-                const int slot = bslot + __popc(peers & lanemask_lt());
+                int slot = bslot + __popc(peers & lanemask_lt());
+                if (cta) {
+                    __syncthreads();
+                    if (wi >= 0) slot = s_slot[ph][wi] + rank;
+                    ph ^= 1;
+                }
                 int64_t dst = (int64_t)baser + slot;
                 const bool ovf = act && slot >= capr;
                 const uint32_t om = __ballot_sync(0xffffffffu, ovf);
@@ -496,7 +584,9 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                 }
             }
         }
-        __syncthreads();  // s_item is rewritten by thread 0 next
+        // orders the flush before the next deposits, and the next item's
+        // descriptor and field rows after this item's use of theirs
+        __syncthreads();
     }
     // the ring range of the new cells (massgn's jrad / krad): one atomic
     // pair per warp
@@ -911,12 +1001,16 @@ int gx_bucket_unload(GxCtx* c, float* aos) {
 template <int ND, bool COMP, bool DEP = false>
 static int bk_launch_push(GxCtx* c, int cur, int nxt) {
     const DevGeo& g = c->g;
-    const size_t sm = sizeof(uint32_t) * (ND == 3 ? 16 : 4) * g.na;
+    // the deposit window and, for the push, the staged field rows
+    const size_t sb = sizeof(uint32_t) * (ND == 3 ? 16 : 4) * g.na;
+    const size_t sf = sb + sizeof(float4) * (ND == 3 ? 4 : 2) * g.na;
+    const size_t sm = DEP ? sb : sf;
     auto kp = k_push_bkt<ND, COMP, DEP>;
     GX_CUDA(c, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     if (!c->bk_grid) {
         int per = 0, sms = 148;
-        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_push_bkt<ND, COMP>, BK_THREADS, sm));
+        GX_CUDA(c, cudaFuncSetAttribute(k_push_bkt<ND, COMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
+        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_push_bkt<ND, COMP>, BK_THREADS, sf));
         GX_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
         c->bk_grid = std::max(1, per) * sms;
     }

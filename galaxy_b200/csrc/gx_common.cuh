@@ -590,6 +590,22 @@ __device__ __forceinline__ void gx_disc_force(const DevGeo& g, float x, float y,
     ph -= g.halo_v2 / sd;
 }
 
+// the rigid force of a particle on the grid (halfrc, or the fixed disc force)
+__device__ __forceinline__ void gx_rigid_force(const DevGeo& g, float x, float y, float z, float& ax, float& ay,
+                                               float& az, float& ph) {
+    if (g.halo == 1) {
+        // cored isothermal halo (frhalo.f:55-56): F(r) = -v^2 r / (r^2 + rc^2)
+        const float r2 = x * x + y * y + ((g.ndim == 3) ? z * z : 0.f);
+        const float f = -g.halo_v2 / (r2 + g.halo_rc2);
+        ax += f * x;
+        ay += f * y;
+        if (g.ndim == 3) az += f * z;
+        ph += 0.5f * g.halo_v2 * logf(1.f + r2 / g.halo_rc2);
+    } else if (g.halo == 2) {
+        gx_disc_force(g, x, y, z, ax, ay, az, ph);
+    }
+}
+
 // interpolated acceleration and potential of a particle at (x, y, z) whose
 // interpolation cell is cw: grdacc + halfrc (or the fixed disc force)
 template <bool Q, int ND = 0>
@@ -645,21 +661,7 @@ __device__ __forceinline__ void gx_accel_cell_t(const DevGeo& g, const float4* _
             ph += f.w * w[k];
         }
     }
-    if (g.halo == 1) {
-        // cored isothermal halo (frhalo.f:55-56): F(r) = -v^2 r / (r^2 + rc^2)
-        float r2 = x * x + y * y + ((g.ndim == 3) ? z * z : 0.f);
-        float rr = sqrtf(r2);
-        float fr = -g.halo_v2 * rr / (r2 + g.halo_rc2);
-        if (fr != 0.f) {
-            fr = fr / rr;
-            ax += fr * x;
-            ay += fr * y;
-            if (g.ndim == 3) az += fr * z;
-        }
-        ph += 0.5f * g.halo_v2 * logf(1.f + r2 / g.halo_rc2);
-    } else if (g.halo == 2) {
-        gx_disc_force(g, x, y, z, ax, ay, az, ph);
-    }
+    gx_rigid_force(g, x, y, z, ax, ay, az, ph);
 }
 
 __device__ __forceinline__ void gx_accel_cell(const DevGeo& g, const float4* __restrict__ F,
