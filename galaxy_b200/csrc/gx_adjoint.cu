@@ -107,17 +107,14 @@ __device__ __forceinline__ void adj_deposit(const DevGeo& g, float x, float y, u
     }
 }
 
-// the ring range of a pass (rng[0] first, rng[1] last), one atomic pair per warp
+// the ring range of a pass (rng[0] first, rng[1] last)
 __device__ __forceinline__ void adj_range(int rlo, int rhi, int32_t* __restrict__ rng) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         rlo = min(rlo, __shfl_xor_sync(0xffffffffu, rlo, o));
         rhi = max(rhi, __shfl_xor_sync(0xffffffffu, rhi, o));
     }
-    if ((threadIdx.x & 31) == 0 && rhi >= 0) {
-        atomicMin(rng, rlo);
-        atomicMax(rng + 1, rhi);
-    }
+    if ((threadIdx.x & 31) == 0 && rhi >= 0) gx_atomic_range(rng, rlo, rhi);
 }
 
 // The sweeps' particle passes.  The particles stay in load order (16-byte
@@ -126,8 +123,8 @@ __device__ __forceinline__ void adj_range(int rlo, int rhi, int32_t* __restrict_
 // four 64-bit reductions into the accumulator inside the pass replaces a
 // pass that keyed the particles, their counting sort, the row deposit, the
 // combine and two copies of the positions (50 us a solve at 400k particles,
-// 128 x 256; the fused forward pass takes 23.7).  CTAs stride over the
-// particles so that the ring range costs one atomic pair per resident warp.
+// 128 x 256; the fused forward pass takes 20.4, 23.7 while every warp queued its
+// ring range on two words).
 
 // the mass of the records S (the first solve, and the context's mass afterwards)
 __global__ void __launch_bounds__(ADJ_BS) k_adj_mass(DevGeo g, const float4* __restrict__ S, int64_t n,

@@ -562,6 +562,15 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// [lo, hi] into the range words r[0] (min) and r[1] (max): the words are read
+// first, so that only the few contributions that widen the range queue an
+// atomic on its one address
+__device__ __forceinline__ void gx_atomic_range(int32_t* r, int lo, int hi) {
+    const volatile int32_t* v = r;
+    if (lo < v[0]) atomicMin(r, lo);
+    if (hi > v[1]) atomicMax(r + 1, hi);
+}
+
 #define ROW_TILE 256  // rows per block of the row reduce / scan
 
 // warp-aggregated count of row (all 32 lanes must call)
