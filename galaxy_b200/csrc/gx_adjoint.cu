@@ -537,7 +537,6 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     b.psi = (float*)(c->adj_ws + opsi);
     b.drift = (unsigned int*)(c->adj_ws + odrift);
     cudaStream_t st = c->stream;
-    int32_t* rng = c->bk_ctl + 13;  // ring range of the accumulated mass (k_mass_convert reads and resets it)
     c->launches = 0;
     GX_CUDA(c, cudaEventRecord(c->ev0, st));
     // initial state in load order
@@ -547,13 +546,13 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     GX_CUDA(c, cudaMemcpyAsync(b.ck, b.S, sbytes, cudaMemcpyDeviceToDevice, st));
     // forward sweep with checkpoints
     if (nsteps > 0) {
-        k_adj_mass<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->macc, rng);
+        k_adj_mass<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->macc, gx_mass_ranges(c));
         GX_LAUNCHED(c);
     }
     for (int s = 0; s < nsteps; s++) {
         int rc = adj_solve(c);
         if (rc) return rc;
-        k_adj_fwd<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->field, c->macc, rng);
+        k_adj_fwd<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->field, c->macc, gx_mass_ranges(c));
         GX_LAUNCHED(c);
         if ((s + 1) % ckpt_every == 0)
             GX_CUDA(c, cudaMemcpyAsync(b.ck + (size_t)((s + 1) / ckpt_every) * n, b.S, sbytes,
@@ -587,7 +586,7 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
         const bool ck = (s % ckpt_every) == 0;
         // the psi term of step s + 1, the drift back to x_s and its deposit
         k_adj_b<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, s == nsteps - 1 ? nullptr : b.psi, g.pmass, 1,
-                                       ck ? b.ck + (size_t)(s / ckpt_every) * n : nullptr, b.drift, c->macc, rng);
+                                       ck ? b.ck + (size_t)(s / ckpt_every) * n : nullptr, b.drift, c->macc, gx_mass_ranges(c));
         GX_LAUNCHED(c);
         int rc = adj_solve(c);
         if (rc) return rc;
@@ -599,7 +598,7 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
         GX_LAUNCHED(c);
     }
     if (nsteps > 0) {
-        k_adj_b<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, b.psi, g.pmass, 0, nullptr, b.drift, c->macc, rng);
+        k_adj_b<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, b.psi, g.pmass, 0, nullptr, b.drift, c->macc, gx_mass_ranges(c));
         GX_LAUNCHED(c);
     }
     GX_CUDA(c, cudaEventRecord(c->ev1, st));

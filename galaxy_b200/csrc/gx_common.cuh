@@ -177,15 +177,17 @@ struct GxCtx {
     int32_t* bk_base[2] = {nullptr, nullptr};
     int32_t* bk_fill[2] = {nullptr, nullptr};
     int32_t* bk_ctl = nullptr;               // [2][4]: overflow count of each buffer; [8] items, [9] work
-                                             // counter, [10..11] plane range, [12] compaction counter,
-                                             // [13..14] ring range (of the pass's new cells)
+                                             // counter, [12] compaction counter; [16 + 4 p ..]: ring
+                                             // range and plane range of a pass's new cells, p = mpar
+    int mpar = 0;                            // set of ranges the next deposit pass adds to and the next
+                                             // conversion reads (which clears the other set)
     int4* bk_items = nullptr;                // work items of pbuf[cur]: row (-1: overflow), first, end slot
     int64_t bk_maxitems = 0;
     int bk_item = BK_ITEM;                   // particles per work item of the fused pass
     int32_t* bk_cnt = nullptr;               // [nrow + 1] row counts of the dense store (bucketing)
     unsigned long long* macc = nullptr;      // [mesh] fixed-point mass (2^-20 of a particle), zero between steps
-    int32_t* zr_d = nullptr;                 // [2] first, last plane holding the fused pass's mass
-                                             // (ngz, -1 when empty)
+    int32_t* zr_d = nullptr;                 // [2][2] first, last plane holding the fused pass's mass
+                                             // (ngz, -1 when empty), at 2 p of the conversion of set p
     bool zr_valid = false;                   // the mass array is the fused pass's (zr_d describes it)
     int bk_grid = 0;                         // CTAs of the fused pass
     cudaStream_t bk_side = nullptr;          // the plan's stream (overlaps the field solve)
@@ -720,6 +722,7 @@ int gx_fast_step(GxCtx* c, int nsteps, int phys);
 int gx_dense(GxCtx* c);  // bucketed store -> dense store (no-op when dense)
 int gx_bucket_unload(GxCtx* c, float* aos);  // unload from the bucketed store
 int gx_fast_masset(GxCtx* c);  // masset by the deposit-only fused pass
+static inline int32_t* gx_mass_ranges(const GxCtx* c) { return c->bk_ctl + 16 + 4 * c->mpar; }  // of the next deposit
 int gx_mass_convert(GxCtx* c);  // mass accumulator -> mass array (accumulator cleared)
 int gx_bucket_alloc(GxCtx* c);
 int gx_bucket_words(const GxCtx* c);  // float4 words per record of the bucketed store
