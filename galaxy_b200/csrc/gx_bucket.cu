@@ -50,7 +50,9 @@
 #include "gx_common.cuh"
 
 #define BK_FIXQ 1048576.0f  // 2^20: the fixed-point quantum of gx_deposit.cu
-#define BK_SPARSE 256       // items with fewer particles add straight into the mesh
+// items with fewer particles add straight into the mesh (the flush of a window
+// costs about as much; 32 to 256 are within 2 % at 170 to 310 particles a row)
+#define BK_SPARSE 128
 // items with at least this many particles copy the field rows of their cells
 // (4 rows in 3D, 2 in 2D) into shared memory and gather there: the gathers of a
 // row's particles touch some 20 lines of the first-level cache per load, in
@@ -306,8 +308,13 @@ __device__ __forceinline__ void rec_store(float4* __restrict__ Q, int64_t bcap, 
 // DEP: the deposit alone (masset on the bucketed store): the cell of each
 // particle's current position, its weights into the bins and the mesh, the
 // ring and plane range; no field, no move, the store is not rewritten
-template <int ND, bool COMP, bool DEP = false>
-__global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
+// Q: the quadratic scheme (3D): 27 nodes around the central one, the window 5
+// rings x 5 planes around the item's row, so that the nodes of every cell a
+// move of less than a cell reaches lie in it; four CTAs per SM (64 registers).
+// 500k particles on 64 x 128 x 45: 58.7 us, where the sorted path's push, sort,
+// 27-weight deposit and combine took 75
+template <int ND, bool COMP, bool DEP = false, bool Q = false>
+__global__ void __launch_bounds__(BK_THREADS, Q ? 4 : BK_MINB) k_push_bkt(
     DevGeo g, const float4* __restrict__ Qin, float4* __restrict__ Qout, int64_t bcap,
     const float4* __restrict__ F,
     const int4* __restrict__ items, int32_t* __restrict__ ctl, const int32_t* __restrict__ cap_o,
@@ -317,7 +324,8 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
     __shared__ int s_it[2];
     __shared__ int4 s_I[2];
     constexpr bool d3 = ND == 3;
-    constexpr int WROWS = d3 ? 16 : 4;
+    constexpr int WROWS = Q ? 25 : d3 ? 16 : 4;
+    constexpr int W = Q ? 5 : 4, WLO = Q ? 2 : 1;  // window rings and planes, those below the item's row
     // 2D: an iteration's particles of each window row and their first slot
     // (double-buffered: the next iteration counts while this one stores)
     constexpr int OWN = 1;  // the item's row in its window
@@ -329,7 +337,7 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
     int zmin_l = 0x7fffffff, zmax_l = -1;  // and their plane range (3D)
     // the field rows of a cell of the item's row: (row, row + 1) and in 3D
     // (row + ngz, row + ngz + 1), na float4 each
-    float4* fw = reinterpret_cast<float4*>(bins + WROWS * na);
+    float4* fw = reinterpret_cast<float4*>(bins + (Q ? 28 : WROWS) * na);
     auto fetch = [&](int b) {
         const int it = atomicAdd(ctl + 1, 1);
         s_it[b] = it;
@@ -351,8 +359,16 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
         const int wir = I.w;
         const int wiz = d3 ? row - wir * ngz : 0;
         const bool cta = !d3 && (s1 - s0) >= BK_CTASLOT;
-        const bool stage = !DEP && row >= 0 && row + (d3 ? ngz : 0) + 1 < nrow && (s1 - s0) >= BK_STAGE;
-        if (stage) {
+        bool stage = !DEP && row >= 0 && row + (d3 ? ngz : 0) + 1 < nrow && (s1 - s0) >= BK_STAGE;
+        if (Q) stage = stage && wir >= 1 && wir + 1 < g.nr && wiz >= 1 && wiz + 1 < ngz;
+        if (Q && stage) {
+            // the 3 x 3 rows around the central one
+            for (int i = threadIdx.x; i < 9 * na; i += BK_THREADS) {
+                const int q = i / na, j = i - q * na;
+                fw[i] = __ldg(F + (size_t)(row + (q / 3 - 1) * ngz + (q % 3 - 1)) * na + j);
+            }
+            __syncthreads();
+        } else if (stage) {
             const float4* f0 = F + (size_t)row * na;
 #pragma unroll 4
             for (int i = threadIdx.x; i < (d3 ? 4 : 2) * na; i += BK_THREADS)
@@ -376,7 +392,41 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                 if (!DEP) {
                     const CellW cw = gx_cell_t<false, ND>(g, x, y, z, true);
                     float ax, ay, az, ph;
-                    if (stage && cw.key >= 0 && cw.row == row) {
+                    if (Q && cw.key >= 0) {
+                        // grdacc.f:267-299, in the order of gx_accel_cell_t
+                        float f[3][3];
+                        gx_factors27(cw, f);
+                        const bool st = stage && cw.row == row;
+                        const int jm = (cw.jt == 0) ? na - 1 : cw.jt - 1, jp = (cw.jt == na - 1) ? 0 : cw.jt + 1;
+                        ax = ay = az = ph = 0.f;
+#pragma unroll
+                        for (int k = 0; k < 3; k++)
+#pragma unroll
+                            for (int j = 0; j < 3; j++) {
+                                const int r = cw.row + (j - 1) + (k - 1) * ngz;
+                                if (r < 0 || r >= nrow) continue;
+                                float4 v[3];
+                                if (st) {
+                                    const float4* p = fw + (3 * k + j) * na;
+                                    v[0] = p[jm];
+                                    v[1] = p[cw.jt];
+                                    v[2] = p[jp];
+                                } else {
+                                    const float4* p = F + (size_t)r * na;
+                                    v[0] = __ldg(p + jm);
+                                    v[1] = __ldg(p + cw.jt);
+                                    v[2] = __ldg(p + jp);
+                                }
+#pragma unroll
+                                for (int i = 0; i < 3; i++) {
+                                    const float w = 0.125f * f[0][i] * f[1][j] * f[2][k];
+                                    ax += v[i].x * w;
+                                    ay += v[i].y * w;
+                                    az += v[i].z * w;
+                                }
+                            }
+                        gx_rigid_force(g, x, y, z, ax, ay, az, ph);
+                    } else if (!Q && stage && cw.key >= 0 && cw.row == row) {
                         // the common case: the corners from the staged rows
                         // (in the order of gx_accel_cell_t)
                         float w[8];
@@ -395,7 +445,7 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                         }
                         gx_rigid_force(g, x, y, z, ax, ay, az, ph);
                     } else {
-                        gx_accel_cell_t<false, ND>(g, F, cw, x, y, z, ax, ay, az, ph);
+                        gx_accel_cell_t<Q, ND>(g, F, cw, x, y, z, ax, ay, az, ph);
                     }
                     float& vx = P[ND];
                     float& vy = P[ND + 1];
@@ -418,7 +468,12 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                 if (cn.key >= 0) {
                     rmin_l = min(rmin_l, cn.ju);
                     rmax_l = max(rmax_l, cn.ju);
-                    if (d3) {
+                    if (Q) {
+                        // nodes in the planes below and above; below plane 0 lies
+                        // the last plane of the ring below (flat offsets)
+                        zmin_l = min(zmin_l, max(cn.iz - 1, 0));
+                        zmax_l = max(zmax_l, cn.iz == 0 ? ngz - 1 : cn.iz);
+                    } else if (d3) {
                         // a cell in the top plane (a spoke coordinate that
                         // rounded up to na moved it there) has its upper
                         // corners in plane 0 of the next ring
@@ -479,7 +534,39 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
             // the mesh) and no negative weight: eight shared-memory adds
             int va[8];
             bool fast = false;
-            if (act && cn.key >= 0) {
+            if (Q && act && cn.key >= 0) {
+                // massgn.f:173-202
+                float f[3][3];
+                gx_factors27(cn, f);
+                const int jm = (cn.jt == 0) ? na - 1 : cn.jt - 1, jp = (cn.jt == na - 1) ? 0 : cn.jt + 1;
+                const int a0 = cn.ju - wir + WLO - 1, b0 = cn.iz - wiz + WLO - 1;  // window place of the lowest node
+                // only the middle factors can be negative (at clamped indices)
+                const bool in = win && (unsigned)a0 <= 2u && (unsigned)b0 <= 2u && cn.iz >= 1 && f[1][1] >= 0.f &&
+                                f[2][1] >= 0.f;
+                uint32_t* bw = bins + (in ? W * a0 + b0 : 0) * na;
+#pragma unroll
+                for (int k = 0; k < 3; k++)
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        int v[3];
+#pragma unroll
+                        for (int i = 0; i < 3; i++) v[i] = bk_fix(0.125f * f[0][i] * f[1][j] * f[2][k]);
+                        if (in) {
+                            uint32_t* br = bw + (W * k + j) * na;
+                            atomicAdd(br + jm, (uint32_t)v[0]);
+                            atomicAdd(br + cn.jt, (uint32_t)v[1]);
+                            atomicAdd(br + jp, (uint32_t)v[2]);
+                        } else {
+                            const int r = cn.row + (j - 1) + (k - 1) * ngz;
+                            if (r < 0 || r >= nrow) continue;  // outside the mesh: dropped, as massgn does
+                            unsigned long long* ar = acc + (size_t)r * na;
+                            if (v[0]) red_add_s64(ar + jm, v[0]);
+                            if (v[1]) red_add_s64(ar + cn.jt, v[1]);
+                            if (v[2]) red_add_s64(ar + jp, v[2]);
+                        }
+                    }
+            }
+            if (!Q && act && cn.key >= 0) {
                 float w[8];
                 gx_weights<ND>(g, cn, w);
                 int neg = 0;
@@ -504,7 +591,7 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
                     }
                 }
             }
-            if (act && cn.key >= 0 && !fast) {
+            if (!Q && act && cn.key >= 0 && !fast) {
                 const int jt0 = cn.jt, jt1 = (cn.jt == na - 1) ? 0 : cn.jt + 1;
                 // the corner rows: row, row + 1 (the next plane, or ring in
                 // 2D), and in 3D row + ngz, row + ngz + 1, with their window
@@ -573,7 +660,7 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
             __syncthreads();
 #pragma unroll 4
             for (int wr = 0; wr < WROWS; wr++) {
-                const int R = d3 ? (wir - 1 + (wr >> 2)) * ngz + (wiz - 1 + (wr & 3)) : wir - 1 + wr;
+                const int R = d3 ? (wir - WLO + wr / W) * ngz + (wiz - WLO + wr % W) : wir - 1 + wr;
                 uint32_t* br = bins + wr * na;
                 for (int j = threadIdx.x; j < na; j += BK_THREADS) {
                     const uint32_t v = br[j];
@@ -614,7 +701,8 @@ __global__ void __launch_bounds__(BK_THREADS, BK_MINB) k_push_bkt(
 __global__ void __launch_bounds__(256) k_mass_convert(unsigned long long* __restrict__ acc,
                                float* __restrict__ mass, float pm, const int32_t* __restrict__ rg, int32_t* __restrict__ rgo,
                                int32_t* __restrict__ jrk, int nr, int na,
-                               int32_t* __restrict__ zr, const int32_t* __restrict__ zro, int ngz, bool zonly) {
+                               int32_t* __restrict__ zr, const int32_t* __restrict__ zro, int ngz, bool quad,
+                               bool zonly) {
     // the active ring range of the new mass, as massgn tracks it (jrad =
     // first ring + 1, krad = min(last ring + 2, nr), 1-based), and the planes
     // holding mass (the cells' planes and the next, clamped), from the
@@ -628,7 +716,7 @@ __global__ void __launch_bounds__(256) k_mass_convert(unsigned long long* __rest
     }
     if (first) {
         const int mn = rg[0], mx = rg[1];
-        jrk[0] = (mx >= 0) ? mn + 1 : nr;
+        jrk[0] = (mx >= 0) ? mn + (quad ? 0 : 1) : nr;  // quadratic: the ring below (massgn.f:180)
         jrk[1] = (mx >= 0) ? min(mx + 2, nr) : 0;
         zr[0] = z0;
         zr[1] = z1;
@@ -777,7 +865,7 @@ __global__ void k_bk_densify(const float4* __restrict__ Qin, int64_t bcap, float
 
 // ---------------------------------------------------------------------------
 bool gx_fast_ok(const GxCtx* c) {
-    return !c->fp64 && c->nzones == 1 && !c->g.quad && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT);
+    return !c->fp64 && c->nzones == 1 && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT);
 }
 
 static inline int bk_nplanes(const GxCtx* c) { return 2 * c->g.ndim + (c->g.comp ? c->g.ndim : 0); }
@@ -1018,19 +1106,20 @@ int gx_bucket_unload(GxCtx* c, float* aos) {
     return GX_OK;
 }
 
-template <int ND, bool COMP, bool DEP = false>
+template <int ND, bool COMP, bool DEP = false, bool Q = false>
 static int bk_launch_push(GxCtx* c, int cur, int nxt) {
     const DevGeo& g = c->g;
     // the deposit window and, for the push, the staged field rows
-    const size_t sb = sizeof(uint32_t) * (ND == 3 ? 16 : 4) * g.na;
-    const size_t sf = sb + sizeof(float4) * (ND == 3 ? 4 : 2) * g.na;
+    const size_t sb = sizeof(uint32_t) * (Q ? 28 : ND == 3 ? 16 : 4) * g.na;  // 25 rows and a pad: 16-byte aligned
+    const size_t sf = sb + sizeof(float4) * (Q ? 9 : ND == 3 ? 4 : 2) * g.na;
     const size_t sm = DEP ? sb : sf;
-    auto kp = k_push_bkt<ND, COMP, DEP>;
+    auto kp = k_push_bkt<ND, COMP, DEP, Q>;
     GX_CUDA(c, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     if (!c->bk_grid) {
         int per = 0, sms = 148;
-        GX_CUDA(c, cudaFuncSetAttribute(k_push_bkt<ND, COMP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
-        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_push_bkt<ND, COMP>, BK_THREADS, sf));
+        auto kf = k_push_bkt<ND, COMP, false, Q>;
+        GX_CUDA(c, cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
+        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kf, BK_THREADS, sf));
         GX_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
         c->bk_grid = std::max(1, per) * sms;
     }
@@ -1048,7 +1137,7 @@ int gx_mass_convert(GxCtx* c) {
     const int p = c->mpar, q = p ^ 1;
     k_mass_convert<<<std::min((g.nrow + 7) / 8, 148 * 8), 256, 0, c->stream>>>(
         c->macc, c->mass, g.pmass, c->bk_ctl + 16 + 4 * p, c->bk_ctl + 16 + 4 * q, c->jrk_d, g.nr, g.na,
-        c->zr_d + 2 * p, c->zr_d + 2 * q, g.ngz, g.ndim == 3 && c->zr_valid);
+        c->zr_d + 2 * p, c->zr_d + 2 * q, g.ngz, g.quad, g.ndim == 3 && c->zr_valid);
     GX_LAUNCHED(c);
     c->mpar = q;
     return GX_OK;
@@ -1072,7 +1161,9 @@ int gx_fast_masset(GxCtx* c) {
     int rc = c->bucketed ? bk_join(c) : gx_bucketize(c);
     if (rc) return rc;
     const int cur = c->bcur, nxt = cur ^ 1;
-    if (g.ndim == 3)
+    if (g.quad)
+        rc = g.comp ? bk_launch_push<3, true, true, true>(c, cur, nxt) : bk_launch_push<3, false, true, true>(c, cur, nxt);
+    else if (g.ndim == 3)
         rc = g.comp ? bk_launch_push<3, true, true>(c, cur, nxt) : bk_launch_push<3, false, true>(c, cur, nxt);
     else
         rc = g.comp ? bk_launch_push<2, true, true>(c, cur, nxt) : bk_launch_push<2, false, true>(c, cur, nxt);
@@ -1099,7 +1190,9 @@ static int fast_one_step(GxCtx* c, bool lpot) {
     if (rc) return rc;
     rc = gx_phase_mark(c, PH_PUSH);
     if (rc) return rc;
-    if (g.ndim == 3) rc = g.comp ? bk_launch_push<3, true>(c, cur, nxt) : bk_launch_push<3, false>(c, cur, nxt);
+    if (g.quad)
+        rc = g.comp ? bk_launch_push<3, true, false, true>(c, cur, nxt) : bk_launch_push<3, false, false, true>(c, cur, nxt);
+    else if (g.ndim == 3) rc = g.comp ? bk_launch_push<3, true>(c, cur, nxt) : bk_launch_push<3, false>(c, cur, nxt);
     else rc = g.comp ? bk_launch_push<2, true>(c, cur, nxt) : bk_launch_push<2, false>(c, cur, nxt);
     if (rc) return rc;
     if (c->prof) {

@@ -252,7 +252,7 @@ struct CellW {
     int key;      // ncl - 1, or -1 when off the grid / in the hole
     float du, dt, dz;  // fractions in the cell; quadratic: coord + 1/2 - index
     int row, jt;  // ring-plane row and spoke of key (set by gx_cell)
-    int ju, iz;   // ring and plane of row (linear scheme; row = ju * ngz + iz)
+    int ju, iz;   // ring and plane of row (row = ju * ngz + iz)
 };
 
 // floor of a float in [0, 2^23) and the exact fraction v - floor(v), on the
@@ -340,6 +340,8 @@ __device__ __forceinline__ CellW gx_cell27(const DevGeo& g, float u, float t, fl
     jz = min(max(jz, 0), g.ngz - 2);
     c.du = uh - gx_i2f(ju);
     c.dz = zh - gx_i2f(jz);
+    c.ju = ju;
+    c.iz = jz;
     c.row = ju * g.ngz + jz;
     c.jt = (jt == g.na) ? 0 : jt;
     c.key = c.row * g.na + c.jt;
@@ -490,16 +492,20 @@ __device__ __forceinline__ int gx_div_na(const DevGeo& g, int v, int& r) {
 // 27 quadratic weights (weight.f:299-311): per axis (1 - 2dd + dd^2,
 // 1 + 2dd - 2dd^2, dd^2); weight l = 9 k + 3 j + i (theta i fastest, then z
 // j, then u k) = 1/8 f_theta(i) f_z(j) f_u(k)
-__device__ __forceinline__ void gx_weights27(const CellW& c, float* w) {
-    float f[3][3];
+__device__ __forceinline__ void gx_factors27(const CellW& c, float (*f)[3]) {
     const float d[3] = {c.dt, c.dz, c.du};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        const float dd = d[a], d2 = dd * dd;
-        f[a][0] = (1.f - 2.f * dd) + d2;
-        f[a][1] = (1.f + 2.f * dd) - 2.f * d2;
+        // explicit roundings: every pass forms the same bits
+        const float dd = d[a], d2 = __fmul_rn(dd, dd);
+        f[a][0] = __fadd_rn(__fmaf_rn(-2.f, dd, 1.f), d2);
+        f[a][1] = __fmaf_rn(-2.f, d2, __fmaf_rn(2.f, dd, 1.f));
         f[a][2] = d2;
     }
+}
+__device__ __forceinline__ void gx_weights27(const CellW& c, float* w) {
+    float f[3][3];
+    gx_factors27(c, f);
 #pragma unroll
     for (int k = 0; k < 3; k++)
 #pragma unroll
@@ -717,7 +723,7 @@ int gx_zone_masset(GxCtx* c);
 int gx_zone_step(GxCtx* c, int nsteps, int phys);
 int gx_comm_reduce_range(GxCtx* c);
 // fused step on the bucketed store (gx_bucket.cu)
-bool gx_fast_ok(const GxCtx* c);  // single zone, linear scheme, mixed, not GX_FLAG_SORTED_DEPOSIT
+bool gx_fast_ok(const GxCtx* c);  // single zone, mixed, not GX_FLAG_SORTED_DEPOSIT
 int gx_fast_step(GxCtx* c, int nsteps, int phys);
 int gx_dense(GxCtx* c);  // bucketed store -> dense store (no-op when dense)
 int gx_bucket_unload(GxCtx* c, float* aos);  // unload from the bucketed store

@@ -12,7 +12,7 @@ grid); the 3D benchmark grid; a context with no particles."""
 import numpy as np
 import pytest
 
-from galaxy_b200 import (Galaxy, make_config, GX_FLAG_COMPENSATED, GX_FLAG_SORTED_DEPOSIT,
+from galaxy_b200 import (Galaxy, make_config, GX_FLAG_COMPENSATED, GX_FLAG_QUADRATIC, GX_FLAG_SORTED_DEPOSIT,
                          GX_RMAP_LOG, GX_RMAP_STDPOL, GX_GRID_MASS)
 from galaxy_b200.disk import kt_disk
 
@@ -48,6 +48,15 @@ def case(name):
         rec = rec.copy()
         rec[:, 2:] *= 25.0
         return cfg2(), rec, pm, 0
+    if name.startswith("3d-quadratic"):
+        nr, na, ngz = (32, 64, 15) if name == "3d-quadratic" else (29, 50, 27)
+        rec, pm = kt_disk(200_000 if name == "3d-quadratic" else 60_000, seed=6, rmax=4.5, ndim=3, z0=0.1, dt=0.025)
+        rec = rec.copy()
+        rec[::40, 2] *= 6.0    # to the lowest and highest planes, and off the grid
+        rec[::30, :2] *= 0.1   # to the clamped inner ring and the hole
+        rec[::50, 3:] *= 20.0  # several cells per step
+        flags = GX_FLAG_QUADRATIC | (0 if name == "3d-quadratic" else GX_FLAG_COMPENSATED)
+        return cfg3(nr=nr, na=na, ngz=ngz), rec, pm, flags
     if name == "bench3":
         rec, pm = kt_disk(1_000_000, seed=12345, rmax=4.8, ndim=3, z0=0.1, dt=0.02)
         return cfg3(nr=128, na=256, ngz=125, dzg=0.04, ng=17, softl=0.1), rec, pm, 0
@@ -82,7 +91,8 @@ def run(cfg, rec, pm, flags):
 
 
 @pytest.mark.parametrize("name", ["3d", "2d", "3d-compensated", "3d-fast-movers",
-                                  "2d-fast-movers", "bench3"])
+                                  "2d-fast-movers", "bench3", "3d-quadratic",
+                                  "3d-quadratic-compensated"])
 def test_fused_step_is_bitwise_the_sorted_deposit(name):
     cfg, rec, pm, flags = case(name)
     a = run(cfg, rec, pm, flags)
