@@ -470,7 +470,7 @@ __global__ void k_adj_scatter(const float4* __restrict__ S, int64_t n, float* __
 // the deposited accumulator -> the mass, then its field
 static int adj_solve(GxCtx* c) {
     c->zr_valid = false;  // the mass array is no longer a fused pass's
-    int rc = gx_mass_convert(c);
+    int rc = gx_mass_defer(c);
     if (rc) return rc;
     return gx_mixed_findf(c, 0, true);
 }

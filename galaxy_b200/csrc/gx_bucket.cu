@@ -1143,6 +1143,14 @@ int gx_mass_convert(GxCtx* c) {
     return GX_OK;
 }
 
+// 2D: the forward transform converts its ring itself (gx_mixed_findf, which
+// has to come next).  Not across ranks, which reduce the ring range first.
+int gx_mass_defer(GxCtx* c) {
+    if (c->g.ndim != 2 || c->nranks > 1 || c->prof) return gx_mass_convert(c);
+    c->acc_pending = true;
+    return GX_OK;
+}
+
 // the main stream waits for the plan queued on the side stream
 static int bk_join(GxCtx* c) {
     if (!c->bk_pending) return GX_OK;
@@ -1178,7 +1186,8 @@ int gx_fast_masset(GxCtx* c) {
 
 // one fused step: the solve of the current mass (only the planes that hold
 // it once they are known), the pass, its plan on the side stream, the mass
-static int fast_one_step(GxCtx* c, bool lpot) {
+// (left to the next step's solve in 2D, except after the last step of a call)
+static int fast_one_step(GxCtx* c, bool lpot, bool last) {
     const DevGeo& g = c->g;
     // once the mass is a fused pass's, the solve knows the planes that
     // hold it, and the field is needed only where the particles are
@@ -1213,7 +1222,7 @@ static int fast_one_step(GxCtx* c, bool lpot) {
     }
     rc = gx_phase_mark(c, PH_COMBINE);
     if (rc) return rc;
-    rc = gx_mass_convert(c);
+    rc = last ? gx_mass_convert(c) : gx_mass_defer(c);
     if (rc) return rc;
     c->zr_valid = true;
     c->bcur = nxt;
@@ -1241,7 +1250,7 @@ static cudaGraphExec_t fast_capture(GxCtx* c, int64_t* per) {
         cudaGetLastError();
         return nullptr;
     }
-    bool ok = fast_one_step(c, false) == GX_OK && fast_one_step(c, false) == GX_OK && bk_join(c) == GX_OK;
+    bool ok = fast_one_step(c, false, false) == GX_OK && fast_one_step(c, false, false) == GX_OK && bk_join(c) == GX_OK;
     const cudaError_t ec = cudaStreamEndCapture(c->stream, &graph);
     ok = ok && ec == cudaSuccess && graph;
     if (ok) ok = cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
@@ -1250,6 +1259,7 @@ static cudaGraphExec_t fast_capture(GxCtx* c, int64_t* per) {
     *per = c->launches - l0;
     c->bcur = b;
     c->mpar = mp;
+    c->acc_pending = true;  // as it was: the caller captures after a deferred step
     c->bk_pending = false;
     c->launches = l0;
     c->err.clear();
@@ -1281,7 +1291,7 @@ int gx_fast_step(GxCtx* c, int nsteps, int phys) {
     while (s < nsteps) {
         const bool last = (s == nsteps - 1);
         const int pairs = (nsteps - s - 1) / 2;  // the last step runs as plain launches (phys)
-        if (graphs && c->zr_valid && pairs >= 4 && !tried) {
+        if (graphs && c->zr_valid && c->acc_pending && pairs >= 4 && !tried) {
             tried = true;
             exec = fast_capture(c, &per);
         }
@@ -1296,7 +1306,7 @@ int gx_fast_step(GxCtx* c, int nsteps, int phys) {
             s += 2 * pairs;
             continue;
         }
-        rc = fast_one_step(c, phys && last);
+        rc = fast_one_step(c, phys && last, last);
         if (rc) break;
         s++;
     }

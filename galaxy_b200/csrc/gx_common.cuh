@@ -186,6 +186,7 @@ struct GxCtx {
     int bk_item = BK_ITEM;                   // particles per work item of the fused pass
     int32_t* bk_cnt = nullptr;               // [nrow + 1] row counts of the dense store (bucketing)
     unsigned long long* macc = nullptr;      // [mesh] fixed-point mass (2^-20 of a particle), zero between steps
+    bool acc_pending = false;                // the mass is still in macc: the next 2D solve converts it
     int32_t* zr_d = nullptr;                 // [2][2] first, last plane holding the fused pass's mass
                                              // (ngz, -1 when empty), at 2 p of the conversion of set p
     bool zr_valid = false;                   // the mass array is the fused pass's (zr_d describes it)
@@ -729,6 +730,7 @@ int gx_dense(GxCtx* c);  // bucketed store -> dense store (no-op when dense)
 int gx_bucket_unload(GxCtx* c, float* aos);  // unload from the bucketed store
 int gx_fast_masset(GxCtx* c);  // masset by the deposit-only fused pass
 static inline int32_t* gx_mass_ranges(const GxCtx* c) { return c->bk_ctl + 16 + 4 * c->mpar; }  // of the next deposit
+int gx_mass_defer(GxCtx* c);    // leave that to the next solve where it can (2D), else do it
 int gx_mass_convert(GxCtx* c);  // mass accumulator -> mass array (accumulator cleared)
 int gx_bucket_alloc(GxCtx* c);
 int gx_bucket_words(const GxCtx* c);  // float4 words per record of the bucketed store

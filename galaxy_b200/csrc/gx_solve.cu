@@ -632,13 +632,38 @@ static size_t fwd_ring_smem(const DevGeo& g, const Spec& sp) {
 #define F2_H 16
 #define F2_Q 16
 #define F2_THREADS (F2_H * F2_Q)
-__global__ void __launch_bounds__(F2_THREADS) k_fwd2(DevGeo g, int nact, int ncp, const float* __restrict__ mass,
-                                                     const float* __restrict__ Taz, float4* __restrict__ S) {
+// ACC: the mass is still the deposit's integers; the ring's CTA converts them
+// as k_mass_convert does, writes the mass, clears the accumulator and keeps the
+// ring ranges (a launch of 2 us and its gap less per step).
+template <bool ACC>
+__global__ void __launch_bounds__(F2_THREADS) k_fwd2(DevGeo g, int nact, int ncp, float* __restrict__ mass,
+                                                     const float* __restrict__ Taz, float4* __restrict__ S,
+                                                     unsigned long long* __restrict__ acc,
+                                                     const int32_t* __restrict__ rg, int32_t* __restrict__ rgo,
+                                                     int32_t* __restrict__ jrk) {
     extern __shared__ __align__(16) float sm[];
     __shared__ float2 part[F2_Q][F2_H];
     const int na = g.na, nr = g.nr, ir = blockIdx.x;
     float* x = sm;  // [na]
-    for (int j = threadIdx.x; j < na; j += blockDim.x) x[j] = __ldg(mass + (size_t)ir * na + j);
+    if (ACC) {
+        for (int j = threadIdx.x; j < na; j += blockDim.x) {
+            const size_t i = (size_t)ir * na + j;
+            const unsigned long long v = acc[i];
+            const float m = (float)((double)(long long)v * (1.0 / 1048576.0)) * g.pmass;
+            x[j] = m;
+            mass[i] = m;
+            if (v) acc[i] = 0ull;
+        }
+        if (ir == 0 && threadIdx.x == 0) {
+            const int mn = rg[0], mx = rg[1];
+            jrk[0] = (mx >= 0) ? mn + 1 : nr;
+            jrk[1] = (mx >= 0) ? min(mx + 2, nr) : 0;
+            rgo[0] = rgo[2] = 0x7fffffff;
+            rgo[1] = rgo[3] = -1;
+        }
+    } else {
+        for (int j = threadIdx.x; j < na; j += blockDim.x) x[j] = mass[(size_t)ir * na + j];
+    }
     __syncthreads();
     const int h = threadIdx.x % F2_H, q = threadIdx.x / F2_H;
     for (int a0 = 0; a0 < nact; a0 += F2_H) {
@@ -844,8 +869,13 @@ int gx_mixed_findf(GxCtx* c, int lpot, bool polcat_only_field, const int32_t* fr
             GX_LAUNCHED(c);
         }
         const size_t sm = sizeof(float) * (size_t)g.na;
-        GX_CUDA(c, cudaFuncSetAttribute(k_fwd2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        k_fwd2<<<g.nr, F2_THREADS, sm, c->stream>>>(g, nact, ncp, c->mass, c->fwdtab, c->specS);
+        auto kf = c->acc_pending ? k_fwd2<true> : k_fwd2<false>;
+        kf<<<g.nr, F2_THREADS, sm, c->stream>>>(g, nact, ncp, c->mass, c->fwdtab, c->specS, c->macc, gx_mass_ranges(c),
+                                                c->bk_ctl + 16 + 4 * (c->mpar ^ 1), c->jrk_d);
+        if (c->acc_pending) {
+            c->acc_pending = false;
+            c->mpar ^= 1;
+        }
         GX_LAUNCHED(c);
     }
     rc = gx_comm_reduce_spectrum(c);
