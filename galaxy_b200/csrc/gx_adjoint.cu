@@ -54,7 +54,7 @@ __device__ __forceinline__ bool adj_wgrad(const DevGeo& g, float x, float y, Cel
 }
 
 // acceleration at (x, y) from the Cartesian field and the halo (grdacc + halfrc)
-__device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* __restrict__ F, const CellW& cw,
+__device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* F, const CellW& cw,
                                           const float* w, float x, float y, float& ax, float& ay) {
     ax = ay = 0.f;
     if (cw.key < 0) return;
@@ -63,7 +63,7 @@ __device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* __restr
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (ic[k] < 0) continue;
-        const float4 f = __ldg(F + ic[k]);
+        const float4 f = F[ic[k]];
         ax += f.x * w[k];
         ay += f.y * w[k];
     }
@@ -140,12 +140,13 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_mass(DevGeo g, const float4* __r
 
 // forward step: v += a(x); x += v (stpgrp.f:26-32); the new position deposited
 __global__ void __launch_bounds__(ADJ_BS) k_adj_fwd(DevGeo g, float4* __restrict__ S, int64_t n,
-                                                    const float4* __restrict__ F,
+                                                    const float4* F,
                                                     unsigned long long* __restrict__ acc,
                                                     int32_t* __restrict__ rng) {
+    gx_chain();
     int rlo = 0x7fffffff, rhi = -1;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 s = S[i];
+        float4 s = __ldcg(S + i);
         const CellW cw = gx_cell_t<true, 2>(g, s.x, s.y, 0.f, true);
         float w[8];
         if (cw.key >= 0) gx_weights<2>(g, cw, w);
@@ -218,12 +219,13 @@ __global__ void k_adj_init(const float4* __restrict__ S, int64_t n, double a2r, 
 // slope . (F . mu) + halo Jacobian . mu, Q += W mu (x and y of a cell side
 // by side), halo parameter terms
 __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float4* __restrict__ S, float4* __restrict__ L,
-                                                  int64_t n, const float4* __restrict__ F, int kick,
+                                                  int64_t n, const float4* F, int kick,
                                                   double* __restrict__ Q, double* __restrict__ tpart) {
+    gx_chain();
     __shared__ double sh[2][ADJ_BS / 32];
     double drc = 0.0, dv2 = 0.0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 s = S[i], l = L[i];
+        float4 s = __ldcg(S + i), l = __ldcg(L + i);
         const float x = s.x, y = s.y;
         CellW cw;
         float w[8], dw[4][2];
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float4* __restrict__
 #pragma unroll
             for (int k = 0; k < 4; k++) {
                 if (ic[k] < 0) continue;
-                const float4 f = __ldg(F + ic[k]);
+                const float4 f = F[ic[k]];
                 const float fdot = f.x * m0 + f.y * m1;
                 lx += dw[k][0] * fdot;
                 ly += dw[k][1] * fdot;
@@ -282,8 +284,8 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float4* __restrict__
             b += sh[1][w];
         }
         // each block owns its slot and the steps run in order: deterministic
-        tpart[2 * blockIdx.x] += a;
-        tpart[2 * blockIdx.x + 1] += b;
+        tpart[2 * blockIdx.x] = __ldcg(tpart + 2 * blockIdx.x) + a;
+        tpart[2 * blockIdx.x + 1] = __ldcg(tpart + 2 * blockIdx.x + 1) + b;
     }
 }
 
@@ -294,13 +296,14 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_a(DevGeo g, float4* __restrict__
 //   floats as ordered integers: order-free), then the checkpoint itself; the
 //   position deposited for the next solve.
 __global__ void __launch_bounds__(ADJ_BS) k_adj_b(DevGeo g, float4* __restrict__ S, float4* __restrict__ L, int64_t n,
-                                                  const float* __restrict__ psi, float pmass, int move,
+                                                  const float* psi, float pmass, int move,
                                                   const float4* __restrict__ ck, unsigned int* __restrict__ drift,
                                                   unsigned long long* __restrict__ acc, int32_t* __restrict__ rng) {
+    gx_chain();
     int rlo = 0x7fffffff, rhi = -1;
     float dm = 0.f;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        float4 s = S[i];
+        float4 s = __ldcg(S + i);
         if (psi) {
             CellW cw;
             float w[8], dw[4][2];
@@ -311,12 +314,12 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_b(DevGeo g, float4* __restrict__
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     if (ic[k] < 0) continue;
-                    const float p = __ldg(psi + ic[k]);
+                    const float p = psi[ic[k]];
                     gx += dw[k][0] * p;
                     gy += dw[k][1] * p;
                 }
                 float2* l = reinterpret_cast<float2*>(L + i);
-                const float2 v = *l;
+                const float2 v = __ldcg(l);
                 *l = make_float2(v.x + pmass * gx, v.y + pmass * gy);
             }
         }
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(ADJ_BS) k_adj_b(DevGeo g, float4* __restrict__
         s.x -= s.z;
         s.y -= s.w;
         if (ck) {
-            const float4 c = __ldg(ck + i);
+            const float4 c = __ldcg(ck + i);
             dm = fmaxf(dm, fmaxf(fabsf(s.x - c.x), fabsf(s.y - c.y)));
             s = c;
         }
@@ -360,12 +363,14 @@ struct AdjAct {
 __global__ void __launch_bounds__(AT_H * AT_Q) k_adjt_syn(DevGeo g, AdjAct act, int nact, int ncp,
                                                           double2* __restrict__ Q, const float* __restrict__ T,
                                                           float2* __restrict__ V) {
+    gx_chain();
     extern __shared__ __align__(16) float2 gv[];  // [na]: radial, azimuthal
     __shared__ float4 part[AT_Q][AT_H];
     const int nr = g.nr, na = g.na, ir = blockIdx.x;
     for (int j = threadIdx.x; j < na; j += blockDim.x) {
         double2* q = Q + (size_t)ir * na + j;
-        const float qx = (float)q->x, qy = (float)q->y;
+        const double2 qv = __ldcg(q);
+        const float qx = (float)qv.x, qy = (float)qv.y;
         *q = make_double2(0.0, 0.0);
         float sn, cs;
         sincospif(2.0f * (float)j / (float)na, &sn, &cs);
@@ -412,6 +417,7 @@ __global__ void __launch_bounds__(AT_H * AT_Q) k_adjt_syn(DevGeo g, AdjAct act, 
 __global__ void __launch_bounds__(ADJ_BS) k_adjt_conv(DevGeo g, AdjAct act, int nact, int ncp,
                                                       const float* __restrict__ G, const float2* __restrict__ V,
                                                       const float* __restrict__ T, float* __restrict__ psi) {
+    gx_chain();
     __shared__ float2 AB[64];
     const int lane = threadIdx.x & 31, nr = g.nr, na = g.na, is = blockIdx.x;
     for (int a = threadIdx.x >> 5; a < nact; a += ADJ_BS / 32) {
@@ -426,12 +432,12 @@ __global__ void __launch_bounds__(ADJ_BS) k_adjt_conv(DevGeo g, AdjAct act, int 
 #pragma unroll 4
         for (int ir = lane; ir < nr; ir += 32) {
             const float g0 = __ldg(G0 + ir);
-            const float2 v0 = __ldg(V0 + ir);
+            const float2 v0 = __ldcg(V0 + ir);
             sa += g0 * v0.x;
             if (hasb) sb += g0 * v0.y;
             if (ft) {
                 const float g1 = __ldg(G1 + ir);
-                const float2 v1 = __ldg(V1 + ir);
+                const float2 v1 = __ldcg(V1 + ir);
                 sb += g1 * v1.x;
                 sa -= g1 * v1.y;
             }
@@ -552,7 +558,7 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     for (int s = 0; s < nsteps; s++) {
         int rc = adj_solve(c);
         if (rc) return rc;
-        k_adj_fwd<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->field, c->macc, gx_mass_ranges(c));
+        GX_CUDA(c, gx_launch_chain(k_adj_fwd, np, ADJ_BS, 0, st, g, b.S, n, c->field, c->macc, gx_mass_ranges(c)));
         GX_LAUNCHED(c);
         if ((s + 1) % ckpt_every == 0)
             GX_CUDA(c, cudaMemcpyAsync(b.ck + (size_t)((s + 1) / ckpt_every) * n, b.S, sbytes,
@@ -585,16 +591,20 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     for (int s = nsteps - 1; s >= 0; s--) {
         const bool ck = (s % ckpt_every) == 0;
         // the psi term of step s + 1, the drift back to x_s and its deposit
-        k_adj_b<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, s == nsteps - 1 ? nullptr : b.psi, g.pmass, 1,
-                                       ck ? b.ck + (size_t)(s / ckpt_every) * n : nullptr, b.drift, c->macc, gx_mass_ranges(c));
+        GX_CUDA(c, gx_launch_chain(k_adj_b, np, ADJ_BS, 0, st, g, b.S, b.L, n, s == nsteps - 1 ? nullptr : b.psi, g.pmass,
+                                   1, ck ? b.ck + (size_t)(s / ckpt_every) * n : nullptr, b.drift, c->macc,
+                                   gx_mass_ranges(c)));
         GX_LAUNCHED(c);
         int rc = adj_solve(c);
         if (rc) return rc;
-        k_adj_a<<<np, ADJ_BS, 0, st>>>(g, b.S, b.L, n, c->field, ck ? 0 : 1, reinterpret_cast<double*>(b.Q), b.tpart);
+        GX_CUDA(c, gx_launch_chain(k_adj_a, np, ADJ_BS, 0, st, g, b.S, b.L, n, c->field, ck ? 0 : 1,
+                                   reinterpret_cast<double*>(b.Q), b.tpart));
         GX_LAUNCHED(c);
-        k_adjt_syn<<<g.nr, AT_H * AT_Q, sizeof(float2) * g.na, st>>>(g, act, nact, ncp, b.Q, c->fwdtab, b.V);
+        GX_CUDA(c, gx_launch_chain(k_adjt_syn, g.nr, AT_H * AT_Q, sizeof(float2) * g.na, st, g, act, nact, ncp, b.Q,
+                                   c->fwdtab, b.V));
         GX_LAUNCHED(c);
-        k_adjt_conv<<<g.nr, ADJ_BS, 0, st>>>(g, act, nact, ncp, c->green32, b.V, c->fwdtab, b.psi);
+        GX_CUDA(c, gx_launch_chain(k_adjt_conv, g.nr, ADJ_BS, 0, st, g, act, nact, ncp, c->green32, b.V, c->fwdtab,
+                                   b.psi));
         GX_LAUNCHED(c);
     }
     if (nsteps > 0) {

@@ -626,7 +626,12 @@ __device__ __forceinline__ void gx_rigid_force(const DevGeo& g, float x, float y
 
 // interpolated acceleration and potential of a particle at (x, y, z) whose
 // interpolation cell is cw: grdacc + halfrc (or the fixed disc force)
-template <bool Q, int ND = 0>
+// (CG: the field read past the first-level cache, see gx_chain)
+template <bool CG>
+__device__ __forceinline__ float4 gx_ld4(const float4* p) {
+    return CG ? __ldcg(p) : __ldg(p);
+}
+template <bool Q, int ND = 0, bool CG = false>
 __device__ __forceinline__ void gx_accel_cell_t(const DevGeo& g, const float4* __restrict__ F,
                                                 const CellW& cw, float x, float y, float z,
                                                 float& ax, float& ay, float& az, float& ph) {
@@ -643,7 +648,7 @@ __device__ __forceinline__ void gx_accel_cell_t(const DevGeo& g, const float4* _
 #pragma unroll
         for (int k = 0; k < 27; k++) {
             if (ic[k] < 0) continue;
-            const float4 f = __ldg(F + ic[k]);
+            const float4 f = gx_ld4<CG>(F + ic[k]);
             ax += f.x * w[k];
             ay += f.y * w[k];
             az += f.z * w[k];
@@ -657,7 +662,7 @@ __device__ __forceinline__ void gx_accel_cell_t(const DevGeo& g, const float4* _
         gx_corners_rt<ND>(g, cw.key, cw.jt, ic);
         float4 f[NC];
 #pragma unroll
-        for (int k = 0; k < NC; k++) f[k] = (ic[k] >= 0) ? __ldg(F + ic[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < NC; k++) f[k] = (ic[k] >= 0) ? gx_ld4<CG>(F + ic[k]) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < NC; k++) {
             ax += f[k].x * w[k];
@@ -690,6 +695,34 @@ __device__ __forceinline__ void gx_accel_cell(const DevGeo& g, const float4* __r
 }
 
 // ---------------------------------------------------------------------------
+// Launches of the short kernels of a solve and of the particle passes around it
+// overlap their start with the end of the kernel before them (programmatic
+// dependent launch): a kernel lets its successor start at once, and waits, before
+// it touches memory, until everything before it has completed.  Data another
+// kernel of the chain wrote is read past the first-level cache, or (gathers that
+// gain from that cache) with ordinary loads, never through the read-only path.
+// Zoned step of 15000 particles, five launches: 26.6 -> 20.5 us; adjoint of 400k
+// particles on 128 x 256, 13 launches a step: 126.5 -> 117.4 us.
+__device__ __forceinline__ void gx_chain() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+static inline cudaError_t gx_launch_chain(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... a) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, static_cast<P>(a)...);
+}
+
 // host-side entry points implemented in the .cu files
 int setgrd(const GxConfig* c, GxGeometry* g, std::string& err);
 void fill_devgeo(GxCtx* c);

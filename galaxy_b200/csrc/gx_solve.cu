@@ -643,26 +643,27 @@ __global__ void __launch_bounds__(F2_THREADS) k_fwd2(DevGeo g, int nact, int ncp
                                                      int32_t* __restrict__ jrk) {
     extern __shared__ __align__(16) float sm[];
     __shared__ float2 part[F2_Q][F2_H];
+    gx_chain();
     const int na = g.na, nr = g.nr, ir = blockIdx.x;
     float* x = sm;  // [na]
     if (ACC) {
         for (int j = threadIdx.x; j < na; j += blockDim.x) {
             const size_t i = (size_t)ir * na + j;
-            const unsigned long long v = acc[i];
+            const unsigned long long v = __ldcg(acc + i);
             const float m = (float)((double)(long long)v * (1.0 / 1048576.0)) * g.pmass;
             x[j] = m;
             mass[i] = m;
             if (v) acc[i] = 0ull;
         }
         if (ir == 0 && threadIdx.x == 0) {
-            const int mn = rg[0], mx = rg[1];
+            const int mn = __ldcg(rg), mx = __ldcg(rg + 1);
             jrk[0] = (mx >= 0) ? mn + 1 : nr;
             jrk[1] = (mx >= 0) ? min(mx + 2, nr) : 0;
             rgo[0] = rgo[2] = 0x7fffffff;
             rgo[1] = rgo[3] = -1;
         }
     } else {
-        for (int j = threadIdx.x; j < na; j += blockDim.x) x[j] = mass[(size_t)ir * na + j];
+        for (int j = threadIdx.x; j < na; j += blockDim.x) x[j] = __ldcg(mass + (size_t)ir * na + j);
     }
     __syncthreads();
     const int h = threadIdx.x % F2_H, q = threadIdx.x / F2_H;
@@ -720,11 +721,12 @@ __global__ void __launch_bounds__(256) k_conv(DevGeo g, int nact, int tmask,
                                               float4* __restrict__ O,
                                               const int32_t* __restrict__ jrk) {
     extern __shared__ __align__(16) float4 sh4[];
+    gx_chain();
     const int nr = g.nr, nkz = g.nkz, ng = g.ng, mmax = g.mmax, ngz = g.ngz;
     const int t = blockIdx.z & 3, ir0 = (blockIdx.z >> 2) * NC * 32;
     if (!((tmask >> t) & 1)) return;
     // source rings jrs..krs (p3conv.f:149-150)
-    const int js = max(jrk[0], 1) - 1, ks = min(jrk[1], nr) - 1;
+    const int js = max(__ldcg(jrk), 1) - 1, ks = min(__ldcg(jrk + 1), nr) - 1;
     const int a = blockIdx.x, k = blockIdx.y, m = g.act[a];
     const int rings = min(NC * 32, nr - ir0);
     // ring-major output [t][ir][kz][a] (read as one block per ring by the synthesis)
@@ -740,7 +742,7 @@ __global__ void __launch_bounds__(256) k_conv(DevGeo g, int nact, int tmask,
     float4* Sin = sh4;              // [nr]
     float4* part = sh4 + nr;        // [8][32 NC]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = js + threadIdx.x; i <= ks; i += blockDim.x) Sin[i] = S[((size_t)a * nkz + k) * nr + i];
+    for (int i = js + threadIdx.x; i <= ks; i += blockDim.x) Sin[i] = __ldcg(S + ((size_t)a * nkz + k) * nr + i);
     __syncthreads();
     const float* Gt = G + ((((size_t)t * ng + m) * nkz + k) * nr) * (size_t)nr + ir0 + lane;
     float4 acc[NC];
@@ -870,8 +872,8 @@ int gx_mixed_findf(GxCtx* c, int lpot, bool polcat_only_field, const int32_t* fr
         }
         const size_t sm = sizeof(float) * (size_t)g.na;
         auto kf = c->acc_pending ? k_fwd2<true> : k_fwd2<false>;
-        kf<<<g.nr, F2_THREADS, sm, c->stream>>>(g, nact, ncp, c->mass, c->fwdtab, c->specS, c->macc, gx_mass_ranges(c),
-                                                c->bk_ctl + 16 + 4 * (c->mpar ^ 1), c->jrk_d);
+        GX_CUDA(c, gx_launch_chain(kf, g.nr, F2_THREADS, sm, c->stream, g, nact, ncp, c->mass, c->fwdtab, c->specS,
+                                   c->macc, gx_mass_ranges(c), c->bk_ctl + 16 + 4 * (c->mpar ^ 1), c->jrk_d));
         if (c->acc_pending) {
             c->acc_pending = false;
             c->mpar ^= 1;
@@ -895,8 +897,8 @@ int gx_mixed_findf(GxCtx* c, int lpot, bool polcat_only_field, const int32_t* fr
         const size_t sm = sizeof(float4) * ((size_t)g.nr + 8 * 32 * nc);
         auto kc = nc == 1 ? k_conv<1> : nc == 2 ? k_conv<2> : nc == 3 ? k_conv<3> : k_conv<4>;
         GX_CUDA(c, cudaFuncSetAttribute(kc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-        kc<<<dim3(nact, g.nkz, 4 * ((nch + nc - 1) / nc)), 256, sm, c->stream>>>(g, nact, tmask, c->green32, c->specS,
-                                                                                c->specO, c->jrk_d);
+        GX_CUDA(c, gx_launch_chain(kc, dim3(nact, g.nkz, 4 * ((nch + nc - 1) / nc)), 256, sm, c->stream, g, nact, tmask,
+                                   c->green32, c->specS, c->specO, c->jrk_d));
         GX_LAUNCHED(c);
     }
     rc = gx_phase_mark(c, PH_SYN);

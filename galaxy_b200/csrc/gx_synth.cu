@@ -825,16 +825,17 @@ __global__ void __launch_bounds__(SYNAZ_THREADS) k_synaz(DevGeo g, int nact, int
                                               const int32_t* __restrict__ zr,
                                               const float4* __restrict__ O2) {
     extern __shared__ __align__(16) float sm[];
+    gx_chain();
     const int ir = blockIdx.x, zb = blockIdx.y * SYN_ZB;
-    if (frk && (ir + 1 < frk[0] || ir + 1 > frk[1])) return;  // rings no moving particle reads
+    if (frk && (ir + 1 < __ldcg(frk) || ir + 1 > __ldcg(frk + 1))) return;  // rings no moving particle reads
     const int nr = g.nr, ngz = g.ngz, na = g.na, njp = tb.njp;
     // with zr, only the planes the next particle pass reads: those holding
     // mass, one wider each side (a particle's interpolation cell may sit one
     // plane off its deposit cell); the block's planes [zb0, zb1)
     int zb0 = zb, zb1 = min(zb + SYN_ZB, ngz);
     if (zr) {
-        zb0 = max(zb0, zr[0] - 1);
-        zb1 = min(zb1, zr[1] + 2);
+        zb0 = max(zb0, __ldcg(zr) - 1);
+        zb1 = min(zb1, __ldcg(zr + 1) + 2);
         if (zb1 <= zb0) return;
     }
     const int nz = zb1 - zb0;
@@ -875,11 +876,11 @@ __global__ void __launch_bounds__(SYNAZ_THREADS) k_synaz(DevGeo g, int nact, int
                     // part): column 2a the cosine term, 2a + 1 the sine term
                     const int a = c >> 1;
                     if (a < nact) {
-                        const float4 o = __ldg(O2 + ((size_t)t * nr + ir) * nact + a);
+                        const float4 o = __ldcg(O2 + ((size_t)t * nr + ir) * nact + a);
                         v[u] = (c & 1) ? o.z : o.x;
                     }
                 } else {
-                    v[u] = __ldg(R + (((size_t)t * nr + ir) * ngz + zb0 + z) * ncp + c);
+                    v[u] = __ldcg(R + (((size_t)t * nr + ir) * ngz + zb0 + z) * ncp + c);
                 }
             }
         }
@@ -1007,9 +1008,9 @@ int gx_synthesis(GxCtx* c, int tmask, float* polar, const int32_t* frk, const in
         GX_CUDA(c, cudaFuncSetAttribute(k_synaz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
         dim3 grid(g.nr, (g.ngz + SYN_ZB - 1) / SYN_ZB);
         // 2D has no vertical part: the azimuthal synthesis reads the contracted spectrum
-        k_synaz<<<grid, SYNAZ_THREADS, sm, c->stream>>>(g, nact, ncp, tmask, c->synR, tb, c->field, polar, frk,
-                                                        g.ndim == 3 ? zr : nullptr,
-                                                        g.ndim == 3 ? nullptr : c->specO);
+        GX_CUDA(c, gx_launch_chain(k_synaz, grid, SYNAZ_THREADS, sm, c->stream, g, nact, ncp, tmask, c->synR, tb,
+                                   c->field, polar, frk, g.ndim == 3 ? zr : nullptr,
+                                   g.ndim == 3 ? nullptr : c->specO));
         GX_LAUNCHED(c);
     }
     return GX_OK;

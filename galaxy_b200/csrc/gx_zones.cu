@@ -208,18 +208,19 @@ struct ZoneSrc {
 __device__ __forceinline__ void zone_ranges(int nz, int nr, int mz, int32_t* __restrict__ zjrk,
                                             int32_t* __restrict__ jrk) {
     int jrs = nr, krs = 0;
+    volatile int32_t* z = zjrk;  // an earlier launch of the chain wrote them
     for (int k = 0; k < nz; k++) {
-        jrs = min(jrs, zjrk[2 * k]);
-        krs = max(krs, zjrk[2 * k + 1]);
-        if (k > 0 && krs > zjrk[2 * k + 1]) zjrk[2 * k + 1] = krs;
+        jrs = min(jrs, z[2 * k]);
+        krs = max(krs, z[2 * k + 1]);
+        if (k > 0 && krs > z[2 * k + 1]) z[2 * k + 1] = krs;
     }
     jrk[0] = jrs;
     jrk[1] = krs;
     // p3fndf.f:66-80, p2fndf.f:41-55: from jrad(1) to krad(mz), the
     // outer edge moved out while it lies inside jrad(1)
-    int jrf = zjrk[0] < nr ? zjrk[0] : 1;
-    int kz = mz - 1, krf = zjrk[2 * kz + 1];
-    while (krf < jrf && kz + 1 < nz) krf = zjrk[2 * (++kz) + 1];
+    int jrf = z[0] < nr ? z[0] : 1;
+    int kz = mz - 1, krf = z[2 * kz + 1];
+    while (krf < jrf && kz + 1 < nz) krf = z[2 * (++kz) + 1];
     int32_t* frk = zjrk + 2 * GX_MAX_ZONES;
     frk[0] = krf < jrf ? 1 : jrf;
     frk[1] = krf < jrf ? nr : min(krf, nr);
@@ -342,21 +343,22 @@ __global__ void __launch_bounds__(256) k_zone_push(DevGeo g, ZoneTab zt, int mzo
                                                    ZoneAcc A) {
     __shared__ int sr[GX_MAX_ZONES][2];
     zone_rows_begin(sr);
+    gx_chain();
     constexpr int nd = ND, nw = 2 * ND;
     const int nz = zt.nz, off = nz + 1;
     for (int64_t i0 = blockIdx.x * (int64_t)blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = i0 + threadIdx.x;
-        const int z0 = i < n ? zone[i] : off + 1;
+        const int z0 = i < n ? __ldcg(zone + i) : off + 1;
         int dz = 0, ring = 0;
         if (z0 <= mzone || (z0 == off && mzone == nz)) {
             float q[6], qo[6];
 #pragma unroll
-            for (int k = 0; k < nw; k++) q[k] = qo[k] = P[k * cap + i];
+            for (int k = 0; k < nw; k++) q[k] = qo[k] = __ldcg(P + k * cap + i);
             float a[3] = {0.f, 0.f, 0.f}, ph;
             if (z0 != off) {
                 const float z = (ND == 3) ? q[2] : 0.f;
                 const CellW cw = gx_cell_t<true, ND>(g, q[0], q[1], z, true);
-                gx_accel_cell_t<Q, ND>(g, F, cw, q[0], q[1], z, a[0], a[1], a[2], ph);
+                gx_accel_cell_t<Q, ND, true>(g, F, cw, q[0], q[1], z, a[0], a[1], a[2], ph);
             }
             if (z0 > 1) {
                 const float t = zt_tsfac(zt, z0);
@@ -415,6 +417,7 @@ struct ZoneMix {
 // arrays, cleared; then zoncmb + scaled, and the ring ranges, as k_zone_combine
 __global__ void __launch_bounds__(256) k_zone_mix(int mesh, float* __restrict__ mass, ZoneAcc A, ZoneMix X, float pm, int nz, int nr, int mdep,
                            int mz, int quad, int32_t* __restrict__ zjrk, int32_t* __restrict__ jrk) {
+    gx_chain();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < mesh) {
         float v = 0.f;
@@ -422,26 +425,26 @@ __global__ void __launch_bounds__(256) k_zone_mix(int mesh, float* __restrict__ 
             float w = 0.f;
             if (k < mdep) {
                 unsigned long long* a = A.of(k + 1, mesh) + i;
-                const unsigned long long q = *a;
+                const unsigned long long q = __ldcg(a);
                 if (q) *a = 0ull;
                 w = (float)((double)(long long)q * (1.0 / 1048576.0)) * 1.f;
                 if (k > 0) X.znew[k][i] = w;
             } else if (X.un[k]) {
-                w = X.znew[k][i];
+                w = __ldcg(X.znew[k] + i);
             }
             if (k == 0) {
                 v = w;
                 continue;
             }
             if (X.un[k]) v = __fadd_rn(v, __fmul_rn(X.fn[k], w));
-            if (X.uo[k]) v = __fadd_rn(v, __fmul_rn(X.fo[k], X.zold[k][i]));
+            if (X.uo[k]) v = __fadd_rn(v, __fmul_rn(X.fo[k], __ldcg(X.zold[k] + i)));
         }
         mass[i] = v * pm;
     }
     if (i == 0) {
         for (int k = 0; k < mdep; k++) {
             // as the sort's row scan gives it: jrad, krad 1-based (empty: nr, 0)
-            const int lo = A.rng[2 * k], hi = A.rng[2 * k + 1];
+            const int lo = __ldcg(A.rng + 2 * k), hi = __ldcg(A.rng + 2 * k + 1);
             zjrk[2 * k] = hi >= 0 ? lo + (quad ? 0 : 1) : nr;
             zjrk[2 * k + 1] = hi >= 0 ? min(hi + 2, nr) : 0;
             A.rng[2 * k] = 0x7fffffff;
@@ -506,8 +509,8 @@ static void zone_direct_launch(GxCtx* c, int mzone) {
     const int64_t n = c->n;
     const unsigned nb = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8);
     if (mzone)
-        k_zone_push<ND, Q><<<nb, 256, 0, c->stream>>>(c->g, c->zt, mzone, c->pbuf[c->cur], c->cap, n, c->field,
-                                                      c->pzone[c->cur], zone_acc(c));
+        gx_launch_chain(k_zone_push<ND, Q>, nb, 256, 0, c->stream, c->g, c->zt, mzone, c->pbuf[c->cur], c->cap, n,
+                        c->field, c->pzone[c->cur], zone_acc(c));  // (its status: GX_LAUNCHED)
     else
         k_zone_dep<ND, Q><<<nb, 256, 0, c->stream>>>(c->g, c->nzones, c->pbuf[c->cur], c->cap, n, c->pzone[c->cur],
                                                      zone_acc(c));
@@ -549,8 +552,8 @@ static int zone_combine(GxCtx* c, int mdep) {
     const int mesh = c->g.mesh, mz = zone_mzone(c, c->istep);
     const unsigned nb = (unsigned)((mesh + 255) / 256);
     if (zone_direct(c))
-        k_zone_mix<<<nb, 256, 0, c->stream>>>(mesh, c->mass, zone_acc(c), mix, c->g.pmass, c->nzones, c->g.nr, mdep, mz,
-                                              c->g.quad, c->zjrk_d, c->jrk_d);
+        GX_CUDA(c, gx_launch_chain(k_zone_mix, nb, 256, 0, c->stream, mesh, c->mass, zone_acc(c), mix, c->g.pmass,
+                                   c->nzones, c->g.nr, mdep, mz, c->g.quad, c->zjrk_d, c->jrk_d));
     else
         k_zone_combine<<<nb, 256, 0, c->stream>>>(mesh, c->mass, src, c->g.pmass, c->nzones, c->g.nr, mz, c->zjrk_d,
                                                   c->jrk_d);
