@@ -54,6 +54,7 @@ __device__ __forceinline__ bool type_valid(const DevGeo& g, int t, int m, int k)
 template <int NJ, int NCW, int MINB>
 __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) {
     extern __shared__ __align__(128) unsigned char smraw[];
+    gx_chain();
     const DevGeo& g = A.g;
     const int nr = g.nr, nkz = g.nkz;
     const int R = A.rows_per_tile, NST = A.nst;
@@ -67,7 +68,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) 
     uint64_t* sempty = sfull + 2;      // [2] spectrum no longer read
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // with no mass on the grid (ks < js) no tile is copied and every output is 0
-    const int js = max(A.jrk[0], 1) - 1, ks = min(A.jrk[1], nr) - 1;
+    const int js = max(__ldcg(A.jrk), 1) - 1, ks = min(__ldcg(A.jrk + 1), nr) - 1;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NST; s++) {
@@ -268,7 +269,7 @@ int gx_conv_bulk(GxCtx* c, int nact, int tmask) {
     for (int i = 0; i < 260; i++) A.act_m[i] = (i < nact) ? c->spec.m[i] : 0;
     const int grid = std::min(A.nitems, dev_sms);
     GX_CUDA(c, cudaFuncSetAttribute(k_conv_bulk<1, ncw, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_conv_bulk<1, ncw, 1><<<grid, (ncw + 1) * 32, smem, c->stream>>>(A);
+    GX_CUDA(c, gx_launch_chain(k_conv_bulk<1, ncw, 1>, grid, (ncw + 1) * 32, smem, c->stream, A));
     GX_LAUNCHED(c);
     return GX_OK;
 }

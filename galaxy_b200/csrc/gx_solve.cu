@@ -194,15 +194,16 @@ __global__ void __launch_bounds__(288) k_fwd_az(DevGeo g, int ncp, const int32_t
                                                 const float* __restrict__ Taz,
                                                 float* __restrict__ C1) {
     extern __shared__ __align__(16) float sm[];
+    gx_chain();
     const int na = g.na, ngz = g.ngz, nr = g.nr;
     const int row0 = blockIdx.x * FWD_RB;
-    const int rlo = (max(jrk[0], 1) - 1) * ngz, rhi = min(jrk[1], nr) * ngz;  // active rows [rlo, rhi)
+    const int rlo = (max(__ldcg(jrk), 1) - 1) * ngz, rhi = min(__ldcg(jrk + 1), nr) * ngz;  // active rows [rlo, rhi)
     if (row0 + FWD_RB <= rlo || row0 >= rhi) return;
     const int nrows = min(FWD_RB, g.nrow - row0);
     if (zr) {
         // only blocks with a row in the planes the vertical part sums (the
         // planes holding mass, the first rounded down to a multiple of 4)
-        const int zs = zr[0] & ~3, ze = zr[1];
+        const int zs = __ldcg(zr) & ~3, ze = __ldcg(zr + 1);
         int in = 0;
         if ((int)threadIdx.x < nrows) {
             const int iz = (row0 + (int)threadIdx.x) % ngz;
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(288) k_fwd_az(DevGeo g, int ncp, const int32_t
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const int i = b + u * blockDim.x, r = i / na;
-            v[u] = (i < FWD_RB * na && r < nrows) ? __ldg(mass + (size_t)row0 * na + i) : 0.f;
+            v[u] = (i < FWD_RB * na && r < nrows) ? __ldcg(mass + (size_t)row0 * na + i) : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
@@ -280,16 +281,17 @@ __global__ void __launch_bounds__(288) k_fwd_z(DevGeo g, int nact, int ncp,
                                                const float* __restrict__ C1,
                                                const float* __restrict__ Tz, float4* __restrict__ S) {
     extern __shared__ __align__(16) float sm[];
+    gx_chain();
     const int ngz = g.ngz, nkz = g.nkz, nr = g.nr;
     // the planes summed: all, or those holding mass with the first rounded
     // down to a multiple of 4, so that every lane of the K split below sums
     // the same planes in the same order as over the whole grid (the others
     // add exact zeros): the spectrum is bitwise the whole-grid one
-    const int zs = zr ? (zr[0] & ~3) : 0;
-    const int nzs = zr ? max(zr[1] - zs + 1, 0) : ngz;
+    const int zs = zr ? (__ldcg(zr) & ~3) : 0;
+    const int nzs = zr ? max(__ldcg(zr + 1) - zs + 1, 0) : ngz;
     const int ir = blockIdx.x, kr0 = blockIdx.y * FWD_KR;   // first output row (2 kz0)
     const int nrow_out = min(FWD_KR, 2 * nkz - kr0);
-    if (ir < jrk[0] - 1 || ir > min(jrk[1], nr) - 1) {
+    if (ir < __ldcg(jrk) - 1 || ir > min(__ldcg(jrk + 1), nr) - 1) {
         // only the rings that hold mass are transformed (p3fndf.f:44-57); the
         // others get a zero spectrum so that the sum over ranks stays exact
         for (int i = threadIdx.x; i < nact * (nrow_out / 2); i += blockDim.x) {
@@ -310,7 +312,7 @@ __global__ void __launch_bounds__(288) k_fwd_z(DevGeo g, int nact, int ncp,
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const int i = b + u * blockDim.x;
-                if (i < n4) v[u] = __ldg(src + i);
+                if (i < n4) v[u] = __ldcg(src + i);
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -397,10 +399,11 @@ __global__ void __launch_bounds__(FWR_THREADS) k_fwd_ring(DevGeo g, int nact, in
                                                           int32_t* __restrict__ errword, GreenAhead ga) {
     extern __shared__ __align__(128) float sm[];
     __shared__ uint64_t bar;
+    gx_chain();
     const int na = g.na, ngz = g.ngz, nkz = g.nkz, nr = g.nr;
     const int ir = blockIdx.x;
     if (ir >= nr) {
-        const int js = max(jrk[0], 1) - 1, ks = min(jrk[1], nr) - 1;
+        const int js = max(__ldcg(jrk), 1) - 1, ks = min(__ldcg(jrk + 1), nr) - 1;
         if (ks < js) return;
         for (int i = (ir - nr) + ga.ctas * (int)threadIdx.x; i < ga.nitems * 4; i += ga.ctas * (int)blockDim.x) {
             const int it = i >> 2, t = i & 3, a = it / nkz, k = it - a * nkz, m = ga.act_m[a];
@@ -411,14 +414,14 @@ __global__ void __launch_bounds__(FWR_THREADS) k_fwd_ring(DevGeo g, int nact, in
         }
         return;
     }
-    if (ir < jrk[0] - 1 || ir > min(jrk[1], nr) - 1) {
+    if (ir < __ldcg(jrk) - 1 || ir > min(__ldcg(jrk + 1), nr) - 1) {
         // a ring without mass: zero spectrum (p3fndf.f:44-57)
         for (int i = threadIdx.x; i < nact * nkz; i += blockDim.x)
             S[(size_t)i * nr + ir] = make_float4(0.f, 0.f, 0.f, 0.f);
         return;
     }
-    const int zs = zr ? (zr[0] & ~3) : 0;
-    const int nzs = zr ? max(zr[1] - zs + 1, 0) : ngz;
+    const int zs = zr ? (__ldcg(zr) & ~3) : 0;
+    const int nzs = zr ? max(__ldcg(zr + 1) - zs + 1, 0) : ngz;
     const int ldx = na + 4, ldt = ru4(2 * nkz), tnN = ncpf >> 2;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tml = lane >> 3, tnl = lane & 7;
     float* C1 = sm;                            // [ru4(ngz)][ncpf]   harmonics m > 0 (or all)
@@ -845,21 +848,21 @@ int gx_mixed_findf(GxCtx* c, int lpot, bool polcat_only_field, const int32_t* fr
                 ga.ctas = g.nr < sms ? std::min(sms - g.nr, 32) : 0;
                 for (int a = 0; a < nact; a++) ga.act_m[a] = c->spec.m[a];
             }
-            k_fwd_ring<<<g.nr + ga.ctas, FWR_THREADS, smr, c->stream>>>(g, nact, ncpf, cb, c->jrk_d, zr, c->mass, Tf,
-                                                                        TzT, c->specS, c->errword, ga);
+            GX_CUDA(c, gx_launch_chain(k_fwd_ring, g.nr + ga.ctas, FWR_THREADS, smr, c->stream, g, nact, ncpf, cb,
+                                       c->jrk_d, zr, c->mass, Tf, TzT, c->specS, c->errword, ga));
             GX_LAUNCHED(c);
         } else {
             if (!c->fwdC1) GX_CUDA(c, cudaMalloc((void**)&c->fwdC1, sizeof(float) * (size_t)g.nrow * ncp));
             size_t sm = sizeof(float) * ((size_t)FWD_RB * (g.na + 1) + ntaz);
             GX_CUDA(c, cudaFuncSetAttribute(k_fwd_az, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-            k_fwd_az<<<(g.nrow + FWD_RB - 1) / FWD_RB, 288, sm, c->stream>>>(g, ncp, c->jrk_d, zr, c->mass,
-                                                                             c->fwdtab, c->fwdC1);
+            GX_CUDA(c, gx_launch_chain(k_fwd_az, (g.nrow + FWD_RB - 1) / FWD_RB, 288, sm, c->stream, g, ncp, c->jrk_d,
+                                       zr, c->mass, c->fwdtab, c->fwdC1));
             GX_LAUNCHED(c);
             sm = sizeof(float) * ((size_t)g.ngz * ncp + (size_t)FWD_KR * g.ngz);
             GX_CUDA(c, cudaFuncSetAttribute(k_fwd_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
             dim3 gz(g.nr, (2 * g.nkz + FWD_KR - 1) / FWD_KR);
-            k_fwd_z<<<gz, 288, sm, c->stream>>>(g, nact, ncp, c->jrk_d, zr, c->fwdC1, c->fwdtab + ntaz,
-                                                c->specS);
+            GX_CUDA(c, gx_launch_chain(k_fwd_z, gz, 288, sm, c->stream, g, nact, ncp, c->jrk_d, zr, c->fwdC1,
+                                       c->fwdtab + ntaz, c->specS));
             GX_LAUNCHED(c);
         }
     } else {

@@ -550,13 +550,14 @@ __global__ void __launch_bounds__(SZR_THREADS, 1) k_syn_ring(DevGeo g, int nact,
     extern __shared__ __align__(128) float sm[];
     __shared__ uint64_t bar;
     __shared__ int s_blk[SZR_MAXBLK], s_nblk;
+    gx_chain();
     const int ir = blockIdx.x;
-    if (frk && (ir + 1 < frk[0] || ir + 1 > frk[1])) return;  // rings no moving particle reads
+    if (frk && (ir + 1 < __ldcg(frk) || ir + 1 > __ldcg(frk + 1))) return;  // rings no moving particle reads
     const int nr = g.nr, nkz = g.nkz, ngz = g.ngz, Z0 = tb.Z0, nz4 = szr_stride(Z0);
     float4* OS = reinterpret_cast<float4*>(sm);            // [4][nkz][nact]
     float* TP = sm + (size_t)16 * nkz * nact;              // [nkz][nz4]
     float* TQ = TP + (size_t)nkz * nz4;
-    const int zlo = zr ? max(zr[0] - 1, 0) : 0, zhi = zr ? min(zr[1] + 1, ngz - 1) : ngz - 1;
+    const int zlo = zr ? max(__ldcg(zr) - 1, 0) : 0, zhi = zr ? min(__ldcg(zr + 1) + 1, ngz - 1) : ngz - 1;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         mbar_fence_init();
@@ -982,8 +983,8 @@ int gx_synthesis(GxCtx* c, int tmask, float* polar, const int32_t* frk, const in
             // vertical and azimuthal synthesis and polcat of one ring per CTA
             const int a0 = c->spec.m[0] == 0 ? 1 : 0;
             GX_CUDA(c, cudaFuncSetAttribute(k_syn_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
-            k_syn_ring<<<g.nr, SZR_THREADS, smr, c->stream>>>(g, nact, a0, ncp, tmask, c->specO, tb, c->synR,
-                                                               c->field, polar, frk, zr, c->errword);
+            GX_CUDA(c, gx_launch_chain(k_syn_ring, g.nr, SZR_THREADS, smr, c->stream, g, nact, a0, ncp, tmask, c->specO,
+                                       tb, c->synR, c->field, polar, frk, zr, c->errword));
             GX_LAUNCHED(c);
             return GX_OK;
         }
