@@ -54,7 +54,7 @@ __device__ __forceinline__ bool type_valid(const DevGeo& g, int t, int m, int k)
 template <int NJ, int NCW, int MINB>
 __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    gx_chain();
+    gx_chain_go();
     const DevGeo& g = A.g;
     const int nr = g.nr, nkz = g.nkz;
     const int R = A.rows_per_tile, NST = A.nst;
@@ -87,7 +87,15 @@ __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) 
         // ------------------------------------------------------------ producer
         if (lane != 0) return;
         int tile = 0, li = 0, s_issued = 0;
-        bool ok = true;
+        bool ok = true, ahead = true;
+        // the spectrum needs the forward transform, the Green table does not: the
+        // first stages fill while the transform's last CTAs run
+        auto spectrum = [&](int a, int k, int sb) {
+            mbar_expect_tx(&sfull[sb], (uint32_t)(nr * sizeof(float4)));
+            bulk_g2s(Sbuf + sb * nr, A.S + ((size_t)a * nkz + k) * nr, (uint32_t)(nr * sizeof(float4)),
+                     &sfull[sb]);
+            s_issued++;
+        };
         for (int it = blockIdx.x; ok && it < A.nitems; it += gridDim.x, li++) {
             const int a = it / A.nkr, k = A.krank + A.ksplit * (it - a * A.nkr), m = A.act_m[a];
             // the item's spectrum into its half of the double buffer
@@ -96,16 +104,18 @@ __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) 
                 ok = false;
                 break;
             }
-            mbar_expect_tx(&sfull[sb], (uint32_t)(nr * sizeof(float4)));
-            bulk_g2s(Sbuf + sb * nr, A.S + ((size_t)a * nkz + k) * nr, (uint32_t)(nr * sizeof(float4)),
-                     &sfull[sb]);
-            s_issued++;
+            if (!ahead) spectrum(a, k, sb);
             for (int t = 0; ok && t < 4; t++) {
                 if (!((A.tmask >> t) & 1) || !type_valid(g, t, m, k)) continue;
                 const float* Gt = A.G + ((((size_t)t * g.ng + m) * nkz + k) * nr) * (size_t)nr;
                 for (int r0 = js; r0 <= ks; r0 += R) {
                     const int rows = min(R, ks - r0 + 1);
                     const int s = tile % NST;
+                    if (ahead && tile == NST) {
+                        gx_chain_wait();
+                        spectrum(a, k, sb);
+                        ahead = false;
+                    }
                     if (tile >= NST && !mbar_wait(&empty[s], ((tile / NST) - 1) & 1)) {
                         ok = false;
                         break;
@@ -116,7 +126,13 @@ __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) 
                     tile++;
                 }
             }
+            if (ahead) {
+                gx_chain_wait();
+                spectrum(a, k, sb);
+                ahead = false;
+            }
         }
+        if (ahead) gx_chain_wait();
         if (!ok) {
             atomicExch(A.errword, 3);
             // drain the copies that may still be in flight (the latest phase of each buffer)
@@ -127,6 +143,7 @@ __global__ void __launch_bounds__((NCW + 1) * 32, MINB) k_conv_bulk(ConvArgs A) 
     }
 
     // ---------------------------------------------------------------- consumers
+    gx_chain_wait();
     int tile = 0, li = 0;
     bool dead = false;
     for (int it = blockIdx.x; it < A.nitems; it += gridDim.x, li++) {

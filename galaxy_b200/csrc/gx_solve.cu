@@ -194,7 +194,8 @@ __global__ void __launch_bounds__(288) k_fwd_az(DevGeo g, int ncp, const int32_t
                                                 const float* __restrict__ Taz,
                                                 float* __restrict__ C1) {
     extern __shared__ __align__(16) float sm[];
-    gx_chain();
+    gx_chain_wait();
+    gx_chain_go();  // the contraction reads the ring range ahead of its own wait
     const int na = g.na, ngz = g.ngz, nr = g.nr;
     const int row0 = blockIdx.x * FWD_RB;
     const int rlo = (max(__ldcg(jrk), 1) - 1) * ngz, rhi = min(__ldcg(jrk + 1), nr) * ngz;  // active rows [rlo, rhi)
@@ -281,7 +282,8 @@ __global__ void __launch_bounds__(288) k_fwd_z(DevGeo g, int nact, int ncp,
                                                const float* __restrict__ C1,
                                                const float* __restrict__ Tz, float4* __restrict__ S) {
     extern __shared__ __align__(16) float sm[];
-    gx_chain();
+    gx_chain_wait();
+    gx_chain_go();  // the contraction reads the ring range ahead of its own wait
     const int ngz = g.ngz, nkz = g.nkz, nr = g.nr;
     // the planes summed: all, or those holding mass with the first rounded
     // down to a multiple of 4, so that every lane of the K split below sums
@@ -399,7 +401,8 @@ __global__ void __launch_bounds__(FWR_THREADS) k_fwd_ring(DevGeo g, int nact, in
                                                           int32_t* __restrict__ errword, GreenAhead ga) {
     extern __shared__ __align__(128) float sm[];
     __shared__ uint64_t bar;
-    gx_chain();
+    gx_chain_wait();
+    gx_chain_go();  // the contraction reads the ring range ahead of its own wait
     const int na = g.na, ngz = g.ngz, nkz = g.nkz, nr = g.nr;
     const int ir = blockIdx.x;
     if (ir >= nr) {

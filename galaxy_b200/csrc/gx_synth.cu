@@ -550,27 +550,32 @@ __global__ void __launch_bounds__(SZR_THREADS, 1) k_syn_ring(DevGeo g, int nact,
     extern __shared__ __align__(128) float sm[];
     __shared__ uint64_t bar;
     __shared__ int s_blk[SZR_MAXBLK], s_nblk;
-    gx_chain();
+    gx_chain_go();
     const int ir = blockIdx.x;
+    if (frk) gx_chain_wait();
     if (frk && (ir + 1 < __ldcg(frk) || ir + 1 > __ldcg(frk + 1))) return;  // rings no moving particle reads
     const int nr = g.nr, nkz = g.nkz, ngz = g.ngz, Z0 = tb.Z0, nz4 = szr_stride(Z0);
     float4* OS = reinterpret_cast<float4*>(sm);            // [4][nkz][nact]
     float* TP = sm + (size_t)16 * nkz * nact;              // [nkz][nz4]
     float* TQ = TP + (size_t)nkz * nz4;
     const int zlo = zr ? max(__ldcg(zr) - 1, 0) : 0, zhi = zr ? min(__ldcg(zr + 1) + 1, ngz - 1) : ngz - 1;
+    const uint32_t ob = (uint32_t)(nkz * nact) * 16u;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
         mbar_fence_init();
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const uint32_t ob = (uint32_t)(nkz * nact) * 16u, tb4 = (uint32_t)(nkz * nz4) * 4u;
+        const uint32_t tb4 = (uint32_t)(nkz * nz4) * 4u;
         uint32_t tot = 2 * tb4;
         for (int t = 0; t < 4; t++)
             if ((tmask >> t) & 1) tot += ob;
         mbar_expect_tx(&bar, tot);
         bulk_g2s(TP, tb.TP, tb4, &bar);
         bulk_g2s(TQ, tb.TQ, tb4, &bar);
+    }
+    gx_chain_wait();  // the tables above need nothing of the contraction's
+    if (threadIdx.x == 0) {
         for (int t = 0; t < 4; t++)
             if ((tmask >> t) & 1)
                 bulk_g2s(OS + (size_t)t * nkz * nact, O + ((size_t)t * nr + ir) * nkz * nact, ob, &bar);
@@ -955,7 +960,8 @@ int gx_synthesis(GxCtx* c, int tmask, float* polar, const int32_t* frk, const in
     const int nz4 = ru4s(Z0);
     const size_t nWe = (size_t)nz4 * KE, nWo = (size_t)nz4 * KO, nT = (size_t)nact * njp;
     const size_t nTk = g.ndim == 3 ? (size_t)szr_stride(Z0) * g.nkz : 0;  // TP, TQ
-    if (!c->syntab) {
+    const bool fresh = !c->syntab;
+    if (fresh) {
         if (nact > 64) return c->err = "more than 64 active harmonics", GX_ERR_RANGE;
         const size_t tot = 2 * nWe + 2 * nWo + 2 * nT + 2 * (size_t)njp + 2 * nTk;
         GX_CUDA(c, cudaMalloc((void**)&c->syntab, sizeof(float) * tot));
@@ -983,8 +989,14 @@ int gx_synthesis(GxCtx* c, int tmask, float* polar, const int32_t* frk, const in
             // vertical and azimuthal synthesis and polcat of one ring per CTA
             const int a0 = c->spec.m[0] == 0 ? 1 : 0;
             GX_CUDA(c, cudaFuncSetAttribute(k_syn_ring, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr));
-            GX_CUDA(c, gx_launch_chain(k_syn_ring, g.nr, SZR_THREADS, smr, c->stream, g, nact, a0, ncp, tmask, c->specO,
-                                       tb, c->synR, c->field, polar, frk, zr, c->errword));
+            // tables built just now are complete only after a plain launch's start
+            // (the kernel reads them ahead of its wait)
+            if (fresh)
+                k_syn_ring<<<g.nr, SZR_THREADS, smr, c->stream>>>(g, nact, a0, ncp, tmask, c->specO, tb, c->synR,
+                                                                   c->field, polar, frk, zr, c->errword);
+            else
+                GX_CUDA(c, gx_launch_chain(k_syn_ring, g.nr, SZR_THREADS, smr, c->stream, g, nact, a0, ncp, tmask,
+                                           c->specO, tb, c->synR, c->field, polar, frk, zr, c->errword));
             GX_LAUNCHED(c);
             return GX_OK;
         }
