@@ -181,8 +181,8 @@ def step_bytes(cfg, geo, n):
     return n * 2 * 2 * cfg.ndim * 4 + npairs * geo.nr * geo.nr * 4 + geo.mesh * 4 * (2 + 2 * nf)
 
 
-KERNEL_OF = {"push": "k_push_bkt", "conv": "k_conv_bulk", "syn": "k_synz_tc+k_synaz",
-             "fwd": "k_fwd_az+k_fwd_z", "sort": "k_bk_plan", "combine": "k_mass_convert"}
+KERNEL_OF = {"push": "k_push_bkt", "conv": "k_conv_bulk", "syn": "k_syn_ring",
+             "fwd": "k_fwd_ring", "sort": "k_bk_plan", "combine": "k_mass_convert"}
 
 
 def ncu_traffic(workload):
@@ -454,7 +454,7 @@ def run_ensemble(ndisc=64, steps=1000, loop_steps=20, seed=12345):
     """Batched ensemble: ndisc seeded Kuzmin-Toomre discs (seeds 0..ndisc-1),
     particle counts log-uniform in [2e4, 2e6], each on its own 64 x 128 2D
     grid (log rings 0.05..5, m = 0..8, Plummer 0.1), dt = 0.025; one
-    persistent launch per step under a CUDA graph after the autotuner.
+    persistent launch per 64 steps after the autotuner.
     Against the plain per-run loop (one single-disc context per disc, the
     same arithmetic), timed over loop_steps steps per disc."""
     from galaxy_b200 import Galaxy, make_config, GX_RMAP_LOG

@@ -16,7 +16,7 @@
 // and K the linear map mass -> (fx, fy): forward DFT of the active
 // harmonics (p2manl.f:32-45), radial contraction (p2conv.f:114-181),
 // synthesis (p2fsyn.f:34-56), polcat (polcat.f:22-41); K^T runs those
-// steps transposed in reverse order (k_adjt_syn, k_adjt_conv, k_adjt_fwd).
+// steps transposed in reverse order (k_adjt_syn, k_adjt_conv).
 // dJ/d(halo_rc, halo_v2) accumulate the halo's parameter derivatives . mu
 // per block in FP64.
 #include <algorithm>

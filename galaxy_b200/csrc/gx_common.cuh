@@ -703,12 +703,12 @@ __device__ __forceinline__ void gx_accel_cell(const DevGeo& g, const float4* __r
 // gain from that cache) with ordinary loads, never through the read-only path.
 // Zoned step of 15000 particles, five launches: 26.6 -> 20.5 us; adjoint of 400k
 // particles on 128 x 256, 13 launches a step: 126.5 -> 117.4 us; 3D step of 200k particles on
-// an odd grid, solve kernels only: 86.4 -> 85.2 us.  What a kernel may read ahead of
+// an odd grid, solve kernels only: 86.4 -> 85.7 us.  What a kernel may read ahead of
 // its wait is complete because a forward transform waits before it lets the
 // contraction start: constant tables, and the mass's ring and plane ranges (the
 // contraction's first Green tiles and the ring synthesis' tables so: 85.2 -> 84.5
 // us).  The mass conversion is not chained: CTAs of the transform that wait beside
-// it cost the plan on the side stream its place (84.5 -> 89 us).
+// it cost the plan on the side stream its place (85.6 -> 89.9 us).
 __device__ __forceinline__ void gx_chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void gx_chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void gx_chain() {

@@ -401,7 +401,8 @@ int gx_sfp_last_ms(const GxSfp* sfp, float* ms, int64_t* launches);
  * (gx_sfp_sum's arithmetic at `precision`, scaled by pmass), then
  * v += a(x) dt, x += v dt (stpgrp.f:26-32 with the time step explicit:
  * positions, velocities and dt in the caller's units, G = 1).  The
- * particles stay on the device; coeff_out (may be NULL) receives the
+ * particles, the sums and the force tables stay on the device: a call of
+ * nsteps synchronises once; coeff_out (may be NULL) receives the
  * coefficients of the final positions. */
 int gx_sfp_step(GxSfp* sfp, int nsteps, double dt, int precision, double pmass, double* coeff_out);
 
@@ -427,9 +428,9 @@ int gx_adjoint(GxCtx* ctx, int nsteps, int ckpt_every, double* J, float* grad, d
                float* drift);
 
 /* Ensemble of independent 2D discs sharing one grid geometry (one Green
- * table), advanced together: every step is one persistent cooperative
- * launch for all discs (field solve per disc, then push + deposit of every
- * particle), and batches of 16 step launches are replayed from a CUDA graph.
+ * table), advanced together by persistent cooperative launches of up to 64
+ * steps for all discs (per step the field solve of each disc, then push +
+ * deposit of its particles).
  * Each disc follows the single-disc run of SRC/progs/galaxy.f:107-148
  * (findf, getacc + stpgrp, massgn: the same cell keys, weights and integer
  * deposit; FP32 transforms summed in a different order, so fields agree to
@@ -453,9 +454,8 @@ const char* gx_ensemble_last_error(const GxEnsemble* ens);
  * keeps the fastest; returns the choice. */
 int gx_ensemble_tune(GxEnsemble* ens, int* threads, int* chunk);
 
-/* Current launch shape: threads per CTA, particles per chunk, CTAs, and
- * whether the steps are replayed from a CUDA graph (1) or launched one by
- * one (0). */
+/* Current launch shape: threads per CTA, particles per chunk, CTAs; graph
+ * is 0 (the steps of a launch run inside it, no CUDA graph replays them). */
 int gx_ensemble_config(const GxEnsemble* ens, int* threads, int* chunk, int* grid, int* graph);
 
 /* Advance every disc nsteps leapfrog steps. */
