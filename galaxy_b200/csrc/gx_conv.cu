@@ -14,7 +14,8 @@
 // contiguous block of rows, into a ring of NST shared-memory stages with
 // cp.async.bulk; an mbarrier per stage counts the bytes in (full) and the
 // consumer warps out (empty).  The item's spectrum (nr float4) comes the same
-// way into a double buffer.  Every wait is bounded: on time-out the CTA
+// way into a double buffer.  The first stages are copied before the forward
+// transform has ended (only the spectrum needs it).  Every wait is bounded: on time-out the CTA
 // raises the device error word, drains its own copies in flight (bounded)
 // and returns; a consumer warp that timed out keeps taking the named
 // barriers so that its partners are not left waiting.
