@@ -481,8 +481,8 @@ static int adj_solve(GxCtx* c) {
     return gx_mixed_findf(c, 0, true);
 }
 
-extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, float* grad,
-                          double* dtheta, float* drift_out) {
+static int adj_run(GxCtx* c, int nsteps, int ckpt_every, double* J_out, float* grad, double* dtheta,
+                   float* drift_out) {
     if (!c || nsteps < 0 || ckpt_every < 1 || !J_out || !grad || !dtheta) return GX_ERR_ARG;
     if (c->fp64 || c->g.ndim != 2 || c->g.nsect != 1)
         return c->err = "the adjoint runs 2D one-sector grids on the mixed path", GX_ERR_ARG;
@@ -492,6 +492,7 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     if (c->spec.nact > 64) return c->err = "more than 64 active harmonics", GX_ERR_RANGE;
     const int64_t n = c->n;
     if (n < 1) return c->err = "no particles loaded", GX_ERR_STATE;
+    if (nsteps > 0 && c->spec.nact == 0) return c->err = "no active harmonics", GX_ERR_ARG;  // (as the solve)
     cudaSetDevice(c->dev);
     {
         const int rc = gx_dense(c);
@@ -552,12 +553,15 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     GX_CUDA(c, cudaMemcpyAsync(b.ck, b.S, sbytes, cudaMemcpyDeviceToDevice, st));
     // forward sweep with checkpoints
     if (nsteps > 0) {
+        c->have_mass = c->have_field = false;  // the sweeps' from here to the end of the call
+        c->acc_open = true;
         k_adj_mass<<<np, ADJ_BS, 0, st>>>(g, b.S, n, c->macc, gx_mass_ranges(c));
         GX_LAUNCHED(c);
     }
     for (int s = 0; s < nsteps; s++) {
         int rc = adj_solve(c);
         if (rc) return rc;
+        c->acc_open = true;
         GX_CUDA(c, gx_launch_chain(k_adj_fwd, np, ADJ_BS, 0, st, g, b.S, n, c->field, c->macc, gx_mass_ranges(c)));
         GX_LAUNCHED(c);
         if ((s + 1) % ckpt_every == 0)
@@ -591,6 +595,7 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     for (int s = nsteps - 1; s >= 0; s--) {
         const bool ck = (s % ckpt_every) == 0;
         // the psi term of step s + 1, the drift back to x_s and its deposit
+        c->acc_open = true;
         GX_CUDA(c, gx_launch_chain(k_adj_b, np, ADJ_BS, 0, st, g, b.S, b.L, n, s == nsteps - 1 ? nullptr : b.psi, g.pmass,
                                    1, ck ? b.ck + (size_t)(s / ckpt_every) * n : nullptr, b.drift, c->macc,
                                    gx_mass_ranges(c)));
@@ -648,4 +653,11 @@ extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, f
     GX_CUDA(c, cudaMemcpy(&ew, c->errword, sizeof ew, cudaMemcpyDeviceToHost));
     if (ew) return c->err = "device check raised the error word", GX_ERR_DEVICE;
     return GX_OK;
+}
+
+extern "C" int gx_adjoint(GxCtx* c, int nsteps, int ckpt_every, double* J_out, float* grad,
+                          double* dtheta, float* drift_out) {
+    const int rc = adj_run(c, nsteps, ckpt_every, J_out, grad, dtheta, drift_out);
+    if (c && rc) gx_mass_discard(c);
+    return rc;
 }

@@ -556,7 +556,7 @@ int gx_masset(GxCtx* c) {
     cudaSetDevice(c->dev);
     if (gx_fast_ok(c)) {
         int rc = gx_fast_masset(c);
-        if (rc) return rc;
+        if (rc) return gx_mass_discard(c), rc;
         GX_CUDA(c, cudaStreamSynchronize(c->stream));
         c->have_mass = true;
         c->have_field = false;
@@ -566,7 +566,7 @@ int gx_masset(GxCtx* c) {
     if (rc) return rc;
     c->zr_valid = false;
     rc = c->fp64 ? gx_fp64_masset(c) : (c->nzones > 1 ? gx_zone_masset(c) : gx_mixed_masset(c));
-    if (rc) return rc;
+    if (rc) return gx_mass_discard(c), rc;
     GX_CUDA(c, cudaStreamSynchronize(c->stream));
     c->have_mass = true;
     c->have_field = false;
@@ -621,7 +621,7 @@ int gx_step(GxCtx* c, int nsteps, int phys) {
         c->zr_valid = false;
         rc = (c->nzones > 1) ? gx_zone_step(c, nsteps, phys) : gx_mixed_step(c, nsteps, phys);
     }
-    if (rc) return rc;
+    if (rc) return gx_mass_discard(c), rc;
     GX_CUDA(c, cudaEventRecord(c->ev1, c->stream));
     GX_CUDA(c, cudaEventSynchronize(c->ev1));
     GX_CUDA(c, cudaEventElapsedTime(&c->last_ms, c->ev0, c->ev1));

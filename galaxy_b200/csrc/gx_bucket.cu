@@ -1123,6 +1123,7 @@ static int bk_launch_push(GxCtx* c, int cur, int nxt) {
         GX_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
         c->bk_grid = std::max(1, per) * sms;
     }
+    c->acc_open = true;
     kp<<<c->bk_grid, BK_THREADS, sm, c->stream>>>(g, c->bq[cur], c->bq[nxt], c->bcap, c->field, c->bk_items,
                                                   c->bk_ctl + 8, c->bk_cap[nxt], c->bk_base[nxt],
                                                   c->bk_fill[nxt], c->bk_ctl + 4 * nxt, c->bk_main, c->macc,
@@ -1140,7 +1141,32 @@ int gx_mass_convert(GxCtx* c) {
         c->zr_d + 2 * p, c->zr_d + 2 * q, g.ngz, g.quad, g.ndim == 3 && c->zr_valid);
     GX_LAUNCHED(c);
     c->mpar = q;
+    c->acc_open = c->acc_pending = false;
     return GX_OK;
+}
+
+// A call that fails between a deposit pass and the conversion of what it
+// deposited leaves both accumulators and their ranges as a new context has
+// them, so that the next masset adds to nothing; the mass array no longer
+// belongs to the particles.  (A call refused before its deposit keeps its mass.)
+void gx_mass_discard(GxCtx* c) {
+    if (!c->acc_open) return;
+    int32_t none[2 * GX_MAX_ZONES];
+    for (int i = 0; i < 2 * GX_MAX_ZONES; i += 2) {
+        none[i] = 0x7fffffff;
+        none[i + 1] = -1;
+    }
+    static_assert(2 * GX_MAX_ZONES >= 8, "both sets of ranges");
+    // (no status: where these fail, so do the calls that follow)
+    cudaMemsetAsync(c->macc, 0, sizeof(unsigned long long) * c->g.mesh, c->stream);
+    cudaMemcpyAsync(c->bk_ctl + 16, none, 8 * sizeof(int32_t), cudaMemcpyHostToDevice, c->stream);
+    if (c->zacc && c->nzones > 1) {
+        cudaMemsetAsync(c->zacc, 0, sizeof(unsigned long long) * (c->nzones - 1) * c->g.mesh, c->stream);
+        cudaMemcpyAsync(c->zjrk_d + 2 * GX_MAX_ZONES + 2, none, sizeof none, cudaMemcpyHostToDevice, c->stream);
+    }
+    cudaStreamSynchronize(c->stream);
+    c->acc_open = c->acc_pending = false;
+    c->have_mass = c->zones_ready = c->zr_valid = false;
 }
 
 // 2D: the forward transform converts its ring itself (gx_mixed_findf, which
@@ -1259,7 +1285,7 @@ static cudaGraphExec_t fast_capture(GxCtx* c, int64_t* per) {
     *per = c->launches - l0;
     c->bcur = b;
     c->mpar = mp;
-    c->acc_pending = true;  // as it was: the caller captures after a deferred step
+    c->acc_pending = c->acc_open = true;  // as it was: the caller captures after a deferred step
     c->bk_pending = false;
     c->launches = l0;
     c->err.clear();

@@ -187,6 +187,7 @@ struct GxCtx {
     int32_t* bk_cnt = nullptr;               // [nrow + 1] row counts of the dense store (bucketing)
     unsigned long long* macc = nullptr;      // [mesh] fixed-point mass (2^-20 of a particle), zero between steps
     bool acc_pending = false;                // the mass is still in macc: the next 2D solve converts it
+    bool acc_open = false;                   // macc or zacc hold a deposit that no conversion has taken
     int32_t* zr_d = nullptr;                 // [2][2] first, last plane holding the fused pass's mass
                                              // (ngz, -1 when empty), at 2 p of the conversion of set p
     bool zr_valid = false;                   // the mass array is the fused pass's (zr_d describes it)
@@ -773,6 +774,7 @@ int gx_fast_masset(GxCtx* c);  // masset by the deposit-only fused pass
 static inline int32_t* gx_mass_ranges(const GxCtx* c) { return c->bk_ctl + 16 + 4 * c->mpar; }  // of the next deposit
 int gx_mass_defer(GxCtx* c);    // leave that to the next solve where it can (2D), else do it
 int gx_mass_convert(GxCtx* c);  // mass accumulator -> mass array (accumulator cleared)
+void gx_mass_discard(GxCtx* c);  // after a failed call: a deposit that was not converted is dropped
 int gx_bucket_alloc(GxCtx* c);
 int gx_bucket_words(const GxCtx* c);  // float4 words per record of the bucketed store
 int gx_synthesis(GxCtx* c, int tmask, float* polar, const int32_t* frk = nullptr,

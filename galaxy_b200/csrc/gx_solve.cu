@@ -881,7 +881,7 @@ int gx_mixed_findf(GxCtx* c, int lpot, bool polcat_only_field, const int32_t* fr
         GX_CUDA(c, gx_launch_chain(kf, g.nr, F2_THREADS, sm, c->stream, g, nact, ncp, c->mass, c->fwdtab, c->specS,
                                    c->macc, gx_mass_ranges(c), c->bk_ctl + 16 + 4 * (c->mpar ^ 1), c->jrk_d));
         if (c->acc_pending) {
-            c->acc_pending = false;
+            c->acc_pending = c->acc_open = false;
             c->mpar ^= 1;
         }
         GX_LAUNCHED(c);

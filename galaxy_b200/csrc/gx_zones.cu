@@ -517,6 +517,7 @@ static void zone_direct_launch(GxCtx* c, int mzone) {
 }
 static int zone_direct_pass(GxCtx* c, int mzone) {
     if (c->n == 0) return GX_OK;
+    c->acc_open = true;
     if (c->g.quad) zone_direct_launch<3, true>(c, mzone);
     else if (c->g.ndim == 3) zone_direct_launch<3, false>(c, mzone);
     else zone_direct_launch<2, false>(c, mzone);
@@ -551,12 +552,14 @@ static int zone_combine(GxCtx* c, int mdep) {
     }
     const int mesh = c->g.mesh, mz = zone_mzone(c, c->istep);
     const unsigned nb = (unsigned)((mesh + 255) / 256);
-    if (zone_direct(c))
+    if (zone_direct(c)) {
         GX_CUDA(c, gx_launch_chain(k_zone_mix, nb, 256, 0, c->stream, mesh, c->mass, zone_acc(c), mix, c->g.pmass,
                                    c->nzones, c->g.nr, mdep, mz, c->g.quad, c->zjrk_d, c->jrk_d));
-    else
+        c->acc_open = false;
+    } else {
         k_zone_combine<<<nb, 256, 0, c->stream>>>(mesh, c->mass, src, c->g.pmass, c->nzones, c->g.nr, mz, c->zjrk_d,
                                                   c->jrk_d);
+    }
     GX_LAUNCHED(c);
     return GX_OK;
 }

@@ -1,0 +1,63 @@
+"""Calls that fail after a deposit pass: what the next calls see.  A call that
+returns an error leaves no deposited weights behind, so the next gx_masset
+gives the particles' mass and nothing on top of it."""
+import numpy as np
+import pytest
+
+from galaxy_b200 import Galaxy, GxError, make_config, GX_FLAG_SORTED_DEPOSIT, GX_GRID_MASS, GX_RMAP_STDPOL
+from galaxy_b200.disk import kt_disk
+
+pytestmark = pytest.mark.gpu
+
+
+def cfg2(flags=0, **kw):
+    return make_config(2, 40, 64, nsect=1, rmap=GX_RMAP_STDPOL, softl=1.0, tsoft=2, flags=flags, **kw)
+
+
+def test_refused_adjoint_leaves_the_mass_as_it_was():
+    """Every harmonic skipped: the adjoint has no solve to differentiate and
+    refuses.  The mass array is the particles' before and after, and masset
+    gives it again, bit for bit."""
+    rec, pm = kt_disk(5000, seed=2, rmax=4.9, ndim=2, dt=0.05, lscale=10.0)
+    with Galaxy(cfg2(ng=3, skip=(0, 1, 2), pmass=pm)) as gal:
+        gal.greenm()
+        gal.loadup(rec)
+        gal.masset()
+        mass = gal.grid(GX_GRID_MASS)
+        assert mass.sum() > 0
+        for _ in range(2):
+            with pytest.raises(GxError):
+                gal.adjoint(3, 2)
+            assert np.array_equal(gal.grid(GX_GRID_MASS), mass)
+        with pytest.raises(GxError):
+            gal.step(2)
+        assert np.array_equal(gal.unload(), rec)
+        gal.masset()
+        assert np.array_equal(gal.grid(GX_GRID_MASS), mass)
+        # without a step there is nothing to solve
+        J, grad, _, _ = gal.adjoint(0, 1)
+        assert J > 0 and np.isfinite(grad).all()
+
+
+@pytest.mark.parametrize("flags", [0, GX_FLAG_SORTED_DEPOSIT])
+def test_zoned_run_that_fails_leaves_no_deposit_behind(flags):
+    """Step factors that are not multiples of one another (1, 4, 6): the
+    seventh step finds a zone's older mass array at a useless time and the call
+    fails after its particle pass.  The run loaded again starts as a fresh one."""
+    rec, pm = kt_disk(20000, seed=5, rmax=4.9, ndim=2, dt=0.05, lscale=10.0)
+    with Galaxy(cfg2(flags, ng=9, pmass=pm)) as gal:
+        gal.greenm()
+        gal.set_zones([1, 4, 6], [0.0, 3.0, 12.0])
+        gal.loadup(rec)
+        gal.masset()
+        mass = gal.grid(GX_GRID_MASS)
+        gal.step(3)
+        ref = gal.unload(), gal.grid(GX_GRID_MASS)
+        with pytest.raises(GxError):
+            gal.step(4)
+        gal.loadup(rec)
+        gal.masset()
+        assert np.array_equal(gal.grid(GX_GRID_MASS), mass)
+        gal.step(3)
+        assert np.array_equal(gal.unload(), ref[0])
+        assert np.array_equal(gal.grid(GX_GRID_MASS), ref[1])
