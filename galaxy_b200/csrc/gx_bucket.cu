@@ -470,9 +470,12 @@ __global__ void __launch_bounds__(BK_THREADS, Q ? 4 : BK_MINB) k_push_bkt(
                     rmax_l = max(rmax_l, cn.ju);
                     if (Q) {
                         // nodes in the planes below and above; below plane 0 lies
-                        // the last plane of the ring below (flat offsets)
+                        // the last plane of the ring below (flat offsets), where
+                        // the next pass also reads for a cell just above plane
+                        // 0's, whose interpolation cell may come out as plane 0
                         zmin_l = min(zmin_l, max(cn.iz - 1, 0));
-                        zmax_l = max(zmax_l, cn.iz == 0 ? ngz - 1 : cn.iz);
+                        const bool low = cn.iz == 0 || (cn.iz == 1 && cn.dz < g.eps_z);
+                        zmax_l = max(zmax_l, low ? ngz - 1 : cn.iz);
                     } else if (d3) {
                         // a cell in the top plane (a spoke coordinate that
                         // rounded up to na moved it there) has its upper

@@ -138,3 +138,46 @@ def test_fused_2d_graph_replay_is_bitwise_the_sorted_deposit():
             out.append((gal.unload(), gal.grid(GX_GRID_MASS)))
     for x, y in zip(out[0], out[1]):
         assert (x.view(np.uint32) == y.view(np.uint32)).all()
+
+
+def lowest_boundary(ngz):
+    """dzg and z of a point on the boundary between planes 0 and 1 of the
+    quadratic scheme whose plane is 1 by the reference's operations (the
+    deposit) and 0 by the multiplication with 1 / dzg (the interpolation)"""
+    f = np.float32
+    for dzg in np.linspace(0.1, 0.12, 4001).astype(f):
+        zm = f(0.5) * dzg * f(ngz - 1)
+        z0 = f(0.5) * dzg - zm
+        for z in (z0, np.nextafter(z0, f(-9)), np.nextafter(z0, f(9))):
+            s = z + zm
+            if s * (f(1) / dzg) + f(0.5) < 1 <= s / dzg + f(0.5):
+                return float(dzg), z
+    raise AssertionError("no such boundary")
+
+
+def test_fused_quadratic_field_below_the_deposit_planes():
+    """Particles that interpolate one plane below their deposit plane, at the
+    bottom of the grid: their lowest node lies in the last plane of the ring
+    below (flat offsets), which the solve has to cover although no mass is near
+    it.  The field there is made non-finite beforehand, so that a plane the
+    solve leaves out shows in the particles."""
+    ngz = 15
+    dzg, z = lowest_boundary(ngz)
+    cfg = cfg3(ngz=ngz, dzg=dzg)
+    rec, pm = kt_disk(20_000, seed=8, rmax=4.5, ndim=3, z0=0.05, dt=0.025)
+    rec = rec[np.abs(rec[:, 2]) < 2 * dzg].copy()  # the planes next to the middle
+    rec[:200, 2] = z
+    cfg.pmass = pm
+    out = []
+    for flags in (0, GX_FLAG_SORTED_DEPOSIT):
+        cfg.flags = GX_FLAG_QUADRATIC | flags
+        with Galaxy(cfg) as gal:
+            gal.greenm()
+            gal.set_mass(np.full(gal.mesh, 1e38, np.float32))
+            gal.findf(True)
+            gal.loadup(rec)
+            gal.masset()
+            gal.step(1)
+            out.append(gal.unload())
+    assert np.isfinite(out[0]).all()
+    assert np.array_equal(out[0].view(np.uint32), out[1].view(np.uint32))
