@@ -456,7 +456,7 @@ static int alloc_particles(GxCtx* c, int64_t n) {
     // particles, and the overflow area's.  bk_item: at most BK_ITEM, at
     // least a quarter of a deposit window of particles (the bins each item
     // flushes; half of it in 2D), and otherwise small enough that a B200's
-    // resident CTAs (148 SMs x 5) get a few items each: 2 in 3D, where an item
+    // resident CTAs (148 SMs x 5 at most) get a few items each: 2 in 3D, where an item
     // more costs a window's flush (10M particles: 262 us a pass in items of
     // 4095, 292 in items of 1024; 1M: 73 us in items of 2048, 67 in items of
     // 1024), 4 in 2D (3M: 76 and 73 us)
@@ -488,6 +488,7 @@ int gx_loadup(GxCtx* c, const float* coords, int64_t n) {
     c->have_mass = c->have_field = c->have_keys = false;
     c->bucketed = false;
     c->zr_valid = false;
+    c->bk_grid = 0;
     const int nw = 2 * c->g.ndim;
     if (n == 0) return (c->nzones > 1 && !c->fp64) ? gx_zone_loadup(c) : GX_OK;
     float* staging = c->stagebuf;

@@ -45,6 +45,8 @@
 // icheck, the adjoint); unload writes the records straight from the store
 // in load order, and masset deposits from the store with the same kernel
 // run without the field and the move.
+#include <limits.h>
+
 #include <algorithm>
 
 #include "gx_common.cuh"
@@ -59,6 +61,19 @@
 // shared memory some 11 wavefronts (10M particles, 3D: the pass 282 -> 262 us;
 // 3M in 2D and short items: no change)
 #define BK_STAGE 512
+// The staged rows grow with the spokes, and past some width they cost CTAs: their
+// shared memory is reserved where the SM keeps its CTAs with it, or where the
+// particles suffice for items that use it, BK_STAGE_ROW a row on average (they
+// crowd a part of the rows).  3D steps on 64 rings x 45 planes, us, rows reserved
+// and not: 100k particles (35 a row) 86 and 79 at 256 spokes quadratic, 81 and 76
+// at 512 linear; 500k (173 a row) 115 and 123, 110 and 114.
+#define BK_STAGE_ROW 64
+// Quadratic grids with more spokes than let two CTAs of staged rows onto an SM
+// (256 B a spoke each) take the sorted path: fused and sorted steps of 500k and 3M
+// particles 115 and 278 against 131 and 302 us at 256 spokes, 148 and 341 against
+// 151 and 338 at 384, 160 and 355 against 159 and 347 at 444; with one CTA per SM
+// at 512 213 and 526 against 167 and 367 (179 and 372 without the rows).
+#define BK_QUAD_NA 444
 #define BK_CTASLOT 768      // 2D items with at least this many take their slots by CTA
 #define BK_THREADS 256
 #define PLAN_THREADS 512
@@ -310,7 +325,8 @@ __device__ __forceinline__ void rec_store(float4* __restrict__ Q, int64_t bcap, 
 // ring and plane range; no field, no move, the store is not rewritten
 // Q: the quadratic scheme (3D): 27 nodes around the central one, the window 5
 // rings x 5 planes around the item's row, so that the nodes of every cell a
-// move of less than a cell reaches lie in it; four CTAs per SM (64 registers).
+// move of less than a cell reaches lie in it; four CTAs per SM (64 registers) up
+// to 220 spokes, where the staged rows leave room for them.
 // 500k particles on 64 x 128 x 45: 58.7 us, where the sorted path's push, sort,
 // 27-weight deposit and combine took 75
 template <int ND, bool COMP, bool DEP = false, bool Q = false>
@@ -319,7 +335,7 @@ __global__ void __launch_bounds__(BK_THREADS, Q ? 4 : BK_MINB) k_push_bkt(
     const float4* __restrict__ F,
     const int4* __restrict__ items, int32_t* __restrict__ ctl, const int32_t* __restrict__ cap_o,
     const int32_t* __restrict__ base_o, int32_t* __restrict__ fill_o, int32_t* __restrict__ ovf_o,
-    int64_t ovf_base, unsigned long long* __restrict__ acc, int32_t* __restrict__ rg) {
+    int64_t ovf_base, unsigned long long* __restrict__ acc, int32_t* __restrict__ rg, int stage_min) {
     extern __shared__ __align__(16) uint32_t bins[];
     __shared__ int s_it[2];
     __shared__ int4 s_I[2];
@@ -359,7 +375,7 @@ __global__ void __launch_bounds__(BK_THREADS, Q ? 4 : BK_MINB) k_push_bkt(
         const int wir = I.w;
         const int wiz = d3 ? row - wir * ngz : 0;
         const bool cta = !d3 && (s1 - s0) >= BK_CTASLOT;
-        bool stage = !DEP && row >= 0 && row + (d3 ? ngz : 0) + 1 < nrow && (s1 - s0) >= BK_STAGE;
+        bool stage = !DEP && row >= 0 && row + (d3 ? ngz : 0) + 1 < nrow && (s1 - s0) >= stage_min;
         if (Q) stage = stage && wir >= 1 && wir + 1 < g.nr && wiz >= 1 && wiz + 1 < ngz;
         if (Q && stage) {
             // the 3 x 3 rows around the central one
@@ -868,7 +884,8 @@ __global__ void k_bk_densify(const float4* __restrict__ Qin, int64_t bcap, float
 
 // ---------------------------------------------------------------------------
 bool gx_fast_ok(const GxCtx* c) {
-    return !c->fp64 && c->nzones == 1 && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT);
+    return !c->fp64 && c->nzones == 1 && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT) &&
+           !(c->g.quad && c->g.na > BK_QUAD_NA);
 }
 
 static inline int bk_nplanes(const GxCtx* c) { return 2 * c->g.ndim + (c->g.comp ? c->g.ndim : 0); }
@@ -1115,22 +1132,25 @@ static int bk_launch_push(GxCtx* c, int cur, int nxt) {
     // the deposit window and, for the push, the staged field rows
     const size_t sb = sizeof(uint32_t) * (Q ? 28 : ND == 3 ? 16 : 4) * g.na;  // 25 rows and a pad: 16-byte aligned
     const size_t sf = sb + sizeof(float4) * (Q ? 9 : ND == 3 ? 4 : 2) * g.na;
-    const size_t sm = DEP ? sb : sf;
-    auto kp = k_push_bkt<ND, COMP, DEP, Q>;
-    GX_CUDA(c, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     if (!c->bk_grid) {
-        int per = 0, sms = 148;
+        // CTAs of the push with and without the rows; the deposit alone runs as many
+        int pb = 0, pf = 0, sms = 148;
         auto kf = k_push_bkt<ND, COMP, false, Q>;
         GX_CUDA(c, cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
-        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kf, BK_THREADS, sf));
+        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, kf, BK_THREADS, sf));
+        GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, kf, BK_THREADS, sb));
         GX_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
-        c->bk_grid = std::max(1, per) * sms;
+        c->bk_stage = pf >= pb || c->n >= (int64_t)BK_STAGE_ROW * g.nrow;
+        c->bk_grid = std::max(1, c->bk_stage ? pf : pb) * sms;
     }
+    const size_t sm = DEP || !c->bk_stage ? sb : sf;
+    auto kp = k_push_bkt<ND, COMP, DEP, Q>;
+    GX_CUDA(c, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     c->acc_open = true;
     kp<<<c->bk_grid, BK_THREADS, sm, c->stream>>>(g, c->bq[cur], c->bq[nxt], c->bcap, c->field, c->bk_items,
                                                   c->bk_ctl + 8, c->bk_cap[nxt], c->bk_base[nxt],
                                                   c->bk_fill[nxt], c->bk_ctl + 4 * nxt, c->bk_main, c->macc,
-                                                  gx_mass_ranges(c));
+                                                  gx_mass_ranges(c), c->bk_stage ? BK_STAGE : INT_MAX);
     GX_LAUNCHED(c);
     return GX_OK;
 }

@@ -191,7 +191,8 @@ struct GxCtx {
     int32_t* zr_d = nullptr;                 // [2][2] first, last plane holding the fused pass's mass
                                              // (ngz, -1 when empty), at 2 p of the conversion of set p
     bool zr_valid = false;                   // the mass array is the fused pass's (zr_d describes it)
-    int bk_grid = 0;                         // CTAs of the fused pass
+    int bk_grid = 0;                         // CTAs of the fused pass (0: to be found, for the loaded particles)
+    bool bk_stage = false;                   // its launches reserve the staged field rows
     cudaStream_t bk_side = nullptr;          // the plan's stream (overlaps the field solve)
     cudaEvent_t bk_ev[2] = {nullptr, nullptr};  // push done (main), plan done (side)
     bool bk_pending = false;                 // a plan on bk_side the main stream has not joined
@@ -766,7 +767,7 @@ int gx_zone_masset(GxCtx* c);
 int gx_zone_step(GxCtx* c, int nsteps, int phys);
 int gx_comm_reduce_range(GxCtx* c);
 // fused step on the bucketed store (gx_bucket.cu)
-bool gx_fast_ok(const GxCtx* c);  // single zone, mixed, not GX_FLAG_SORTED_DEPOSIT
+bool gx_fast_ok(const GxCtx* c);  // single zone, mixed, not GX_FLAG_SORTED_DEPOSIT, not quadratic on a wide grid
 int gx_fast_step(GxCtx* c, int nsteps, int phys);
 int gx_dense(GxCtx* c);  // bucketed store -> dense store (no-op when dense)
 int gx_bucket_unload(GxCtx* c, float* aos);  // unload from the bucketed store

@@ -57,6 +57,16 @@ def case(name):
         rec[::50, 3:] *= 20.0  # several cells per step
         flags = GX_FLAG_QUADRATIC | (0 if name == "3d-quadratic" else GX_FLAG_COMPENSATED)
         return cfg3(nr=nr, na=na, ngz=ngz), rec, pm, flags
+    if name.startswith("wide"):
+        # the widest deposit windows and field rows (512 spokes; 444 is the
+        # largest fused quadratic grid), with particles for items that stage the
+        # rows and with too few for it
+        _, na, scheme, n = name.split("-")
+        rec, pm = kt_disk(int(n), seed=9, rmax=4.5, ndim=3, z0=0.1, dt=0.025)
+        rec = rec.copy()
+        rec[::50, 3:] *= 20.0
+        flags = {"linear": 0, "compensated": GX_FLAG_COMPENSATED, "quadratic": GX_FLAG_QUADRATIC}[scheme]
+        return cfg3(nr=24, na=int(na), ng=5), rec, pm, flags
     if name == "bench3":
         rec, pm = kt_disk(1_000_000, seed=12345, rmax=4.8, ndim=3, z0=0.1, dt=0.02)
         return cfg3(nr=128, na=256, ngz=125, dzg=0.04, ng=17, softl=0.1), rec, pm, 0
@@ -92,7 +102,10 @@ def run(cfg, rec, pm, flags):
 
 @pytest.mark.parametrize("name", ["3d", "2d", "3d-compensated", "3d-fast-movers",
                                   "2d-fast-movers", "bench3", "3d-quadratic",
-                                  "3d-quadratic-compensated"])
+                                  "3d-quadratic-compensated", "wide-512-linear-150000",
+                                  "wide-512-compensated-15000", "wide-444-quadratic-150000",
+                                  "wide-444-quadratic-15000", "wide-446-quadratic-15000",
+                                  "wide-512-quadratic-15000"])
 def test_fused_step_is_bitwise_the_sorted_deposit(name):
     cfg, rec, pm, flags = case(name)
     a = run(cfg, rec, pm, flags)
