@@ -123,3 +123,20 @@ def test_gpu_adjoint_at_the_edges_of_its_tiles(nr, na, ng, n):
     assert abs(J - J_ref) < 1e-6 * J_ref, (J, J_ref)
     assert np.linalg.norm(grad - g_ref) < 3e-5 * np.linalg.norm(g_ref)
     assert np.all(np.abs(dth - th_ref) < 1e-4 * np.abs(th_ref)), (dth, th_ref)
+
+
+@pytest.mark.gpu
+def test_gpu_adjoint_gives_its_large_workspace_back():
+    """32 bytes a particle and 16 per checkpoint: 300 checkpoints of 500k
+    particles are 2.4 GB, more than a context keeps between calls."""
+    import torch
+    rec, pm = disc(500_000, 41)
+    with Galaxy(cfg_adj(pmass=pm)) as gal:
+        gal.greenm()
+        gal.loadup(rec)
+        gal.masset()
+        gal.adjoint(2, 1)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        gal.adjoint(299, 1)
+        assert torch.cuda.mem_get_info()[0] >= before
