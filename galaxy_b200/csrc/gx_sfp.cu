@@ -60,6 +60,7 @@ struct GxSfp {
     int32_t* ord_alt = nullptr;
     int32_t* bins = nullptr;    // [SRT_BINS][blocks] counts, then offsets; + [SRT_BINS] totals
     bool reordered = false;
+    bool no_order = false;      // no room for the order's buffers: the loaded particles stay as they are
     int since_sort = 0;         // steps since the last sort
     std::vector<double> qs_h;   // host staging of the force series
     float* part = nullptr;      // per-warp partial moments
@@ -920,7 +921,7 @@ extern "C" int gx_sfp_load(GxSfp* s, const float* coords, int64_t n, int stride)
         SFP_CUDA(s, cudaMalloc((void**)&s->part, bytes));
     }
     s->n = n;
-    s->reordered = false;
+    s->reordered = s->no_order = false;
     s->since_sort = 0;
     if (n == 0) return GX_OK;
     float* tmp = nullptr;
@@ -1461,17 +1462,31 @@ extern "C" int gx_sfp_acc(GxSfp* s, const double* coeff, float* acc, float* pot)
     return GX_OK;
 }
 
-// the particles into radial order (see k_sfp_count); the buffers stay with
-// the loaded particles
+// the buffers of the radial order, which stay with the loaded particles (24.5
+// bytes a particle beside the 80 of the loop itself); false when they do not
+// fit, and none is kept then
+static bool sfp_order_room(GxSfp* s) {
+    if (s->bins) return true;
+    const size_t cap = s->cap, cblk = (cap + SRT_BLOCK - 1) / SRT_BLOCK;
+    if (cudaMalloc((void**)&s->xy_alt, sizeof(float) * 2 * cap) == cudaSuccess &&
+        cudaMalloc((void**)&s->vel_alt, sizeof(float) * 2 * cap) == cudaSuccess &&
+        cudaMalloc((void**)&s->ord, sizeof(int32_t) * cap) == cudaSuccess &&
+        cudaMalloc((void**)&s->ord_alt, sizeof(int32_t) * cap) == cudaSuccess &&
+        cudaMalloc((void**)&s->bins, sizeof(int32_t) * SRT_BINS * (cblk + 1)) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    void* got[] = {s->xy_alt, s->vel_alt, s->ord, s->ord_alt};
+    for (void* q : got)
+        if (q) cudaFree(q);
+    s->xy_alt = s->vel_alt = nullptr;
+    s->ord = s->ord_alt = s->bins = nullptr;
+    return false;
+}
+
+// the particles into radial order (see k_sfp_count)
 static int sfp_sort(GxSfp* s) {
     const int64_t n = s->n;
     const int nblk = (int)((n + SRT_BLOCK - 1) / SRT_BLOCK);
-    const int cblk = (int)((s->cap + SRT_BLOCK - 1) / SRT_BLOCK);
-    if (!s->xy_alt) SFP_CUDA(s, cudaMalloc((void**)&s->xy_alt, sizeof(float) * 2 * s->cap));
-    if (!s->vel_alt) SFP_CUDA(s, cudaMalloc((void**)&s->vel_alt, sizeof(float) * 2 * s->cap));
-    if (!s->ord) SFP_CUDA(s, cudaMalloc((void**)&s->ord, sizeof(int32_t) * s->cap));
-    if (!s->ord_alt) SFP_CUDA(s, cudaMalloc((void**)&s->ord_alt, sizeof(int32_t) * s->cap));
-    if (!s->bins) SFP_CUDA(s, cudaMalloc((void**)&s->bins, sizeof(int32_t) * SRT_BINS * ((size_t)cblk + 1)));
     int32_t* tot = s->bins + (size_t)SRT_BINS * nblk;
     const float scale = (float)((double)(SRT_BINS - 1) / s->maxr);
     k_sfp_count<<<nblk, SRT_THREADS, 0, s->stream>>>(s->xy, s->xy + s->cap, n, scale, nblk, s->bins);
@@ -1514,8 +1529,11 @@ extern "C" int gx_sfp_step(GxSfp* s, int nsteps, double dt, int precision, doubl
                       precision == GX_PREC_MIXED_TC05, pmass / (s->maxr * s->maxr)};
     for (int k = 0; k < nsteps && n > 0; k++) {
         int rc = GX_OK;
-        if (n >= SRT_MIN && (!s->reordered || s->since_sort >= SRT_EVERY)) rc = sfp_sort(s);
-        if (rc) return rc;
+        if (n >= SRT_MIN && !s->no_order && (!s->reordered || s->since_sort >= SRT_EVERY)) {
+            s->no_order = !sfp_order_room(s);
+            if (!s->no_order) rc = sfp_sort(s);
+            if (rc) return rc;
+        }
         rc = sfp_moments(s, precision);
         if (rc) return rc;
         k_sfp_ftab<<<dim3((SFP_NT + 127) / 128, s->b.maxm + 1), 128, 0, s->stream>>>(f, s->mom, s->acheb_d, s->ftab);

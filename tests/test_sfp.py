@@ -201,3 +201,36 @@ def test_sfp_step_in_radial_order_tracks_oracle(basis, n):
     far = np.abs(out[:, :2] - x).max(axis=1) / np.abs(x).max()
     assert np.mean(far > 1e-5) < 2e-3 and far[ok].max() < 1e-3, far.max()
     assert np.linalg.norm(c - c_ref) < 1e-4 * np.linalg.norm(c_ref)
+
+
+@pytest.mark.gpu
+def test_sfp_step_without_room_for_the_radial_order(basis):
+    """A loop that cannot allocate the second copies of the particles runs in
+    load order instead: the same orbits up to the order of the FP32 sums (the
+    bounds of the loop against the oracle above)."""
+    import torch
+    from galaxy_b200.sfp import Sfp
+    n, nsteps, dt = 8_000_000, 3, 0.05
+    rng = np.random.default_rng(9)
+    rec = np.zeros((n, 4), np.float32)
+    rec[:, :2] = exp_disk(n, seed=29)
+    rec[:, 2:] = 0.4 * rng.standard_normal((n, 2))
+    out = []
+    for full in (False, True):
+        with Sfp(basis, 6.0) as s:
+            s.load(rec)
+            s.sum(pmass=1.0 / n)
+            hold = None
+            if full:
+                # all but 96 MB; the order's buffers take 196 MB
+                hold = torch.empty(torch.cuda.mem_get_info()[0] - (96 << 20), dtype=torch.uint8, device="cuda")
+            try:
+                c = s.step(nsteps, dt, pmass=1.0 / n)
+            finally:
+                del hold
+                torch.cuda.empty_cache()
+            out.append((c, s.unload()))
+    (c0, p0), (c1, p1) = out
+    assert np.linalg.norm(c0 - c1) < 1e-5 * np.linalg.norm(c0)
+    far = np.abs(p0 - p1).max(axis=1)
+    assert np.mean(far > 1e-4) < 1e-6  # a particle at the basis edge may differ by its force
