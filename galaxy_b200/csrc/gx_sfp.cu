@@ -1534,8 +1534,12 @@ extern "C" int gx_sfp_step(GxSfp* s, int nsteps, double dt, int precision, doubl
             if (!s->no_order) rc = sfp_sort(s);
             if (rc) return rc;
         }
+        // (gx_sfp_last_ms: the last sum)
+        s->launches = 0;
+        if (k == nsteps - 1) SFP_CUDA(s, cudaEventRecord(s->e0, s->stream));
         rc = sfp_moments(s, precision);
         if (rc) return rc;
+        if (k == nsteps - 1) SFP_CUDA(s, cudaEventRecord(s->e1, s->stream));
         k_sfp_ftab<<<dim3((SFP_NT + 127) / 128, s->b.maxm + 1), 128, 0, s->stream>>>(f, s->mom, s->acheb_d, s->ftab);
         SFP_CUDA(s, cudaGetLastError());
         k_sfp_kick<<<(unsigned)((n + 255) / 256), 256, 0, s->stream>>>(
@@ -1552,6 +1556,7 @@ extern "C" int gx_sfp_step(GxSfp* s, int nsteps, double dt, int precision, doubl
         return GX_OK;
     }
     SFP_CUDA(s, cudaStreamSynchronize(s->stream));
+    if (nsteps > 0 && n > 0) SFP_CUDA(s, cudaEventElapsedTime(&s->last_ms, s->e0, s->e1));
     return sfp_check(s);
 }
 

@@ -234,3 +234,19 @@ def test_sfp_step_without_room_for_the_radial_order(basis):
     assert np.linalg.norm(c0 - c1) < 1e-5 * np.linalg.norm(c0)
     far = np.abs(p0 - p1).max(axis=1)
     assert np.mean(far > 1e-4) < 1e-6  # a particle at the basis edge may differ by its force
+
+
+@pytest.mark.gpu
+def test_sfp_last_ms_is_of_one_sum_after_a_step_too(basis):
+    """gx_sfp_step without coefficients: the launches reported are those of its
+    last sum, not of all of them."""
+    from galaxy_b200.sfp import Sfp
+    rec = np.zeros((40000, 4), np.float32)
+    rec[:, :2] = exp_disk(40000, seed=31)
+    with Sfp(basis, 6.0) as s:
+        s.load(rec)
+        s.sum()
+        _, nl = s.last_ms()
+        assert s._L.gx_sfp_step(s._h, 5, 0.05, 0, 1e-5, None) == 0
+        ms, nl5 = s.last_ms()
+    assert nl5 == nl and 0.0 < ms < 1.0, (ms, nl5, nl)
