@@ -496,9 +496,10 @@ static int zone_deposit(GxCtx* c, int mzone, int32_t* perm_out) {
     return GX_OK;
 }
 
-// whether this context's particles take the direct path (GX_FLAG_SORTED_DEPOSIT: the sorted one)
+// whether this context's particles take the direct path (GX_FLAG_SORTED_DEPOSIT,
+// or no room for the zones' accumulators: the sorted one)
 static bool zone_direct(const GxCtx* c) {
-    return c->n <= ZONE_DIRECT && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT);
+    return c->zacc && c->n <= ZONE_DIRECT && !(c->cfg.flags & GX_FLAG_SORTED_DEPOSIT);
 }
 
 static ZoneAcc zone_acc(const GxCtx* c) { return {c->macc, c->zacc, c->zjrk_d + 2 * GX_MAX_ZONES + 2}; }
@@ -695,7 +696,6 @@ int gx_set_zones(GxCtx* c, int32_t nzones, const int32_t* nstep, const float* zb
     if (nzones == 1) return GX_OK;
     const size_t mesh = c->g.mesh;
     if (cudaMalloc((void**)&c->zbuf, sizeof(float) * 2 * (nzones - 1) * mesh) != cudaSuccess ||
-        cudaMalloc((void**)&c->zacc, sizeof(unsigned long long) * (nzones - 1) * mesh) != cudaSuccess ||
         cudaMalloc((void**)&c->zjrk_d, sizeof(int32_t) * (4 * GX_MAX_ZONES + 2)) != cudaSuccess) {
         c->nzones = 1;
         return c->err = "cudaMalloc of the zone mass arrays failed", GX_ERR_NOMEM;
@@ -705,7 +705,12 @@ int gx_set_zones(GxCtx* c, int32_t nzones, const int32_t* nstep, const float* zb
         c->zold[k] = c->zbuf + (size_t)(2 * (k - 1) + 1) * mesh;
     }
     GX_CUDA(c, cudaMemset(c->zbuf, 0, sizeof(float) * 2 * (nzones - 1) * mesh));
-    GX_CUDA(c, cudaMemset(c->zacc, 0, sizeof(unsigned long long) * (nzones - 1) * mesh));
+    if (cudaMalloc((void**)&c->zacc, sizeof(unsigned long long) * (nzones - 1) * mesh) != cudaSuccess) {
+        cudaGetLastError();
+        c->zacc = nullptr;
+    } else {
+        GX_CUDA(c, cudaMemset(c->zacc, 0, sizeof(unsigned long long) * (nzones - 1) * mesh));
+    }
     int32_t rng[2 * GX_MAX_ZONES];
     for (int k = 0; k < GX_MAX_ZONES; k++) {
         rng[2 * k] = 0x7fffffff;

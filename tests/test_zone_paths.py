@@ -54,3 +54,33 @@ def test_direct_zone_steps_equal_the_sorted_ones(ndim, flags, nstep, zbr, n):
         assert np.array_equal(a, b)
     if n > 1000:
         assert len(np.unique(out[0][-2])) == len(nstep) + 1  # every zone and the off-grid list
+
+
+def test_zones_without_room_for_their_accumulators():
+    """A large mesh on a nearly full device: the zones' integer accumulators
+    (twice their mass arrays) do not fit, and the run takes the sorted path,
+    which does without them; the same bits."""
+    import torch
+    cfg = make_config(2, 4096, 512, ng=1, rmap=GX_RMAP_LOG, rmap_a=float(np.log(100.0) / 4095), rmap_r0=0.05,
+                      softl=0.05, tsoft=1)
+    rec, pm = kt_disk(30000, seed=6, rmax=4.9, ndim=2, dt=0.05)
+    cfg.pmass = pm
+    out = []
+    for full in (False, True):
+        with Galaxy(cfg) as gal:
+            hold = None
+            if full:
+                # mass arrays of three more zones 50 MB, their accumulators 50 MB
+                gal.loadup(rec)   # the particle arrays first
+                gal.loadup(rec[:0])
+                hold = torch.empty(torch.cuda.mem_get_info()[0] - (80 << 20), dtype=torch.uint8, device="cuda")
+            try:
+                gal.set_zones([1, 2, 4, 8], [0.0, 1.0, 2.0, 3.0])
+            finally:
+                del hold
+                torch.cuda.empty_cache()
+            gal.loadup(rec)
+            gal.masset()
+            out.append((gal.grid(GX_GRID_MASS), *gal.zone_info()[:1]))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
