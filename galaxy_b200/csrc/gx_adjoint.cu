@@ -68,15 +68,8 @@ __device__ __forceinline__ void adj_accel(const DevGeo& g, const float4* F, cons
         ax += f.x * w[k];
         ay += f.y * w[k];
     }
-    if (g.halo == 1) {
-        const float r2 = x * x + y * y, rr = sqrtf(r2);
-        float fr = -g.halo_v2 * rr / (r2 + g.halo_rc2);
-        if (fr != 0.f) {
-            fr = fr / rr;
-            ax += fr * x;
-            ay += fr * y;
-        }
-    }
+    float az = 0.f, ph = 0.f;
+    gx_rigid_force(g, x, y, 0.f, ax, ay, az, ph);
 }
 
 // particles in load order from the context's storage order, one record

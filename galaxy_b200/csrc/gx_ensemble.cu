@@ -412,18 +412,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_ens_step(EnsArgs A, int nsteps) 
                             ay += f.y * w[q];
                         }
                     }
-                    if (g.halo == 1 && cw.key >= 0) {
-                        const float r2 = x * x + y * y;
-                        const float rr = sqrtf(r2);
-                        float fr = -g.halo_v2 * rr / (r2 + g.halo_rc2);
-                        if (fr != 0.f) {
-                            fr = fr / rr;
-                            ax += fr * x;
-                            ay += fr * y;
-                        }
-                    } else if (g.halo == 2 && cw.key >= 0) {
-                        float az_ = 0.f, ph_ = 0.f;
-                        gx_disc_force(g, x, y, 0.f, ax, ay, az_, ph_);
+                    if (cw.key >= 0) {
+                        float az = 0.f, ph = 0.f;
+                        gx_rigid_force(g, x, y, 0.f, ax, ay, az, ph);
                     }
                     // stpgrp.f:26-32
                     vx += ax;

@@ -90,6 +90,27 @@ def test_ensemble_a2_series_matches_particles():
         assert abs(a[5, d] - a2_of(cfg, out[d])) < 1e-10, (d, a[5, d], a2_of(cfg, out[d]))
 
 
+def test_ensemble_disc_in_a_halo_alone_is_its_single_run():
+    """Massless particles: the field is zero and the halo the only force, so an
+    ensemble's disc and the single run differ only if they form the halo's force
+    in different ways.  Bit for bit."""
+    cfg = cfg_c1()
+    cfg.halo, cfg.halo_v2, cfg.halo_rc, cfg.pmass = 1, 0.49 * 0.025 ** 2, 1.0, 0.0
+    recs, _ = discs([5000], seed0=700)
+    ens = Ensemble(cfg, recs, np.zeros(1, np.float32), max_steps=20)
+    ens.step(20)
+    out = ens.unload()[0]
+    ens.close()
+    with Galaxy(cfg) as gal:
+        gal.greenm()
+        gal.loadup(recs[0])
+        gal.masset()
+        gal.step(20)
+        single = gal.unload()
+    assert np.abs(single[:, 2:] - recs[0][:, 2:]).max() > 1e-3
+    assert np.array_equal(out, single)
+
+
 def test_ensemble_graph_and_direct_launches_agree_bitwise():
     cfg = cfg_c1()
     recs, pms = discs([5000, 20000, 700, 11000], seed0=300)
