@@ -126,6 +126,30 @@ def test_gpu_adjoint_at_the_edges_of_its_tiles(nr, na, ng, n):
 
 
 @pytest.mark.gpu
+def test_gpu_adjoint_on_a_used_context():
+    """One context taken through other numbers of particles, steps and
+    checkpoints: every call gives what a fresh context gives (the gradient up to
+    the order of its FP64 sums)."""
+    cfg = cfg_adj()
+    calls = [(3000, 12, 1), (3000, 5, 5), (700, 9, 2), (4001, 3, 1), (3000, 12, 4)]
+    recs = {n: disc(n, n)[0] for n, _, _ in calls}
+    with Galaxy(cfg) as gal:
+        gal.greenm()
+        for n, T, ckpt in calls:
+            gal.loadup(recs[n])
+            gal.masset()
+            got = gal.adjoint(T, ckpt)
+            with Galaxy(cfg) as g2:
+                g2.greenm()
+                g2.loadup(recs[n])
+                g2.masset()
+                ref = g2.adjoint(T, ckpt)
+            assert got[0] == ref[0] and got[3] == ref[3]
+            assert np.linalg.norm(got[1] - ref[1]) <= 1e-6 * np.linalg.norm(ref[1])
+            assert np.all(np.abs(got[2] - ref[2]) <= 1e-9 * np.abs(ref[2]))
+
+
+@pytest.mark.gpu
 def test_gpu_adjoint_gives_its_large_workspace_back():
     """32 bytes a particle and 16 per checkpoint: 300 checkpoints of 500k
     particles are 2.4 GB, more than a context keeps between calls."""

@@ -1,7 +1,7 @@
 """Batched ensemble of 2D discs (gx_ensemble_*): each disc against its own
 single-disc run and the FP64 oracle, the A2 series against the particles,
-determinism across the graph and direct launch paths and across the
-autotuner's launch shapes."""
+determinism across the numbers of steps per launch and across the autotuner's
+launch shapes."""
 import numpy as np
 import pytest
 
@@ -111,21 +111,87 @@ def test_ensemble_disc_in_a_halo_alone_is_its_single_run():
     assert np.array_equal(out, single)
 
 
-def test_ensemble_graph_and_direct_launches_agree_bitwise():
+def test_ensemble_steps_agree_bitwise_however_they_are_launched():
+    """130 steps in one call (two launches of 64 steps and one of 2), step by
+    step, and in calls of 63, 1 and 66: the same particles and series."""
     cfg = cfg_c1()
     recs, pms = discs([5000, 20000, 700, 11000], seed0=300)
-    e1 = Ensemble(cfg, recs, pms, max_steps=20)
-    e1.step(20)  # one replay of the 16-step graph + 4 direct launches
-    e2 = Ensemble(cfg, recs, pms, max_steps=20)
-    for _ in range(20):
-        e2.step(1)
-    p1, p2 = e1.unload(), e2.unload()
-    a1, a2 = e1.a2(), e2.a2()
-    e1.close()
-    e2.close()
-    for x, y in zip(p1, p2):
-        assert np.array_equal(x, y)
-    assert np.array_equal(a1, a2)
+    out = []
+    for calls in ([130], [1] * 130, [63, 1, 66]):
+        e = Ensemble(cfg, recs, pms, max_steps=130)
+        for k in calls:
+            e.step(k)
+        out.append((e.unload(), e.a2()))
+        e.close()
+    for pos, a2 in out[1:]:
+        for x, y in zip(out[0][0], pos):
+            assert np.array_equal(x, y)
+        assert np.array_equal(out[0][1], a2)
+
+
+def test_ensemble_disc_concentrated_in_one_cell():
+    """12000 particles next to one mesh node, in one chunk: its 32-bit bin wraps
+    (4096 whole weights a turn), and more particles than that share each of the
+    neighbours.  The disc against its own single run, whose deposit adds up
+    differently; bounds of the discs above."""
+    cfg = cfg_c1()
+    nsteps = 4
+    a = np.log(100.0) / 63
+    rng = np.random.default_rng(8)
+    r = 0.05 * np.exp(a * (50 + 0.05 + 0.1 * rng.random(12000)))
+    ph = 2 * np.pi * (20 + 0.05 + 0.1 * rng.random(12000)) / 128
+    clump = np.stack([r * np.cos(ph), r * np.sin(ph), -1e-3 * np.sin(ph), 1e-3 * np.cos(ph)], 1).astype(np.float32)
+    key, w = None, None
+    with Galaxy(cfg) as gal:
+        key, w = gal.weight(clump)
+    assert len(np.unique(key)) == 1 and w.sum(axis=0).max() > 2 * 4096
+    recs, pms = discs([3000])
+    recs, pms = [recs[0], clump], np.array([pms[0], 1e-9], np.float32)
+    ens = Ensemble(cfg, recs, pms, max_steps=nsteps)
+    ens.step(nsteps)
+    out = ens.unload()
+    a2 = ens.a2()
+    ens.close()
+    for d, rec in enumerate(recs):
+        c = cfg_c1()
+        c.pmass = float(pms[d])
+        with Galaxy(c) as gal:
+            gal.greenm()
+            gal.loadup(rec)
+            gal.masset()
+            gal.step(nsteps)
+            single = gal.unload().astype(np.float64)
+        dx, frac = close_positions(out[d], single)
+        assert dx < 1e-4 and frac < 1e-3, (d, dx, frac)
+        # and the step lengths, which show the force
+        dv = np.abs(out[d][:, 2:] - single[:, 2:]).max() / np.abs(single[:, 2:] - rec[:, 2:]).max()
+        assert dv < 1e-3, (d, dv)
+        assert abs(a2[-1, d] - a2_of(cfg, out[d])) < 1e-10
+
+
+def test_ensemble_of_many_discs_some_of_them_empty():
+    """More discs than the launch has CTAs, and discs without particles between
+    them: each disc as in an ensemble of its own, bit for bit; an empty disc's
+    series is zero."""
+    cfg = make_config(2, 20, 32, ng=5, rmap=GX_RMAP_LOG, rmap_a=float(np.log(100.0) / 19), rmap_r0=0.05,
+                      softl=0.3, tsoft=1, pmass=1.0)
+    counts = [0 if i % 7 == 3 else 200 + i for i in range(700)]
+    recs, pms = discs([max(c, 1) for c in counts], seed0=900)
+    recs = [r[:c] for r, c in zip(recs, counts)]
+    ens = Ensemble(cfg, recs, pms, max_steps=70)
+    assert ens.config()["grid"] < len(counts)
+    ens.step(70)
+    out, a2 = ens.unload(), ens.a2()
+    ens.close()
+    for d in (0, 1, 2, 3, 10, 350, 698, 699):
+        if not counts[d]:
+            assert len(out[d]) == 0 and not a2[:, d].any()
+            continue
+        e = Ensemble(cfg, [recs[d]], pms[d:d + 1], max_steps=70)
+        e.step(70)
+        assert np.array_equal(e.unload()[0], out[d]), d
+        assert np.array_equal(e.a2()[:, 0], a2[:, d]), d
+        e.close()
 
 
 def test_ensemble_tuner_restores_state_and_keeps_results():

@@ -167,8 +167,8 @@ def test_sfp_sum_64_chebyshev_terms(basis):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n", [32768, 40001])
-def test_sfp_step_in_radial_order_tracks_oracle(basis, n):
+@pytest.mark.parametrize("n,precision", [(32768, 0), (40001, 0), (33001, 1), (33001, 2)])
+def test_sfp_step_in_radial_order_tracks_oracle(basis, n, precision):
     """Enough particles for the loop to keep them in radial order: 18 steps
     (the order renewed twice), some particles outside the basis edge and one
     at the centre.  Records, forces and coefficients come back in load order;
@@ -190,8 +190,8 @@ def test_sfp_step_in_radial_order_tracks_oracle(basis, n):
     c_ref = ox.sfp_coeffs(basis, x, maxr, pmass=pm)
     with Sfp(basis, maxr) as s:
         s.load(rec)
-        s.step(5, dt, pmass=pm)
-        c = s.step(nsteps - 5, dt, pmass=pm)
+        s.step(5, dt, pmass=pm, precision=precision)
+        c = s.step(nsteps - 5, dt, pmass=pm, precision=precision)
         out = s.unload()
         acc, _ = s.acc(c)
         s.load(out)
