@@ -507,7 +507,7 @@ def run_ensemble(ndisc=64, steps=1000, loop_steps=20, seed=12345):
     ach = eb / (ms / steps * 1e-3) / 1e9
     return {"workload": f"ensemble2d-{ndisc}x64x128-{ntot}", "discs": ndisc, "particles": ntot,
             "steps": steps, "ms_per_step": round(ms / steps, 4), "particle_steps_per_s": rate,
-            "launches_per_step": launches / steps, "cuda_graph": conf["graph"],
+            "launches_per_step": launches / steps,
             "tuned": {"threads": threads, "chunk": chunk, "ctas": conf["grid"]},
             "per_run_loop": {"particle_steps_per_s": rate_loop, "steps": loop_steps,
                              "ms_per_step_all_discs": round(t_loop / loop_steps, 4)},

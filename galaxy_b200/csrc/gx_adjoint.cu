@@ -637,7 +637,6 @@ static int adj_run(GxCtx* c, int nsteps, int ckpt_every, double* J_out, float* g
     GX_LAUNCHED(c);
     if (g.comp)  // the low parts of compensated positions start at zero, as after gx_loadup
         GX_CUDA(c, cudaMemsetAsync(c->pbuf[c->cur] + (size_t)4 * c->cap, 0, sizeof(float) * 2 * c->cap, st));
-    c->have_keys = false;
     c->zr_valid = false;
     int rc = gx_mixed_masset(c);
     if (rc) return rc;

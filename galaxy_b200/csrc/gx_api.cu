@@ -485,7 +485,7 @@ int gx_loadup(GxCtx* c, const float* coords, int64_t n) {
     int rc = alloc_particles(c, n);
     if (rc) return rc;
     c->n = n;
-    c->have_mass = c->have_field = c->have_keys = false;
+    c->have_mass = c->have_field = false;
     c->bucketed = false;
     c->zr_valid = false;
     c->bk_grid = 0;

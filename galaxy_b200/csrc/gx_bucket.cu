@@ -56,10 +56,10 @@
 // costs about as much; 32 to 256 are within 2 % at 170 to 310 particles a row)
 #define BK_SPARSE 128
 // items with at least this many particles copy the field rows of their cells
-// (4 rows in 3D, 2 in 2D) into shared memory and gather there: the gathers of a
-// row's particles touch some 20 lines of the first-level cache per load, in
-// shared memory some 11 wavefronts (10M particles, 3D: the pass 282 -> 262 us;
-// 3M in 2D and short items: no change)
+// (4 rows in 3D, 2 in 2D) into shared memory and gather there: a warp's gather
+// touches 29 sectors of the first-level cache, in shared memory it takes 11
+// wavefronts (10M particles, 3D: the pass 282 -> 262 us; 3M in 2D and short
+// items: no change)
 #define BK_STAGE 512
 // The staged rows grow with the spokes, and past some width they cost CTAs: their
 // shared memory is reserved where the SM keeps its CTAs with it, or where the
@@ -1078,7 +1078,6 @@ static int gx_bucketize(GxCtx* c) {
     if (rc) return rc;
     c->bcur = b;
     c->bucketed = true;
-    c->have_keys = false;
     return GX_OK;
 }
 
@@ -1105,7 +1104,6 @@ int gx_dense(GxCtx* c) {
         GX_LAUNCHED(c);
     }
     c->bucketed = false;
-    c->have_keys = false;
     return GX_OK;
 }
 

@@ -87,7 +87,6 @@ struct GxCtx {
     int32_t* pkey[2] = {nullptr, nullptr}; // cell key (ncl - 1, -1 off the grid) of the particles of pbuf[i]
     float* pfr = nullptr;                  // cell fractions du, dt, dz of pkey[cur], SoA [3][cap],
                                            // written by the pass that keyed them for its deposit
-    bool have_keys = false;                // pkey[cur] matches pbuf[cur]
     double* p64 = nullptr;                 // SoA [2*ndim][cap] (FP64 path)
     int32_t* key64 = nullptr;
     double* w64 = nullptr;                 // [8][cap]
@@ -705,11 +704,12 @@ __device__ __forceinline__ void gx_accel_cell(const DevGeo& g, const float4* __r
 // gain from that cache) with ordinary loads, never through the read-only path.
 // Zoned step of 15000 particles, five launches: 26.6 -> 20.5 us; adjoint of 400k
 // particles on 128 x 256, 13 launches a step: 126.5 -> 117.4 us; 3D step of 200k particles on
-// an odd grid, solve kernels only: 86.4 -> 85.7 us.  What a kernel may read ahead of
-// its wait is complete because a forward transform waits before it lets the
-// contraction start: constant tables, and the mass's ring and plane ranges (the
-// contraction's first Green tiles and the ring synthesis' tables so: 85.2 -> 84.5
-// us).  The mass conversion is not chained: CTAs of the transform that wait beside
+// an odd grid, solve kernels only: 86.4 -> 85.7 us.  The 3D forward transforms wait
+// before they let the contraction start, so that the 3D kernels behind them may read
+// ahead of their own wait what was complete by then: constant tables, and the mass's
+// ring and plane ranges (the contraction's first Green tiles and the ring synthesis'
+// tables so: 85.2 -> 84.5 us).  In 2D nothing may be read ahead: k_fwd2 lets the
+// contraction start before it has written those ranges itself.  The mass conversion is not chained: CTAs of the transform that wait beside
 // it cost the plan on the side stream its place (85.6 -> 89.9 us).
 __device__ __forceinline__ void gx_chain_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void gx_chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -456,6 +456,5 @@ int gx_mixed_masset(GxCtx* c) {
     }
     int rc = gx_deposit_rows(c, c->pkey[c->cur], c->pfr, c->perm);
     if (rc) return rc;
-    c->have_keys = true;
     return gx_phase_end(c);
 }

@@ -245,7 +245,7 @@ __global__ void k_zone_combine(int64_t mesh, float* __restrict__ mass, ZoneSrc s
 // Steps of at most ZONE_DIRECT particles.  A zoned step of a few ten thousand
 // particles is bound by its launches: run100 (15000 particles on 93 x 128) took
 // 14 launches and 81 us a step with the per-zone sort, deposit and combine,
-// five launches and 26 us here.  The direct reductions into the mesh and the
+// five launches and 26 us here, 20 with their starts overlapped (gx_chain).  The direct reductions into the mesh and the
 // unordered gathers cost more per particle than the sorted path's passes, so
 // the two meet at the line below.  Step times, direct and sorted, 2 zones:
 // 2D 93 x 128, 100k 30 / 80 us, 300k 45 / 87, 1M 91 / 127, 2M 155 / 183; 3D 85 x
@@ -609,7 +609,6 @@ int gx_zone_masset(GxCtx* c) {
     if (rc) return rc;
     rc = zone_combine(c, c->nzones);
     if (rc) return rc;
-    c->have_keys = true;
     c->zones_ready = true;
     return gx_phase_end(c);
 }

@@ -1,7 +1,7 @@
 """Ensemble of independent 2D discs on one GPU (a GxEnsemble).
 
-The discs share one polar grid geometry and Green table; every step of all
-of them is one persistent launch (gx_ensemble_step in
+The discs share one polar grid geometry and Green table; up to 64 steps of
+all of them are one persistent launch (gx_ensemble_step in
 galaxy_b200/csrc/gx_ensemble.cu).  Each disc follows the single-disc run
 (SRC/progs/galaxy.f:107-148: findf, getacc + stpgrp, massgn).
 """

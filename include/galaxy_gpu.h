@@ -10,6 +10,9 @@
  * Conventions
  *  - Every entry point returns GX_OK (0) or a negative GX_ERR_* code; the
  *    message is available from gx_last_error().  Nothing aborts the process.
+ *    A gx_masset, gx_step or gx_adjoint that fails after it deposited
+ *    particles drops that deposit; the context then has no mass array until
+ *    the next gx_masset.  A call refused before that changes nothing.
  *  - Pointers passed in are host pointers, valid for the duration of the
  *    call only.  Device memory is owned by the context.
  *  - A context is not re-entrant: one host thread at a time; all work is
