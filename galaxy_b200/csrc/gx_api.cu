@@ -148,6 +148,7 @@ static int dalloc(GxCtx* c, T** p, size_t count) {
     cudaError_t e = cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(count, 1));
     if (e != cudaSuccess) {
         c->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
+        cudaGetLastError();  // reported here, not by the next launch
         *p = nullptr;
         return GX_ERR_NOMEM;
     }
@@ -233,6 +234,7 @@ int gx_grdset(const GxConfig* cfg, GxCtx** out) {
         // the active harmonics, once per context (the kernels read them through DevGeo)
         if (cudaMalloc((void**)&c->act_d, sizeof(int) * 260) != cudaSuccess ||
             cudaMemcpy(c->act_d, c->spec.m, sizeof(int) * 260, cudaMemcpyHostToDevice) != cudaSuccess) {
+            cudaGetLastError();
             c->err = "cudaMalloc of the harmonic list failed";
             rc = GX_ERR_NOMEM;
         }
@@ -641,6 +643,7 @@ int gx_host_alloc(int64_t bytes, void** ptr) {
     if (!ptr || bytes < 0) return GX_ERR_ARG;
     *ptr = nullptr;
     if (cudaMallocHost(ptr, (size_t)std::max<int64_t>(bytes, 1)) != cudaSuccess) {
+        cudaGetLastError();
         *ptr = nullptr;
         return GX_ERR_NOMEM;
     }

@@ -949,6 +949,7 @@ template <typename T>
 static int bk_alloc(GxCtx* c, T** p, size_t count) {
     if (*p) return GX_OK;
     if (cudaMalloc((void**)p, sizeof(T) * std::max<size_t>(count, 1)) != cudaSuccess) {
+        cudaGetLastError();
         *p = nullptr;
         c->err = "cudaMalloc of the bucketed store's tables failed";
         return GX_ERR_NOMEM;

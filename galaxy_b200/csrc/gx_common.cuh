@@ -218,6 +218,7 @@ int gx_phase_end(GxCtx* c);
         cudaError_t e_ = (call);                                            \
         if (e_ != cudaSuccess) {                                            \
             (ctx)->err = std::string(#call) + ": " + cudaGetErrorString(e_);\
+            cudaGetLastError(); /* reported here, not by the next launch */ \
             return GX_ERR_CUDA;                                             \
         }                                                                   \
     } while (0)

@@ -551,6 +551,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_ens_step(EnsArgs A, int nsteps) 
         cudaError_t e_ = (call);                                             \
         if (e_ != cudaSuccess) {                                             \
             (e)->err = std::string(#call) + ": " + cudaGetErrorString(e_);   \
+            cudaGetLastError(); /* reported here, not by the next launch */  \
             return GX_ERR_CUDA;                                              \
         }                                                                    \
     } while (0)

@@ -808,6 +808,7 @@ __global__ void k_sfp_kick(float* __restrict__ X, float* __restrict__ Y, float* 
         cudaError_t e_ = (call);                                                 \
         if (e_ != cudaSuccess) {                                                 \
             (s)->err = std::string(#call) + ": " + cudaGetErrorString(e_);       \
+            cudaGetLastError(); /* reported here, not by the next launch */      \
             return GX_ERR_CUDA;                                                  \
         }                                                                        \
     } while (0)
@@ -854,7 +855,8 @@ extern "C" int gx_sfp_init(const GxSfpBasis* b, double maxr, int device, GxSfp**
     if (e == cudaSuccess) e = cudaMemset(s->errword, 0, sizeof(int32_t));
     if (e != cudaSuccess) {
         g_sfp_err = std::string("CUDA: ") + cudaGetErrorString(e);
-        delete s;
+        cudaGetLastError();
+        gx_sfp_destroy(s);
         return GX_ERR_CUDA;
     }
     *out = s;

@@ -569,6 +569,7 @@ int gx_zone_loadup(GxCtx* c) {
     const int64_t n = c->n;
     for (int b = 0; b < 2; b++)
         if (!c->pzone[b] && cudaMalloc((void**)&c->pzone[b], sizeof(int32_t) * c->cap) != cudaSuccess) {
+            cudaGetLastError();
             c->pzone[b] = nullptr;
             return c->err = "cudaMalloc of the zone codes failed", GX_ERR_NOMEM;
         }
@@ -696,6 +697,7 @@ int gx_set_zones(GxCtx* c, int32_t nzones, const int32_t* nstep, const float* zb
     const size_t mesh = c->g.mesh;
     if (cudaMalloc((void**)&c->zbuf, sizeof(float) * 2 * (nzones - 1) * mesh) != cudaSuccess ||
         cudaMalloc((void**)&c->zjrk_d, sizeof(int32_t) * (4 * GX_MAX_ZONES + 2)) != cudaSuccess) {
+        cudaGetLastError();
         c->nzones = 1;
         return c->err = "cudaMalloc of the zone mass arrays failed", GX_ERR_NOMEM;
     }

@@ -61,3 +61,38 @@ def test_zoned_run_that_fails_leaves_no_deposit_behind(flags):
         gal.step(3)
         assert np.array_equal(gal.unload(), ref[0])
         assert np.array_equal(gal.grid(GX_GRID_MASS), ref[1])
+
+
+def almost_full(left):
+    """All of the device's free memory but `left` bytes, held until released"""
+    import torch
+    torch.cuda.init()
+    return torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+
+
+def release():
+    import torch
+    torch.cuda.empty_cache()
+
+
+def test_allocation_that_fails_does_not_fail_the_next_call():
+    """A call that finds no memory returns that error, and the next one, with
+    memory again, is not told of it."""
+    rec, pm = kt_disk(20000, seed=5, rmax=4.9, ndim=2, dt=0.05, lscale=10.0)
+    out = []
+    for full in (False, True):
+        with Galaxy(cfg2(ng=9, pmass=pm)) as gal:
+            gal.greenm()
+            gal.loadup(rec)
+            gal.masset()
+            if full:
+                hold = almost_full(4 << 20)
+                try:
+                    with pytest.raises(GxError):
+                        gal.greenm()
+                finally:
+                    del hold
+                    release()
+            gal.step(2)
+            out.append(gal.unload())
+    assert np.array_equal(*out)
