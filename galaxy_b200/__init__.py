@@ -170,13 +170,13 @@ class Galaxy:
     def loadup(self, coords):
         coords = np.ascontiguousarray(coords, dtype=np.float32)
         assert coords.ndim == 2 and coords.shape[1] == 2 * self.ndim
+        self._chk(self._L.gx_loadup(self._h, _ptr(coords), coords.shape[0]))
         self.n = coords.shape[0]
-        self._chk(self._L.gx_loadup(self._h, _ptr(coords), self.n))
 
     def loadup_ptr(self, ptr, n):
         """loadup from a host pointer (e.g. pinned memory) of n records."""
+        self._chk(self._L.gx_loadup(self._h, C.c_void_p(ptr), int(n)))
         self.n = int(n)
-        self._chk(self._L.gx_loadup(self._h, C.c_void_p(ptr), self.n))
 
     def unload_ptr(self, ptr):
         self._chk(self._L.gx_unload(self._h, C.c_void_p(ptr)))

@@ -392,7 +392,11 @@ __global__ void k_iota(int32_t* p, int64_t n) {
 static int alloc_particles(GxCtx* c, int64_t n) {
     const int nw = 2 * c->g.ndim;
     if (n <= c->cap && c->cap > 0) return GX_OK;
-    // grow: free old
+    // grow: free old.  Until every new array is there the context has no
+    // particles and no capacity, so that a call that finds no memory leaves
+    // nothing that a later one would take for arrays
+    c->n = c->cap = 0;
+    c->have_mass = c->have_field = c->zones_ready = c->zr_valid = false;
     void* old[] = {c->pbuf[0], c->pbuf[1], c->perm, c->origin, c->origin_tmp, c->pkey[0], c->pkey[1],
                    c->pfr, c->p64,
                    c->key64, c->w64, c->acc64, c->pot64, c->ppot, c->pacc, c->perm_next, c->items,
@@ -422,8 +426,7 @@ static int alloc_particles(GxCtx* c, int64_t n) {
     if (c->adj_ws) cudaFree(c->adj_ws);
     c->adj_ws = nullptr;
     c->adj_bytes = 0;
-    int64_t cap = std::max<int64_t>(n, 1);
-    c->cap = cap;
+    const int64_t cap = std::max<int64_t>(n, 1);
     DALLOC(c, c->ppot, cap);
     DALLOC(c, c->pacc, 3 * cap);
     // staging of the host records (AoS) for loadup and unload, once per
@@ -435,6 +438,7 @@ static int alloc_particles(GxCtx* c, int64_t n) {
         DALLOC(c, c->w64, 8 * cap);
         DALLOC(c, c->acc64, 3 * cap);
         DALLOC(c, c->pot64, cap);
+        c->cap = cap;
         return GX_OK;
     }
     // compensated positions keep a low part of every coordinate after the
@@ -475,6 +479,7 @@ static int alloc_particles(GxCtx* c, int64_t n) {
     c->bcap = c->bk_main + cap + 64;
     if (c->bcap > (int64_t)INT32_MAX) return c->err = "too many particles for the bucketed store", GX_ERR_RANGE;
     for (int b = 0; b < 2; b++) DALLOC(c, c->bq[b], (size_t)gx_bucket_words(c) * c->bcap);
+    c->cap = cap;
     return GX_OK;
 }
 
@@ -514,7 +519,7 @@ int gx_loadup(GxCtx* c, const float* coords, int64_t n) {
         GX_LAUNCHED(c);
         if (c->nzones > 1) {
             rc = gx_zone_loadup(c);
-            if (rc) return rc;
+            if (rc) return c->n = 0, rc;  // no zone codes: nothing that could move
         }
     }
     GX_CUDA(c, cudaStreamSynchronize(c->stream));

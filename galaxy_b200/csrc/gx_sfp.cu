@@ -902,7 +902,9 @@ __global__ void k_sfp_unxy(const float* __restrict__ xy, const float* __restrict
 extern "C" int gx_sfp_load(GxSfp* s, const float* coords, int64_t n, int stride) {
     if (!s || n < 0 || stride < 2 || (n > 0 && !coords)) return GX_ERR_ARG;
     cudaSetDevice(s->dev);
+    s->n = 0;  // until the particles are there
     if (n > s->cap) {
+        s->cap = 0;
         if (s->xy) cudaFree(s->xy);
         if (s->vel) cudaFree(s->vel);
         if (s->part) cudaFree(s->part);
@@ -914,15 +916,15 @@ extern "C" int gx_sfp_load(GxSfp* s, const float* coords, int64_t n, int stride)
             if (q) cudaFree(q);
         s->xy_alt = s->vel_alt = nullptr;
         s->ord = s->ord_alt = s->bins = nullptr;
-        s->cap = std::max<int64_t>(n, 1);
-        SFP_CUDA(s, cudaMalloc((void**)&s->xy, sizeof(float) * 2 * s->cap));
-        SFP_CUDA(s, cudaMalloc((void**)&s->vel, sizeof(float) * 2 * s->cap));
-        const int64_t nw = (s->cap + SFP_CHUNK_MIN - 1) / SFP_CHUNK_MIN;
-        const int64_t nb = (s->cap + 255) / 256;
+        const int64_t cap = std::max<int64_t>(n, 1);
+        SFP_CUDA(s, cudaMalloc((void**)&s->xy, sizeof(float) * 2 * cap));
+        SFP_CUDA(s, cudaMalloc((void**)&s->vel, sizeof(float) * 2 * cap));
+        const int64_t nw = (cap + SFP_CHUNK_MIN - 1) / SFP_CHUNK_MIN;
+        const int64_t nb = (cap + 255) / 256;
         const size_t bytes = std::max(sizeof(float) * nw * 64 * 32, sizeof(double) * nb * 64 * 32);
         SFP_CUDA(s, cudaMalloc((void**)&s->part, bytes));
+        s->cap = cap;
     }
-    s->n = n;
     s->reordered = s->no_order = false;
     s->since_sort = 0;
     if (n == 0) return GX_OK;
@@ -933,6 +935,7 @@ extern "C" int gx_sfp_load(GxSfp* s, const float* coords, int64_t n, int stride)
     SFP_CUDA(s, cudaGetLastError());
     SFP_CUDA(s, cudaFreeAsync(tmp, s->stream));
     SFP_CUDA(s, cudaStreamSynchronize(s->stream));
+    s->n = n;
     return GX_OK;
 }
 

@@ -88,8 +88,8 @@ class Sfp:
 
     def load(self, coords):
         coords = np.ascontiguousarray(coords, dtype=np.float32)
+        self._chk(self._L.gx_sfp_load(self._h, coords.ctypes.data, coords.shape[0], coords.shape[1]))
         self.n = coords.shape[0]
-        self._chk(self._L.gx_sfp_load(self._h, coords.ctypes.data, self.n, coords.shape[1]))
 
     def sum(self, pmass=1.0, precision=0):
         b = self.basis

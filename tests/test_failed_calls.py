@@ -4,8 +4,9 @@ gives the particles' mass and nothing on top of it."""
 import numpy as np
 import pytest
 
-from galaxy_b200 import Galaxy, GxError, make_config, GX_FLAG_SORTED_DEPOSIT, GX_GRID_MASS, GX_RMAP_STDPOL
-from galaxy_b200.disk import kt_disk
+from galaxy_b200 import (Galaxy, GxError, make_config, GX_FLAG_SORTED_DEPOSIT, GX_GRID_MASS, GX_PREC_FP64,
+                         GX_PREC_MIXED, GX_RMAP_STDPOL)
+from galaxy_b200.disk import exp_disk, kt_disk
 
 pytestmark = pytest.mark.gpu
 
@@ -96,3 +97,58 @@ def test_allocation_that_fails_does_not_fail_the_next_call():
             gal.step(2)
             out.append(gal.unload())
     assert np.array_equal(*out)
+
+
+@pytest.mark.parametrize("precision", [GX_PREC_MIXED, GX_PREC_FP64])
+def test_particles_that_do_not_fit_leave_an_empty_context(precision):
+    """loadup of more particles than the device holds, in a context that has
+    some: afterwards it has none, and takes the old ones again.  The steps are
+    those of a fresh context (FP64: up to the order of its atomics)."""
+    rec, pm = kt_disk(20000, seed=5, rmax=4.9, ndim=2, dt=0.05, lscale=10.0)
+    big = np.zeros((3_000_000, 4), np.float32)  # more than 100 bytes a particle in device arrays
+    out = []
+    for full in (False, True):
+        with Galaxy(cfg2(ng=9, pmass=pm, precision=precision)) as gal:
+            gal.greenm()
+            gal.loadup(rec)
+            gal.masset()
+            if full:
+                hold = almost_full(100 << 20)
+                try:
+                    with pytest.raises(GxError):
+                        gal.loadup(big)
+                    with pytest.raises(GxError):
+                        gal.step(1)  # no mass array
+                    assert not gal.unload().any()
+                    gal.loadup(rec)
+                    gal.masset()
+                finally:
+                    del hold
+                    release()
+            gal.step(2)
+            out.append(gal.unload())
+    if precision == GX_PREC_MIXED:
+        assert np.array_equal(*out)
+    else:
+        assert np.abs(out[0] - out[1]).max() <= 1e-6 * np.abs(out[0]).max()
+
+
+def test_sfp_particles_that_do_not_fit_leave_an_empty_handle(golden_dir):
+    import os
+    from galaxy_b200.sfp import Basis, Sfp
+    basis = Basis.from_json(os.path.join(golden_dir, "aj07.json"), maxm=8, maxn=19)
+    pos = exp_disk(20000, seed=4)
+    big = np.zeros((3_000_000, 2), np.float32)  # 80 bytes a particle
+    with Sfp(basis, 6.0) as s:
+        s.load(pos)
+        ref = s.sum()
+        hold = almost_full(100 << 20)
+        try:
+            with pytest.raises(GxError):
+                s.load(big)
+            assert not s.sum().any() and not s.unload().any()
+            s.load(pos)
+            assert np.array_equal(s.sum(), ref)
+        finally:
+            del hold
+            release()
