@@ -495,7 +495,6 @@ int gx_loadup(GxCtx* c, const float* coords, int64_t n) {
     c->have_mass = c->have_field = false;
     c->bucketed = false;
     c->zr_valid = false;
-    c->bk_grid = 0;
     const int nw = 2 * c->g.ndim;
     if (n == 0) return (c->nzones > 1 && !c->fp64) ? gx_zone_loadup(c) : GX_OK;
     float* staging = c->stagebuf;

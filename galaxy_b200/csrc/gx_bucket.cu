@@ -1131,25 +1131,27 @@ static int bk_launch_push(GxCtx* c, int cur, int nxt) {
     // the deposit window and, for the push, the staged field rows
     const size_t sb = sizeof(uint32_t) * (Q ? 28 : ND == 3 ? 16 : 4) * g.na;  // 25 rows and a pad: 16-byte aligned
     const size_t sf = sb + sizeof(float4) * (Q ? 9 : ND == 3 ? 4 : 2) * g.na;
-    if (!c->bk_grid) {
-        // CTAs of the push with and without the rows; the deposit alone runs as many
+    if (!c->bk_ctas[0]) {
+        // CTAs of the push without and with the rows, once per context; the deposit
+        // alone runs as many
         int pb = 0, pf = 0, sms = 148;
         auto kf = k_push_bkt<ND, COMP, false, Q>;
         GX_CUDA(c, cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sf));
         GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pf, kf, BK_THREADS, sf));
         GX_CUDA(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pb, kf, BK_THREADS, sb));
         GX_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev));
-        c->bk_stage = pf >= pb || c->n >= (int64_t)BK_STAGE_ROW * g.nrow;
-        c->bk_grid = std::max(1, c->bk_stage ? pf : pb) * sms;
+        c->bk_ctas[1] = std::max(1, pf) * sms;
+        c->bk_ctas[0] = std::max(1, pb) * sms;
     }
-    const size_t sm = DEP || !c->bk_stage ? sb : sf;
+    const bool stage = c->bk_ctas[1] >= c->bk_ctas[0] || c->n >= (int64_t)BK_STAGE_ROW * g.nrow;
+    const size_t sm = DEP || !stage ? sb : sf;
     auto kp = k_push_bkt<ND, COMP, DEP, Q>;
     GX_CUDA(c, cudaFuncSetAttribute(kp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
     c->acc_open = true;
-    kp<<<c->bk_grid, BK_THREADS, sm, c->stream>>>(g, c->bq[cur], c->bq[nxt], c->bcap, c->field, c->bk_items,
+    kp<<<c->bk_ctas[stage], BK_THREADS, sm, c->stream>>>(g, c->bq[cur], c->bq[nxt], c->bcap, c->field, c->bk_items,
                                                   c->bk_ctl + 8, c->bk_cap[nxt], c->bk_base[nxt],
                                                   c->bk_fill[nxt], c->bk_ctl + 4 * nxt, c->bk_main, c->macc,
-                                                  gx_mass_ranges(c), c->bk_stage ? BK_STAGE : INT_MAX);
+                                                  gx_mass_ranges(c), stage ? BK_STAGE : INT_MAX);
     GX_LAUNCHED(c);
     return GX_OK;
 }

@@ -190,8 +190,7 @@ struct GxCtx {
     int32_t* zr_d = nullptr;                 // [2][2] first, last plane holding the fused pass's mass
                                              // (ngz, -1 when empty), at 2 p of the conversion of set p
     bool zr_valid = false;                   // the mass array is the fused pass's (zr_d describes it)
-    int bk_grid = 0;                         // CTAs of the fused pass (0: to be found, for the loaded particles)
-    bool bk_stage = false;                   // its launches reserve the staged field rows
+    int bk_ctas[2] = {0, 0};                 // CTAs of the fused pass without and with staged field rows
     cudaStream_t bk_side = nullptr;          // the plan's stream (overlaps the field solve)
     cudaEvent_t bk_ev[2] = {nullptr, nullptr};  // push done (main), plan done (side)
     bool bk_pending = false;                 // a plan on bk_side the main stream has not joined
